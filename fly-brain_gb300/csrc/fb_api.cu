@@ -14,10 +14,10 @@
 #include <vector>
 
 #include "fb_internal.cuh"
-#include "fb_lagged.cuh"
+#include "fb_window.cuh"
 
 namespace fb {
-cudaError_t launch_rebuild_slots(Trial *Td, int nslots, int32_t *err, cudaStream_t st);
+cudaError_t launch_rebuild_slots(Trial *Td, int B, int nslots, int32_t *err, cudaStream_t st);
 int step_kernel_blocks_per_sm(size_t smem);
 size_t step_smem_bytes(int B);
 cudaError_t launch_step(const StepArgs &a, int grid, size_t smem, cudaStream_t st);
@@ -99,6 +99,7 @@ extern "C" void fb_default_params(fb_params *p) {
 
 // Columns of M^(2^j) for the xorshift32 map M (x ^= x<<13; x ^= x>>17; x ^= x<<5), expanded to 8
 // nibble tables of 16 words each: table[j][n][v] = M^(2^j) applied to (v << 4n).
+constexpr size_t kJumpWords = 32 * 128;
 static void build_jump_tables(std::vector<uint32_t> &tab) {
   auto step = [](uint32_t x) { x ^= x << 13; x ^= x >> 17; x ^= x << 5; return x; };
   uint32_t col[32][32];  // col[j][b] = M^(2^j) e_b
@@ -132,7 +133,7 @@ int set_error(int code, const char *msg) {
 }  // namespace fb
 
 static std::mutex g_dev_mu;
-static uint32_t *g_jump[64];
+static uint32_t *g_jump[64];  // per device: the 2^j jump tables, then the windowed kernel's
 
 static int device_jump(uint32_t **out) {
   int dev = 0;
@@ -146,6 +147,10 @@ static int device_jump(uint32_t **out) {
       return fail(FB_ENODEV, "device %d is sm_%d%d; this library is built for sm_103a", dev, p.major, p.minor);
     std::vector<uint32_t> tab;
     build_jump_tables(tab);
+    const size_t own = tab.size();
+    tab.resize(own + 2 * kWinJumpWords);
+    window_jump_tables(kWinWide, tab.data() + own);
+    window_jump_tables(kWinNarrow, tab.data() + own + kWinJumpWords);
     uint32_t *d = nullptr;
     CU(cudaMalloc(&d, tab.size() * 4));
     CU(cudaMemcpy(d, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice));
@@ -158,6 +163,8 @@ static int device_jump(uint32_t **out) {
 // ---------------------------------------------------------------------------------------------
 // graphs
 // ---------------------------------------------------------------------------------------------
+constexpr int32_t kMaxNeurons = (1 << 29) - 4096;  // delivery keys: rank << 3
+
 struct Topology {
   int32_t N = 0;
   int64_t E = 0;
@@ -165,6 +172,7 @@ struct Topology {
   // per edge, how many earlier edges of its row have the same target (0 .. kMaxRepeat); null
   // when no row repeats a target
   uint8_t *dup = nullptr;
+  uint32_t *inOff = nullptr;  // [N+1] in-degree prefix (where each target's contributions start)
   int refs = 0;
 };
 
@@ -178,6 +186,7 @@ static void topo_release(Topology *t) {
     cudaFree(t->indptr);
     cudaFree(t->indices);
     cudaFree(t->dup);
+    cudaFree(t->inOff);
     delete t;
   }
 }
@@ -197,8 +206,7 @@ extern "C" int fb_graph_create(int32_t N, int64_t E, const uint32_t *indptr, con
   CU(cudaMemcpy(ip.data(), indptr, (size_t)(N + 1) * 4, cudaMemcpyDefault));
   if (E) CU(cudaMemcpy(ix.data(), indices, (size_t)E * 4, cudaMemcpyDefault));
   if (ip[0] != 0 || ip[N] != (uint64_t)E) return fail(FB_EINVAL, "fb_graph_create: indptr[0]=%u indptr[N]=%u, E=%lld", ip[0], ip[N], (long long)E);
-  if (N >= (1 << 29) - kLagPer * kLagThreads * kLagMaxDB)
-    return fail(FB_EINVAL, "fb_graph_create: N=%d exceeds the delivery keys' %d", N, (1 << 29) - kLagPer * kLagThreads * kLagMaxDB);
+  if (N >= kMaxNeurons) return fail(FB_EINVAL, "fb_graph_create: N=%d exceeds the delivery keys' %d", N, kMaxNeurons);
   // a row may name a target more than once (lif.c:40-42 adds each edge in row order): each edge
   // gets its repeat index, which orders a presynaptic neuron's contributions to one target
   std::vector<int32_t> stamp(N, -1);
@@ -247,6 +255,11 @@ extern "C" int fb_graph_create(int32_t N, int64_t E, const uint32_t *indptr, con
                  cudaMemcpy(t->dup, rep.data(), (size_t)E, cudaMemcpyHostToDevice) != cudaSuccess)) {
     cleanup();
     return fail(FB_ECUDA, "fb_graph_create: upload of the repeat indices failed");
+  }
+  if (cudaMalloc(&t->inOff, (size_t)(N + 1) * 4) != cudaSuccess || launch_in_offsets(t->indices, N, E, t->inOff, 0) != cudaSuccess ||
+      cudaStreamSynchronize(0) != cudaSuccess) {
+    cleanup();
+    return fail(FB_ECUDA, "fb_graph_create: in-degree offsets: %s", cudaGetErrorString(cudaGetLastError()));
   }
   *out = g;
   return FB_OK;
@@ -387,7 +400,7 @@ struct DrivenSet {
   std::vector<int32_t> order;  // neuron or -1
   std::vector<int32_t> pos;    // index in order, or -1
   bool dirty = true;
-  uint64_t version = 0;  // changes with the set (ownership of the delay-scheduled kernel)
+  uint64_t version = 0;  // changes with the set (the windowed kernel's list positions)
   void init(int N) { order.clear(); pos.assign(N, -1); dirty = true; version++; }
   void add(int32_t i) {
     if (pos[i] >= 0) return;
@@ -415,24 +428,22 @@ struct DrivenSet {
   }
 };
 
-// Device resources of the delay-scheduled kernel (fb_lagged.cu) for a single brain, allocated
-// at its first use at the largest sizes the brain can need.
-struct LagRes {
+// Device resources of the windowed kernel (fb_window.cu), allocated at its first use.
+struct WinRes {
   bool ready = false;
-  int D = 0, S = 0, nTB = 0, capMax = 0, nDmax = 0, bgCap = 0, grid = 0;
-  uint64_t drivenVersion = ~0ull;
-  std::vector<void *> allocs;
-  uint32_t *inOff = nullptr, *cnt = nullptr, *pend0 = nullptr, *sync = nullptr, *bgList = nullptr;
-  uint32_t *jumpHex = nullptr;
-  uint4 *edgeRec = nullptr;
-  uint2 *buf = nullptr;
-  uint4 *dbList = nullptr;
-  int32_t *bgCount = nullptr, *dbCnt = nullptr, *dbNF = nullptr, *tStage = nullptr, *tCnt = nullptr;
-  int32_t *ndIds = nullptr, *ndLo = nullptr, *drvPosOf = nullptr;
-  int cap = 1, nD = 0;
-  int nDB = 1, nDcap = 32, nDall = 32, dLo[kLagMaxDB + 1] = {0, 0, 0};
-  unsigned long long *liveTag = nullptr;
+  bool noMemory = false;                 // the allocation failed: AUTO does not try again
+  char *arena = nullptr;
+  std::vector<void *> allocs;            // what only some launches need
+  std::vector<WinBrain> host;            // as created: sizes and pointers
+  std::vector<uint64_t> drivenVersion;
+  WinBrain *win = nullptr;
+  uint32_t *sync = nullptr;              // barrier word, tile counters
+  char *backup = nullptr;                // one brain: its state before a launch
   size_t smem = 0;
+  uint32_t barBase = 0;                  // grid-barrier arrivals so far
+  int maxD = 0;
+  // where the spikes in flight are: the ring's lists, the log, or both
+  bool ringValid = true, logValid = true;
 };
 
 struct fb_brains {
@@ -477,12 +488,16 @@ struct fb_brains {
   int32_t subGrab = 4;
   int64_t timeoutNs = 5000000000LL;  // bound of every device-side wait (fb_tuning.timeout_us)
   int32_t tripStep = -1;             // test hook (fb_debug_trip_wait): armed for one launch
-  int32_t lagDB = 0;                 // driven blocks of the delay-scheduled kernel (0: automatic)
+  int32_t lagDB = 0;                 // fb_tuning.lag_driven_blocks (accepted; the schedule needs none)
+  int32_t irregular = 0;             // steps in which a neuron may fire sooner than its refractory time
   int logging = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float lastMs = 0.f;
   int32_t schedule = FB_SCHEDULE_AUTO, lastSchedule = FB_SCHEDULE_GRID;
-  LagRes lag;
+  WinRes win;
+  std::vector<Topology *> topo;      // each brain's (the graphs outlive the batch)
+  int maxSlots = 0;
+  bool everGrid = false;             // the grid kernel has run
 };
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -524,6 +539,9 @@ static uint32_t seed_state(uint32_t seed) {
   return s ? s : 1u;
 }
 
+static bool win_capable(const fb_brains *br);
+static int win_create(fb_brains *br, bool early);
+
 extern "C" int fb_brains_create(const fb_graph *const *graphs, int32_t B, const fb_params *params,
                                 int32_t params_stride, const uint32_t *seeds, fb_brains **out) {
   if (!out) return fail(FB_EINVAL, "fb_brains_create: out is null");
@@ -540,6 +558,7 @@ extern "C" int fb_brains_create(const fb_graph *const *graphs, int32_t B, const 
   }
   br->B = B;
   br->host.assign(B, Trial{});
+  br->topo.assign(B, nullptr);
   br->dts.assign(B, 0.0);
   br->driven.resize(B);
   int tileBase = 0;
@@ -557,6 +576,8 @@ extern "C" int fb_brains_create(const fb_graph *const *graphs, int32_t B, const 
       return brains_fail_cleanup(br, fail(FB_EINVAL, "fb_brains_create: brain %d: delay/dt rounds to %d step; at least 2 are required", b, ns - 1));
     Trial &T = br->host[b];
     br->dts[b] = p.dt;
+    br->topo[b] = g->topo;
+    br->maxSlots = std::max(br->maxSlots, ns);
     T.N = N;
     T.E = E;
     T.nslots = ns;
@@ -663,6 +684,7 @@ extern "C" int fb_brains_create(const fb_graph *const *graphs, int32_t B, const 
     return brains_fail_cleanup(br, fail(FB_ENOMEM, "fb_brains_create: pinned host staging"));
   if (cudaStreamSynchronize(br->stream) != cudaSuccess)
     return brains_fail_cleanup(br, fail(FB_ECUDA, "fb_brains_create: %s", cudaGetErrorString(cudaGetLastError())));
+  if (win_capable(br) && win_create(br, true) != FB_OK) g_err.clear();  // short of memory: the grid kernel only
   *out = br;
   return FB_OK;
 }
@@ -680,7 +702,8 @@ extern "C" int fb_brains_destroy(fb_brains *br) {
   cudaFree(br->d_phase);
   cudaFree(br->d_dbg);
   cudaFree(br->d_ovf[0]); cudaFree(br->d_ovf[1]);
-  for (void *p : br->lag.allocs) cudaFree(p);
+  for (void *p : br->win.allocs) cudaFree(p);
+  cudaFree(br->win.arena);
   if (br->ev0) cudaEventDestroy(br->ev0);
   if (br->ev1) cudaEventDestroy(br->ev1);
   if (br->flushDone) cudaEventDestroy(br->flushDone);
@@ -707,12 +730,9 @@ extern "C" int fb_brains_set_tuning(fb_brains *br, const fb_tuning *t) {
     return fail(FB_EINVAL, "fb_brains_set_tuning: blocks_per_sm %d (1..%d), item_chunks %d (1..64), sub_grab %d (-1, 1..256), "
                 "timeout_us %d (>= 1)", t->blocks_per_sm, br->maxBlocksPerSm, t->item_chunks, t->sub_grab, t->timeout_us);
   if (t->timeout_us) br->timeoutNs = (int64_t)t->timeout_us * 1000;
-  if (t->lag_driven_blocks < 0 || t->lag_driven_blocks > kLagMaxDB)
-    return fail(FB_EINVAL, "fb_brains_set_tuning: lag_driven_blocks %d (0 automatic, 1..%d)", t->lag_driven_blocks, kLagMaxDB);
-  if (t->lag_driven_blocks != br->lagDB) {
-    br->lagDB = t->lag_driven_blocks;
-    br->lag.drivenVersion = ~0ull;  // the ownership is recomputed at the next launch
-  }
+  if (t->lag_driven_blocks < 0 || t->lag_driven_blocks > 2)
+    return fail(FB_EINVAL, "fb_brains_set_tuning: lag_driven_blocks %d (0..2)", t->lag_driven_blocks);
+  br->lagDB = t->lag_driven_blocks;
   if (t->blocks_per_sm) {
     br->blocksPerSm = t->blocks_per_sm;
     br->grid = br->sms * br->blocksPerSm;
@@ -902,6 +922,15 @@ extern "C" int fb_pulse(fb_brains *br, int32_t b, const int32_t *idx, const doub
   return queue(br, b, FB_FIELD_GE, idx, mv, n, "fb_pulse");
 }
 
+// The ring's lists from the log, before anything but the windowed kernel reads them.
+static int ring_from_log(fb_brains *br) {
+  WinRes &R = br->win;
+  if (R.ringValid || !R.ready) return FB_OK;
+  CU(launch_log_export(br->trials, R.win, 0, br->B, R.maxD, false, br->stream));
+  R.ringValid = true;
+  return FB_OK;
+}
+
 extern "C" int fb_reset(fb_brains *br, int32_t b) {
   if (!br) return fail(FB_EINVAL, "fb_reset: null handle");
   if (b != -1) {
@@ -910,12 +939,15 @@ extern "C" int fb_reset(fb_brains *br, int32_t b) {
   }
   int rc = flush(br);
   if (rc) return rc;
+  if ((rc = ring_from_log(br))) return rc;  // the last fired list stays readable
   CU(launch_reset(br->trials, b < 0 ? 0 : b, b < 0 ? br->B : b + 1, br->stream));
   for (int32_t k = b < 0 ? 0 : b; k < (b < 0 ? br->B : b + 1); k++) {  // adapt 0 and res 1 again
     Trial &T = br->host[k];
     T.flags = (T.flags & ~(kAdaptZero | kResRest)) | rest_flags(T);
     CU(cudaMemcpyAsync(&br->trials[k].flags, &T.flags, 4, cudaMemcpyHostToDevice, br->stream));
   }
+  if (br->win.ready && br->win.logValid)  // the spikes in flight are dropped from the log too
+    CU(launch_log_clear(br->win.win, b < 0 ? 0 : b, b < 0 ? br->B : b + 1, br->stream));
   CU(cudaStreamSynchronize(br->stream));
   return FB_OK;
 }
@@ -936,7 +968,7 @@ extern "C" int fb_set_background(fb_brains *br, int32_t b, double rate_hz, doubl
 
 // LIFGpu.setParams (src/lifgpu.js:349): new parameters for brain b's header constants, taking
 // effect at the next step. The ring depth round(delay/dt)+1 must not change (the ring and the
-// delay-scheduled buffers are sized by it). Constant-state flags stay only while their condition
+// windowed buffers are sized by it). Constant-state flags stay only while their condition
 // holds (adapt 0 needs adaptInc 0, res 1 needs depU 0); presynaptic inhibition switches the
 // delivery to the sequential mode and back.
 extern "C" int fb_set_params(fb_brains *br, int32_t b, const fb_params *p) {
@@ -959,6 +991,17 @@ extern "C" int fb_set_params(fb_brains *br, int32_t b, const fb_params *p) {
   int32_t mode = T.mode;
   if (f & kHasPreInh) mode = FB_DELIVER_SEQUENTIAL;
   else if ((T.flags & kHasPreInh) && mode == FB_DELIVER_SEQUENTIAL) mode = FB_DELIVER_EXACT;
+  if (T.tRef != nt.tRef || T.dt != nt.dt) {
+    // neurons may now fire sooner than the windows and the log assume: the windowed kernel's
+    // resources are sized again at its next launch, from the ring
+    br->irregular = std::max(br->irregular, T.nslots - 1);
+    if (br->win.ready) {
+      if ((rc = ring_from_log(br))) return rc;
+      CU(cudaStreamSynchronize(br->stream));
+      br->win.ready = false;
+      br->everGrid = true;
+    }
+  }
   T.coba = nt.coba;
   T.mode = mode;
   T.flags = f;
@@ -977,212 +1020,319 @@ extern "C" int fb_set_params(fb_brains *br, int32_t b, const fb_params *p) {
   return FB_OK;
 }
 
-// ---- the delay-scheduled kernel ----------------------------------------------------------------
+// ---- the windowed (delay-scheduled) kernel -------------------------------------------------------
 
-// AUTO: shorter launches take the grid kernel. The delay-scheduled launch carries a fixed ~110 us
-// (clearing its buffers, loading every block's state into shared memory and writing it back, the
-// ring bookkeeping) against the grid kernel's ~15 us; at the full graph they break even near 6
-// steps (grid 20-26 us per step, delay-scheduled 4-7).
-constexpr int kLagMinSteps = 8;
+// AUTO takes the windowed kernel from this many steps on. Measured on one brain (microseconds per
+// call, spike counts read back; grid / windowed): 165,122 neurons, 2 steps 83 / 62, 16 steps 354 /
+// 72; 1,501 neurons, 1 step 53 / 55, 2 steps 57 / 55. Background events add a phase to a window:
+// 165,122 neurons, 2 steps 88 / 90, 3 steps 107 / 96.
+static int win_min_steps(const fb_brains *br) {
+  for (const Trial &T : br->host)
+    if (T.flags & kHasBg) return 3;
+  return 2;
+}
+// Launches of one brain from this length on (and forced ones) leave the brain as it was when they
+// time out: its state is copied first (about 5 us at the full graph).
+constexpr int kWinBackupSteps = 8;
+constexpr int kWinLogSteps = 64;  // longest launch with per-step logging
 
-// Whether the delay-scheduled kernel applies to this launch (why not, in *why).
+// Steps a neuron of brain T stays silent after a spike: lif.c:61-64 counts refr down in f32; a
+// forced spike starts from tRef + dt in its own step.
+static int silent_steps(const Trial &T) {
+  auto count = [&](float r) {
+    int k = 0;
+    for (; r > 0 && k < kWinMax; k++) r = r - T.dt;
+    return k;
+  };
+  return std::min(count(T.tRef), count((T.tRef + T.dt) - T.dt));
+}
+
+// Steps whose draws fit in a block's shared memory beside the driven entries.
+static int64_t drawn_steps(const Trial &T, int64_t nD) {
+  const int64_t room = std::min<int64_t>(kWinStream, kWinPool - window_entry_words((int)nD));
+  return room / (nD + (T.bgEvents > 0 ? (int64_t)T.bgEvents + 2 : 0) + 1);
+}
+
+// The longest window of brain T: its delay, the steps a neuron stays silent, the draws.
+static int window_steps(const Trial &T, int64_t nD) {
+  return (int)std::min<int64_t>({T.nslots - 1, std::max(1, silent_steps(T)), kWinMax, drawn_steps(T, nD)});
+}
+
+// Whether the windowed kernel can run this batch at all, and whether it applies to this launch
+// under the delay-scheduled schedule (why not, in *why).
+static bool win_capable(const fb_brains *br) {
+  if (br->B > kWinBrains) return false;
+  for (int b = 0; b < br->B; b++) {
+    const Trial &T = br->host[b];
+    const int64_t nD = (int64_t)br->driven[b].order.size();
+    if (T.mode != FB_DELIVER_EXACT || (T.flags & kHasPreInh) || T.nslots - 1 < 4 || T.nslots - 1 > 32 ||
+        T.N >= kWinIds || nD > kWinDriven || !(T.bgEvents < (float)kWinStream) || drawn_steps(T, nD) < 1 ||
+        silent_steps(T) < 1)  // a neuron may be forced and cross its threshold in one step
+      return false;
+  }
+  return true;
+}
 static bool lag_applies(fb_brains *br, int32_t steps, const char **why) {
   const Trial &T = br->host[0];
   *why = nullptr;
   if (br->B != 1) *why = "a batch of more than one brain";
   else if (T.mode != FB_DELIVER_EXACT || (T.flags & kHasPreInh)) *why = "a delivery mode other than exact without presynaptic inhibition";
-  else if (br->profiling && br->schedule != FB_SCHEDULE_LAGGED) *why = "phase profiling";
-  else if (br->logging && steps > kLagRing) *why = "per-step logging of a launch longer than 64 steps";
-  // a block's wait at step s (for step s - L, L = D - help) must not need its own completion of
-  // that step, which it publishes at step s - L + 1: L >= 2
+  else if (br->logging && steps > kWinLogSteps) *why = "per-step logging of a launch longer than 64 steps";
   else if (T.nslots - 1 < 4 || T.nslots - 1 > 32) *why = "a ring depth outside 5..33 slots";
   else if (T.bgEvents > (float)(1 << 20)) *why = "more than 2^20 background events per step";
+  else if ((int)br->driven[0].order.size() > kWinDriven) *why = "more than 4096 driven neurons";
   return *why == nullptr;
 }
 
 template <typename X>
-static int lag_alloc(fb_brains *br, X **p, size_t n) {
+static int win_alloc(fb_brains *br, X **p, size_t n) {
   void *q = nullptr;
   if (cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(X)) != cudaSuccess) {
     cudaGetLastError();
-    return fail(FB_ENOMEM, "fb_step: %zu bytes for the delay-scheduled kernel", n * sizeof(X));
+    return fail(FB_ENOMEM, "fb_step: %zu bytes for the windowed kernel", n * sizeof(X));
   }
-  br->lag.allocs.push_back(q);
+  br->win.allocs.push_back(q);
   *p = (X *)q;
   return FB_OK;
 }
 
-// Allocates the kernel's resources and (when the driven set changed) the neuron ownership.
-static int lag_setup(fb_brains *br) {
-  LagRes &R = br->lag;
-  Trial &T = br->host[0];
-  const int N = T.N;
-  const int64_t E = T.E;
+// The kernel's resources: one allocation for the batch. At the batch's creation (early) they wait
+// for the first launch if they would take much of the free memory.
+static int win_create(fb_brains *br, bool early) {
+  WinRes &R = br->win;
+  const int B = br->B;
+  cudaFree(R.arena);
+  R.arena = nullptr;
+  for (void *p : R.allocs) cudaFree(p);
+  R.allocs.clear();
+  R.host.assign(B, WinBrain{});
+  R.drivenVersion.assign(B, ~0ull);
+  R.backup = nullptr;
+  R.maxD = 0;
+  R.smem = window_smem_bytes(B);
+  if (window_blocks_per_sm(B, R.smem) < 1) return fail(FB_EINVAL, "fb_step: the windowed kernel does not fit on an SM (%zu bytes)", R.smem);
+  auto n4 = [&](int b) { return align256((size_t)br->host[b].N * 4); };
+  // what must start at zero comes first: per brain drvPos, bgMask and arr (wcnt from the offsets)
+  size_t zero = align256(sizeof(WinBrain) * B) + align256(256 * 4), rest = 0;
+  std::vector<uint64_t> cap(B, 1024);
+  for (int b = 0; b < B; b++) {
+    const Trial &T = br->host[b];
+    // spikes of the last D + H steps: a neuron fires at most once in any H of them (H >= 1)
+    const int D = T.nslots - 1, H = std::min(D, silent_steps(T));
+    while (cap[b] < (uint64_t)T.N * ((D + H - 1) / H + 2)) cap[b] *= 2;
+    zero += 2 * n4(b) + align256(T.N);
+    rest += n4(b) + align256(cap[b] * 16) + align256((size_t)T.E * 8) + align256((size_t)kWinDriven * (4 + kWinSaved * 4 + 1));
+  }
+  if (early && zero + rest > ((size_t)8 << 30)) {
+    size_t avail = 0, total = 0;
+    CU(cudaMemGetInfo(&avail, &total));
+    if (zero + rest > avail / 4) return FB_OK;
+  }
+  if (cudaMalloc(&R.arena, zero + rest) != cudaSuccess) {
+    cudaGetLastError();
+    R.arena = nullptr;
+    R.noMemory = true;
+    return fail(FB_ENOMEM, "fb_step: %zu bytes for the windowed kernel", zero + rest);
+  }
+  char *at = R.arena;
+  auto take = [&](size_t bytes) {
+    char *p = at;
+    at += align256(bytes);
+    return p;
+  };
+  CU(cudaMemsetAsync(R.arena, 0, zero, br->stream));
+  R.win = (WinBrain *)take(sizeof(WinBrain) * B);
+  R.sync = (uint32_t *)take(256 * 4);
+  R.barBase = 0;
+  for (int b = 0; b < B; b++) {
+    const Trial &T = br->host[b];
+    WinBrain &W = R.host[b];
+    W.bgMask = (uint32_t *)take(n4(b));
+    W.drvPos = (int32_t *)take(n4(b));
+    W.arr = (uint8_t *)take(T.N);
+  }
+  for (int b = 0; b < B; b++) {
+    const Trial &T = br->host[b];
+    WinBrain &W = R.host[b];
+    W.D = T.nslots - 1;
+    W.inOff = br->topo[b]->inOff;
+    R.maxD = std::max(R.maxD, W.D);
+    W.logMask = (uint32_t)(cap[b] - 1);
+    W.wcnt = (uint32_t *)take(n4(b));
+    W.log = (uint4 *)take(cap[b] * 16);
+    W.wbuf = (uint2 *)take((size_t)T.E * 8);
+    char *d = take((size_t)kWinDriven * (4 + kWinSaved * 4 + 1));
+    W.dSave = (float4 *)d;
+    W.dLive = (uint32_t *)(d + (size_t)kWinDriven * kWinSaved * 4);
+    W.dFired = (uint8_t *)(W.dLive + kWinDriven);
+    CU(cudaMemcpyAsync(W.wcnt, W.inOff, (size_t)T.N * 4, cudaMemcpyDeviceToDevice, br->stream));
+  }
+  CU(cudaMemcpyAsync(R.win, R.host.data(), sizeof(WinBrain) * B, cudaMemcpyHostToDevice, br->stream));
+  CU(cudaStreamSynchronize(br->stream));
+  R.ready = true;
+  R.logValid = !br->everGrid;  // nothing in flight yet, unless the grid kernel ran
+  return FB_OK;
+}
+
+// The resources, with list positions and background buffers up to date.
+static int win_setup(fb_brains *br) {
+  WinRes &R = br->win;
   int rc;
-  if (!R.ready) {
-    int sms = 0, optin = 0;
-    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, br->dev));
-    CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, br->dev));
-    R.grid = sms;
-    R.nTB = sms - 1;
-    R.D = T.nslots - 1;
-    R.S = 2 * R.D;
-    // tile blocks hold at most ceil(N / (sms - kLagMaxDB)) neurons (the fewest tile blocks)
-    R.capMax = std::max(1, (N + sms - kLagMaxDB - 1) / (sms - kLagMaxDB));
-    int perDB = 0;  // driven entries one driven block holds at most
-    for (int nd = 32; nd <= kLagPer * kLagThreads; nd += 32)
-      if (lagged_smem_bytes(R.capMax, nd, kLagMaxDB * nd) <= (size_t)optin) perDB = nd;
-    if (perDB == 0) return fail(FB_EINVAL, "fb_step: the delay-scheduled kernel does not fit in shared memory");
-    R.nDmax = kLagMaxDB * perDB;
-    // in-degree prefix: each target's bucket entries start at inOff[q]
-    std::vector<uint32_t> ix(E), off(N + 1, 0);
-    if (E) CU(cudaMemcpy(ix.data(), T.indices, E * 4, cudaMemcpyDeviceToHost));
-    for (int64_t j = 0; j < E; j++) off[ix[j] + 1]++;
-    for (int q = 0; q < N; q++) off[q + 1] += off[q];
-    if ((rc = lag_alloc(br, &R.inOff, N + 1)) || (rc = lag_alloc(br, &R.cnt, (size_t)R.S * (N + R.nDmax))) ||
-        (rc = lag_alloc(br, &R.buf, (size_t)R.S * std::max<int64_t>(E, 1))) || (rc = lag_alloc(br, &R.pend0, N)) ||
-        (rc = lag_alloc(br, &R.sync, 256)) || (rc = lag_alloc(br, &R.bgCount, kLagRing)) ||
-        (rc = lag_alloc(br, &R.dbList, (size_t)kLagRing * R.nDmax * 2)) ||
-        (rc = lag_alloc(br, &R.dbCnt, (size_t)kLagRing * kLagMaxDB)) ||
-        (rc = lag_alloc(br, &R.liveTag, (size_t)kLagRing * kLagMaxDB)) ||
-        (rc = lag_alloc(br, &R.dbNF, kLagRing)) || (rc = lag_alloc(br, &R.tStage, (size_t)kLagRing * R.grid * R.capMax)) ||
-        (rc = lag_alloc(br, &R.tCnt, (size_t)kLagRing * R.grid)) || (rc = lag_alloc(br, &R.ndIds, N)) ||
-        (rc = lag_alloc(br, &R.ndLo, R.grid + 1)) || (rc = lag_alloc(br, &R.drvPosOf, N)) || (rc = lag_alloc(br, &R.edgeRec, std::max<int64_t>(E, 1))))
-      return rc;
-    CU(cudaMemcpy(R.inOff, off.data(), (N + 1) * 4, cudaMemcpyHostToDevice));
-    std::vector<uint32_t> tab;
-    lagged_jump_tables(tab);
-    if ((rc = lag_alloc(br, &R.jumpHex, tab.size()))) return rc;
-    CU(cudaMemcpyAsync(R.jumpHex, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice, br->stream));
-    CU(cudaStreamSynchronize(br->stream));
-    R.ready = true;
-  }
-  const int bgNeed = T.bgEvents > 0 ? (int)std::ceil((double)T.bgEvents) + 1 : 1;
-  if (bgNeed > R.bgCap) {
-    if ((rc = lag_alloc(br, &R.bgList, (size_t)kLagRing * bgNeed))) return rc;
-    R.bgCap = bgNeed;
-  }
-  const DrivenSet &ds = br->driven[0];
-  if (ds.version != R.drivenVersion) {
-    const int nD = (int)ds.order.size();
-    if (nD > R.nDmax) return fail(FB_EINVAL, "fb_step: %d driven neurons exceed the delay-scheduled kernel's %d", nD, R.nDmax);
-    if ((int64_t)nD + R.bgCap + 64 >= 65536)
-      return fail(FB_EINVAL, "fb_step: %d draws per step exceed the delay-scheduled kernel's jump tables", nD + R.bgCap);
-    std::vector<uint8_t> isD(N, 0);
-    for (int32_t i : ds.order) isD[i] = 1;
-    std::vector<int32_t> nd;
-    nd.reserve(N - nD);
-    for (int i = 0; i < N; i++)
-      if (!isD[i]) nd.push_back(i);
-    const int64_t Nnd = (int64_t)nd.size();
-    // a long driven list is split over two driven blocks in list order (their draws stay in
-    // lif.c's order: each offsets its own by the other's share); the other SMs are tile blocks
-    R.nDB = br->lagDB ? br->lagDB : nD >= kLagSplit ? 2 : 1;
-    if (R.nDB > 1 && nD < R.nDB) R.nDB = 1;  // every driven block owns at least one entry
-    R.nTB = R.grid - R.nDB;
-    for (int d = 0; d <= R.nDB; d++) R.dLo[d] = (int)((int64_t)nD * d / R.nDB);
-    int part = 0;
-    for (int d = 0; d < R.nDB; d++) part = std::max(part, R.dLo[d + 1] - R.dLo[d]);
-    std::vector<int32_t> lo(R.nTB + 1);
-    for (int t = 0; t <= R.nTB; t++) lo[t] = (int32_t)(Nnd * t / R.nTB);
-    std::vector<int32_t> posOf(N, -1);
-    for (int k = 0; k < nD; k++) posOf[ds.order[k]] = k;
-    if (Nnd) CU(cudaMemcpyAsync(R.ndIds, nd.data(), Nnd * 4, cudaMemcpyHostToDevice, br->stream));
-    CU(cudaMemcpyAsync(R.ndLo, lo.data(), (R.nTB + 1) * 4, cudaMemcpyHostToDevice, br->stream));
-    CU(cudaMemcpyAsync(R.drvPosOf, posOf.data(), (size_t)N * 4, cudaMemcpyHostToDevice, br->stream));
-    CU(launch_edge_records(T.indices, T.dup, R.inOff, R.drvPosOf, N, E, R.edgeRec, br->stream));
-    CU(cudaStreamSynchronize(br->stream));
-    R.nD = nD;
-    R.cap = std::max<int>(1, (int)((Nnd + R.nTB - 1) / R.nTB));
-    if (R.cap > std::min(R.capMax, kLagPer * kLagTileWorkers) || part > kLagPer * kLagThreads ||
-        (nD + R.nTB - 1) / R.nTB > kLagHelpMax)
-      return fail(FB_EINVAL, "fb_step: %d neurons per tile block (at most %d) or %d driven neurons per driven block "
-                  "(at most %d) exceed the delay-scheduled kernel", R.cap, std::min(R.capMax, kLagPer * kLagTileWorkers),
-                  part, kLagPer * kLagThreads);
-    R.nDcap = std::max(32, (part + 31) / 32 * 32);
-    R.nDall = std::max(32, (nD + 31) / 32 * 32);
-    R.smem = lagged_smem_bytes(R.cap, R.nDcap, R.nDall);
-    if (lagged_blocks_per_sm(R.smem) < 1)
-      return fail(FB_EINVAL, "fb_step: the delay-scheduled kernel does not fit on an SM (%zu bytes)", R.smem);
-    R.drivenVersion = ds.version;
+  if (!R.ready && (rc = win_create(br, false))) return rc;
+  for (int b = 0; b < br->B; b++) {
+    const Trial &T = br->host[b];
+    WinBrain &W = R.host[b];
+    if ((T.flags & kHasBg) && !W.bgHit) {
+      if ((rc = win_alloc(br, &W.bgHit, (size_t)T.N * std::min(T.nslots - 1, kWinMax)))) return rc;
+      CU(cudaMemsetAsync(W.bgHit, 0, (size_t)T.N * std::min(T.nslots - 1, kWinMax) * 4, br->stream));
+      CU(cudaMemcpyAsync(&R.win[b].bgHit, &W.bgHit, sizeof(void *), cudaMemcpyHostToDevice, br->stream));
+    }
+    const DrivenSet &ds = br->driven[b];
+    if (ds.version != R.drivenVersion[b]) {
+      const int nD = (int)ds.order.size();
+      CU(launch_driven_pos(T.driven, nD, T.N, W.drvPos, br->stream));
+      W.hasDriven = nD > 0;
+      CU(cudaMemcpyAsync(&R.win[b].hasDriven, &W.hasDriven, 4, cudaMemcpyHostToDevice, br->stream));
+      R.drivenVersion[b] = ds.version;
+    }
   }
   return FB_OK;
 }
 
-static int run_lagged(fb_brains *br, int32_t steps) {
-  LagRes &R = br->lag;
-  Trial &T = br->host[0];
-  const int N = T.N;
-  CU(cudaEventRecord(br->ev0, br->stream));  // the launch's clearing is part of its time
-  CU(cudaMemsetAsync(R.sync, 0, 256 * 4, br->stream));
-  CU(cudaMemsetAsync(R.cnt, 0, (size_t)R.S * (N + R.nDmax) * 4, br->stream));
-  CU(cudaMemsetAsync(R.pend0, 0, (size_t)N * 4, br->stream));
-  CU(cudaMemsetAsync(R.liveTag, 0, sizeof(unsigned long long) * kLagRing * kLagMaxDB, br->stream));
-  LagArgs a;
+// One windowed launch of steps[b] steps (windows of at most hCap steps).
+static int win_launch(fb_brains *br, const std::vector<int32_t> &steps, int hCap) {
+  WinRes &R = br->win;
+  WinArgs a;
   memset(&a, 0, sizeof a);
-  a.G = br->trials;
-  a.N = N;
-  a.E = T.E;
-  a.T = steps;
-  a.D = R.D;
-  a.S = R.S;
-  a.help = lag_help(R.D);
-  a.dbPub = a.help - 1;
-  a.L = R.D - a.help;
-  a.nTB = R.nTB;
-  a.cap = R.cap;
-  a.nD = R.nD;
-  a.nDcap = R.nDcap;
-  a.nDall = R.nDall;
-  a.nDB = R.nDB;
-  for (int d = 0; d <= kLagMaxDB; d++) a.dLo[d] = R.dLo[std::min(d, R.nDB)];
-  a.hasBg = T.bgEvents > 0 ? 1 : 0;
-  a.bgCap = R.bgCap;
-  a.dt = T.dt; a.vRest = T.vRest; a.vThresh = T.vThresh; a.vReset = T.vReset; a.tRef = T.tRef;
-  a.adaptInc = T.adaptInc; a.depU = T.depU; a.dE = T.dE; a.dTr = T.dTr; a.dA = T.dA; a.kRec = T.kRec;
-  a.kM = T.kM; a.dtS = T.dtS; a.eExc = T.eExc; a.eInh = T.eInh; a.cE = T.cE; a.cI = T.cI;
-  a.bgEvents = T.bgEvents; a.bgAmp = T.bgAmp; a.coba = T.coba;
-  a.indptr = T.indptr; a.indices = T.indices; a.W = T.W; a.sign = T.sign; a.inOff = R.inOff;
-  a.v = T.v; a.gE = T.gE; a.gI = T.gI; a.refr = T.refr; a.trace = T.trace; a.adapt = T.adapt; a.res = T.res;
-  a.bias = T.bias; a.thr = T.thr; a.drive = T.drive; a.spikeCount = T.spikeCount;
-  a.ring = T.ring; a.ringCount = T.ringCount; a.driven = T.driven;
-  a.ndIds = R.ndIds; a.ndLo = R.ndLo; a.drvPosOf = R.drvPosOf;
-  a.cnt = R.cnt; a.cntStride = N + R.nDmax; a.buf = R.buf; a.pend0 = R.pend0;
-  a.done = R.sync; a.dbDone = R.sync + 64; a.bgReady = R.sync + 72; a.barCount = R.sync + 128;
-  a.liveTag = R.liveTag;
-  a.stepTot = (int32_t *)(R.sync + 192);
-  a.bgList = R.bgList; a.bgCount = R.bgCount; a.dbList = R.dbList; a.dbCnt = R.dbCnt;
-  a.tStage = R.tStage; a.tCnt = R.tCnt;
-  a.log = br->logging;
-  a.logCount = T.logCount; a.logRaster = T.logRaster; a.logCap = T.logCap; a.logRasterCap = T.logRasterCap;
-  a.prof = br->profiling ? br->d_phase : nullptr;
-  a.jumpHex = R.jumpHex;
-  a.edgeRec = R.edgeRec;
+  a.allPlain = 1;
+  for (int b = 0; b < br->B; b++) {
+    const Trial &T = br->host[b];
+    const int32_t H = std::min(window_steps(T, (int64_t)br->driven[b].order.size()), hCap);
+    if (H != R.host[b].H) {
+      R.host[b].H = H;
+      CU(cudaMemcpyAsync(&R.win[b].H, &R.host[b].H, 4, cudaMemcpyHostToDevice, br->stream));
+    }
+    a.nWin = std::max(a.nWin, (steps[b] + H - 1) / H);
+    if (steps[b] > 0 && (T.flags & kHasBg)) a.anyBg = 1;
+    if ((T.flags & (kAdaptZero | kResRest | kHasBg | kHasDep)) != (kAdaptZero | kResRest) || T.coba) a.allPlain = 0;
+  }
+  if (a.nWin == 0) return FB_OK;
+  if (br->stepsUploaded != steps) {  // the last launch's counts stay on the device otherwise
+    std::memcpy(br->h_steps, steps.data(), sizeof(int32_t) * br->B);
+    CU(cudaMemcpyAsync(br->d_steps, br->h_steps, sizeof(int32_t) * br->B, cudaMemcpyHostToDevice, br->stream));
+    br->stepsUploaded = steps;
+  }
+  a.trials = br->trials;
+  a.win = R.win;
+  a.B = br->B;
+  a.steps = br->d_steps;
+  a.dedicated = br->B * 8 <= br->sms;
+  a.jump = br->jump + kJumpWords + (window_threads(br->B) == kWinNarrow ? kWinJumpWords : 0);
+  a.barCount = R.sync;
+  a.uNext = R.sync + 64;
   a.err = br->d_err;
   a.timeoutNs = br->timeoutNs;
   a.tripStep = br->tripStep;
+  a.prof = br->profiling ? br->d_phase : nullptr;
+  a.dbg = br->d_dbg;
+  a.barBase = R.barBase;
+  CU(launch_window(a, br->sms, R.smem, br->stream));
+  R.barBase += (uint32_t)br->sms * (uint32_t)(a.nWin * (a.anyBg ? 3 : 2) - 1);  // arrivals of the launch
+  R.logValid = true;
+  R.ringValid = false;
+  return FB_OK;
+}
+
+// steps[b] steps of every brain through the windowed kernel: the log holds the spikes in flight,
+// the steps after an irregular host write run one at a time, logged launches are recorded a window
+// at a time.
+static int run_window(fb_brains *br, int32_t maxSteps, bool forced) {
+  WinRes &R = br->win;
+  CU(cudaEventRecord(br->ev0, br->stream));
+  const bool backup = br->B == 1 && (forced || maxSteps >= kWinBackupSteps);
+  if (backup) {
+    int rc = ring_from_log(br);
+    if (rc) return rc;
+    const size_t st = 11 * align256((size_t)br->host[0].N * 4);
+    if (!R.backup && (rc = win_alloc(br, &R.backup, st + sizeof(Trial)))) return rc;
+    CU(cudaMemcpyAsync(R.backup, br->host[0].v, st, cudaMemcpyDeviceToDevice, br->stream));
+    CU(cudaMemcpyAsync(R.backup + st, br->trials, sizeof(Trial), cudaMemcpyDeviceToDevice, br->stream));
+  }
+  if (!R.logValid) {
+    CU(launch_log_import(br->trials, R.win, br->B, br->stream));
+    R.logValid = true;
+  }
+  std::vector<int32_t> left = br->stepsHost, part(br->B);
+  auto go = [&](int32_t most, int hCap) -> int {
+    for (int b = 0; b < br->B; b++) {
+      part[b] = std::min(left[b], most);
+      left[b] -= part[b];
+    }
+    return win_launch(br, part, hCap);
+  };
+  int32_t done = 0;
+  while (done < maxSteps) {
+    const bool slow = br->irregular > 0;
+    int32_t n = slow ? std::min(br->irregular, maxSteps - done) : maxSteps - done;
+    if (br->logging) n = std::min(n, (int32_t)window_steps(br->host[0], (int64_t)br->driven[0].order.size()));
+    if (done) CU(cudaStreamSynchronize(br->stream));  // the pinned step counts are free again
+    int rc = go(n, slow ? 1 : kWinMax);
+    if (rc) return rc;
+    br->tripStep = br->tripStep >= n ? br->tripStep - n : -1;
+    if (br->logging) CU(launch_log_record(br->trials, R.win, n, br->stream));
+    if (slow) br->irregular -= n;
+    done += n;
+  }
   br->tripStep = -1;  // one launch only
-  CU(launch_lagged(a, R.grid, R.smem, br->stream));
-  CU(launch_rebuild_slots(br->trials, T.nslots, br->d_err, br->stream));
   CU(cudaEventRecord(br->ev1, br->stream));
   br->lastSchedule = FB_SCHEDULE_LAGGED;
+  return FB_OK;
+}
+
+// After a windowed launch that failed: its scratch cleared, and either the brain as it was (one
+// brain, backed up) or its spikes in flight dropped.
+static int win_recover(fb_brains *br, bool backup) {
+  WinRes &R = br->win;
+  CU(cudaMemsetAsync(R.sync, 0, 256 * 4, br->stream));
+  R.barBase = 0;
+  for (int b = 0; b < br->B; b++) {
+    const Trial &T = br->host[b];
+    const WinBrain &W = R.host[b];
+    CU(cudaMemcpyAsync(W.wcnt, W.inOff, (size_t)T.N * 4, cudaMemcpyDeviceToDevice, br->stream));
+    CU(cudaMemsetAsync(W.bgMask, 0, (size_t)T.N * 4, br->stream));
+    CU(cudaMemsetAsync(W.arr, 0, (size_t)T.N, br->stream));
+    if (W.bgHit) CU(cudaMemsetAsync(W.bgHit, 0, (size_t)T.N * std::min(T.nslots - 1, kWinMax) * 4, br->stream));
+    CU(cudaMemsetAsync(&R.win[b].fDone, 0, 4, br->stream));
+    if (!backup) CU(cudaMemsetAsync(T.ringCount, 0, (size_t)T.nslots * 4, br->stream));
+  }
+  if (backup) {
+    const size_t st = 11 * align256((size_t)br->host[0].N * 4);
+    CU(cudaMemcpyAsync(br->host[0].v, R.backup, st, cudaMemcpyDeviceToDevice, br->stream));
+    CU(cudaMemcpyAsync(br->trials, R.backup + st, sizeof(Trial), cudaMemcpyDeviceToDevice, br->stream));
+  }
+  R.ringValid = true;
+  R.logValid = false;
+  CU(cudaStreamSynchronize(br->stream));
   return FB_OK;
 }
 
 static int run_steps(fb_brains *br, int32_t maxSteps, int32_t *out_nfired) {
   int rc = flush(br, false);
   if (rc) return rc;
-  bool lagged = false;
+  bool windowed = false;
   if (maxSteps > 0 && br->schedule != FB_SCHEDULE_GRID) {
-    const char *why = nullptr;
-    const bool applies = lag_applies(br, maxSteps, &why);
+    const bool may = br->schedule == FB_SCHEDULE_AUTO && maxSteps >= win_min_steps(br) && !br->profiling &&
+                     (!br->logging || (br->B == 1 && maxSteps <= kWinLogSteps)) && !br->win.noMemory;
     if (br->schedule == FB_SCHEDULE_LAGGED) {
-      if (!applies) return fail(FB_EINVAL, "fb_step: the delay-scheduled kernel does not apply to %s", why);
-      if ((rc = lag_setup(br))) return rc;
-      lagged = true;
-    } else if (applies && maxSteps >= kLagMinSteps) {
-      lagged = lag_setup(br) == FB_OK;
-      if (!lagged) g_err.clear();
+      const char *why = nullptr;
+      if (!lag_applies(br, maxSteps, &why)) return fail(FB_EINVAL, "fb_step: the delay-scheduled kernel does not apply to %s", why);
+      if (win_capable(br)) {
+        if ((rc = win_setup(br))) return rc;
+        windowed = true;
+      }
+    } else if (may && win_capable(br)) {
+      windowed = win_setup(br) == FB_OK;
+      if (!windowed) g_err.clear();
     }
   }
   // the error flag and the fired counts come back in one synchronisation
@@ -1195,19 +1345,27 @@ static int run_steps(fb_brains *br, int32_t maxSteps, int32_t *out_nfired) {
     br->flushPending = false;
     return FB_OK;
   };
-  if (lagged) {
-    if ((rc = run_lagged(br, maxSteps))) return rc;
+  if (windowed) {
+    const bool forced = br->schedule == FB_SCHEDULE_LAGGED;
+    if ((rc = run_window(br, maxSteps, forced))) return rc;
     if ((rc = read_back())) return rc;
     const int32_t err = br->h_small[0];
     cudaEventElapsedTime(&br->lastMs, br->ev0, br->ev1);
     if (err) {
       cudaMemsetAsync(br->d_err, 0, 4, br->stream);
-      cudaStreamSynchronize(br->stream);
+      win_recover(br, br->B == 1 && (forced || maxSteps >= kWinBackupSteps));
       return fail(err, err == FB_ETIMEOUT ? "fb_step: a device-side wait timed out; the step was abandoned"
-                                          : "fb_step: delay-scheduled kernel error %d", err);
+                                          : "fb_step: windowed kernel error %d", err);
     }
   } else if (maxSteps > 0) {
     br->lastSchedule = FB_SCHEDULE_GRID;
+    if (br->win.ready && !br->win.ringValid) {
+      if ((rc = ring_from_log(br))) return rc;
+      CU(launch_rebuild_slots(br->trials, br->B, br->maxSlots, br->d_err, br->stream));
+    }
+    br->win.logValid = false;
+    br->everGrid = true;
+    br->irregular = std::max(0, br->irregular - maxSteps);
     if (br->stepsUploaded != br->stepsHost) {  // the last launch's counts stay on the device otherwise
       std::memcpy(br->h_steps, br->stepsHost.data(), sizeof(int32_t) * br->B);
       CU(cudaMemcpyAsync(br->d_steps, br->h_steps, sizeof(int32_t) * br->B, cudaMemcpyHostToDevice, br->stream));
@@ -1357,6 +1515,10 @@ extern "C" int fb_fired(fb_brains *br, int32_t b, int32_t *dst, int32_t cap, int
   const int32_t m = std::min(nf_slot[0], cap);
   if (dst && m > 0) {
     const Trial &T = br->host[b];
+    if (br->win.ready && !br->win.ringValid) {  // the last step's list, in order, from the log
+      CU(launch_log_export(br->trials, br->win.win, b, b + 1, 1, true, br->stream));
+      CU(cudaStreamSynchronize(br->stream));
+    }
     CU(cudaMemcpy(dst, T.ring + (int64_t)nf_slot[1] * T.N, sizeof(int32_t) * m, cudaMemcpyDefault));
   }
   return FB_OK;
@@ -1367,6 +1529,7 @@ extern "C" int fb_ring_read(fb_brains *br, int32_t b, int32_t *ring, int32_t *co
   if (rc) return rc;
   rc = flush(br);
   if (rc) return rc;
+  if ((rc = ring_from_log(br))) return rc;
   CU(cudaStreamSynchronize(br->stream));
   const Trial &T = br->host[b];
   if (ring) CU(cudaMemcpy(ring, T.ring, sizeof(int32_t) * (size_t)T.nslots * T.N, cudaMemcpyDefault));
@@ -1412,6 +1575,7 @@ extern "C" int fb_write(fb_brains *br, int32_t field, int32_t b, const void *src
   if (field == FB_FIELD_DRIVE) return fail(FB_EINVAL, "fb_write: the drive field is written through fb_set_drive, which keeps the driven set");
   rc = flush(br);
   if (rc) return rc;
+  if (field == FB_FIELD_REFR) br->irregular = std::max(br->irregular, br->host[b].nslots - 1);
   const int32_t clear = field == FB_FIELD_ADAPT ? kAdaptZero : field == FB_FIELD_RES ? kResRest
                         : field == FB_FIELD_BIAS ? kBiasZero : field == FB_FIELD_THR ? kThrZero : 0;
   if (br->host[b].flags & clear) {  // the field may no longer be at rest: the update reads it again

@@ -31,7 +31,7 @@ namespace fb {
 int step_kernel_blocks_per_sm(size_t smem);
 size_t step_smem_bytes(int B);
 cudaError_t launch_step(const StepArgs &a, int grid, size_t smem, cudaStream_t st);
-cudaError_t launch_rebuild_slots(Trial *Td, int nslots, int32_t *err, cudaStream_t st);
+cudaError_t launch_rebuild_slots(Trial *Td, int B, int nslots, int32_t *err, cudaStream_t st);
 void host_jump_tables(std::vector<uint32_t> &tab);
 int set_error(int code, const char *msg);
 }  // namespace fb
@@ -268,7 +268,7 @@ extern "C" int fb_lif_step_noalloc(fb_brain_view *v, int32_t nsteps, void *strea
   if (verr)
     return fail_na(FB_EINVAL, "fb_lif_step_noalloc: the view's indptr, indices, driven list or ring lists hold an "
                    "index outside [0, N) (or indptr does not run from 0 to E); nothing was changed");
-  NA_CU(launch_rebuild_slots(Td, v->nslots, errd, st));
+  NA_CU(launch_rebuild_slots(Td, 1, v->nslots, errd, st));
 
   StepArgs a;
   memset(&a, 0, sizeof a);

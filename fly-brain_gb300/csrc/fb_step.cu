@@ -842,11 +842,12 @@ __global__ void reset_kernel(Trial *trials, int32_t b0, int32_t b1) {
 }
 
 // Rebuilds, for every ring slot, the per-arrival edge offsets and row starts, the slot's edge
-// total and its delivery work-item records from the caller's ring lists (one block per slot).
+// total and its delivery work-item records from its list (one block per slot and brain).
 __global__ void rebuild_slots_kernel(Trial *Tp, int32_t *err) {
   __shared__ uint32_t scan[33];
-  const Trial &T = *Tp;
+  const Trial &T = Tp[blockIdx.y];
   const int slot = blockIdx.x, tid = threadIdx.x;
+  if (slot >= T.nslots) return;
   const int N = T.N;
   const int32_t na = T.ringCount[slot];
   if (na < 0 || na > N) {
@@ -936,8 +937,8 @@ cudaError_t launch_deltas(Trial *trials, const Delta *d, const int32_t *gs, int3
 }
 
 
-cudaError_t launch_rebuild_slots(Trial *Td, int nslots, int32_t *err, cudaStream_t st) {
-  rebuild_slots_kernel<<<nslots, kBlock, 0, st>>>(Td, err);
+cudaError_t launch_rebuild_slots(Trial *Td, int B, int nslots, int32_t *err, cudaStream_t st) {
+  rebuild_slots_kernel<<<dim3(nslots, B), kBlock, 0, st>>>(Td, err);
   return cudaGetLastError();
 }
 

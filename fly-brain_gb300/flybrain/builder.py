@@ -17,7 +17,7 @@ CSRC = os.path.join(ROOT, "csrc")
 OUT_DIR = os.path.join(PKG, "_lib")
 LIB = os.path.join(OUT_DIR, "libflybrain.so")
 CHECK_LIB = os.path.join(OUT_DIR, "libflybrain_check.so")
-SOURCES = ["fb_step.cu", "fb_api.cu", "fb_graph.cu", "fb_noalloc.cu", "fb_adjoint.cu", "fb_lagged.cu", "fb_flyvis.cu", "fb_codec.cu"]
+SOURCES = ["fb_step.cu", "fb_api.cu", "fb_graph.cu", "fb_noalloc.cu", "fb_adjoint.cu", "fb_window.cu", "fb_window_narrow.cu", "fb_flyvis.cu", "fb_codec.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2", "--fmad=false"]
 
@@ -45,6 +45,7 @@ def build(verbose: bool = False, force: bool = False, checked: bool = False) -> 
     flags = FLAGS + (["-DFB_CHECK"] if checked else [])
     os.makedirs(obj_dir, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
+    headers.append(os.path.join(CSRC, "fb_window.cu"))  # fb_window_narrow.cu includes it
     headers.append(os.path.join(os.path.dirname(ROOT), "include", "flybrain.h"))
     cc = nvcc()
     srcs = [s for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
