@@ -129,6 +129,14 @@ struct DiffDev {
   const int32_t *roMap;  // neuron -> readout column, -1 elsewhere (per-step dL)
   int32_t *nonfinite;    // counts of non-finite log-gain [0] and drive [1] gradients
   uint32_t ovfCap, pad0;
+  // windows (fb_adjoint_window.cuh): end of each target's contributions and the contributions
+  // (regions by in-degree), 1 + the window step of a neuron's own arrival and forced spike; the
+  // conductance adjoints after each of a window's steps, the step lres was last brought to
+  uint32_t *wCnt;
+  uint4 *wBuf;
+  uint8_t *wArr, *wForced;
+  float *wE, *wI;
+  int32_t *wResT;
   int32_t *err;
   const uint32_t *jump;
 };
@@ -1046,6 +1054,10 @@ __global__ void __launch_bounds__(kDB, 2) k_barrival(const DiffDev *Ds, DP<R> P,
   }
 }
 
+}  // namespace fb
+#include "fb_adjoint_window.cuh"
+namespace fb {
+
 // Per instance, kRB blocks of fixed-order partial sums: the seven per-neuron accumulators
 // (W EI V Kc La A D), the sizeAlpha term through inScale (src/lifdiff.js:650-655, 676-680:
 // gInScale[q] summed over q's in-edges in edge order) and the inhibitory-gain term.
@@ -1183,7 +1195,8 @@ struct Inst {
   float *sizeLogSrc = nullptr, *inScaleSrc = nullptr;
   uint8_t *sensory = nullptr;
   int group = 0;
-  int64_t ckptCap = 0, tStepsCap = 0, dLcap = 0, resAtCap = 0, arenaRows = 0;
+  int64_t ckptCap = 0, tStepsCap = 0, dLcap = 0, resAtCap = 0, arenaRows = 0, histRows = 0;
+  bool windowClear = false;
   int32_t recordedSteps = 0;
   float *dLbuf = nullptr;
   int32_t *roMap = nullptr;
@@ -1590,6 +1603,7 @@ int check_err(fb_diff_batch *b, const char *fn) {
   DCU(cudaStreamSynchronize(b->st));
   if (err) {
     cudaMemset(b->err, 0, 4);
+    for (Inst &I : b->in) I.windowClear = false;
     return dfail(err, "%s: %s", fn, err == FB_EOVERFLOW ? "tape or delivery scratch overflow" : "device error");
   }
   return FB_OK;
@@ -1740,6 +1754,84 @@ void reverse_step(fb_diff_batch *b, cudaStream_t st, int32_t t, int32_t row, int
     k_bneuron<double><<<neuron_grid(b), kDB, 0, st>>>(b->dDevs, b->P64, t, row, scored);
     k_barrival<double><<<arrival_grid(b), kDB, 0, st>>>(b->dDevs, b->P64, t, row);
   }
+}
+
+// Steps per window of the current parameters (0: step by step). The windows need hard spikes, a
+// neuron that stays silent for a window after a spike, and a delay of a window; three steps and
+// more repay the two passes over the neurons' inputs that a window costs.
+constexpr int kWindowMin = 3;
+template <typename R>
+int silent_steps(const DP<R> &P, float refr) {
+  int k = 0;
+  for (; refr > 0 && k < kWindowMax; k++) refr = (float)((R)refr - P.dt);
+  return k;
+}
+template <typename R>
+int window_steps_t(const fb_diff_batch *b, const DP<R> &P) {
+  const DiffDev &D = b->in[0].D;
+  if (D.soft || D.driveSoft) return 0;
+  const int s = std::min(silent_steps(P, (float)P.tRef), silent_steps(P, (float)((R)(float)(P.tRef + P.dt) - P.dt)));
+  const int h = std::min({s, D.nslots - 1, kWindowMax});
+  return h >= kWindowMin && b->maxN < (1 << 26) ? h : 0;
+}
+int window_steps(const fb_diff_batch *b) { return b->f32 ? window_steps_t(b, b->P32) : window_steps_t(b, b->P64); }
+
+// The windows' buffers of every instance; false where memory is short (the pass then goes step by
+// step).
+bool window_buffers(fb_diff_batch *b, int h) {
+  for (Inst &I : b->in) {
+    DiffDev &D = I.D;
+    if (!D.wCnt) {
+      uint8_t *raw = nullptr;
+      const size_t n4 = ((size_t)D.N * 4 + 255) / 256 * 256, n1 = ((size_t)D.N + 255) / 256 * 256;
+      if (!try_talloc(b, &raw, 2 * n4 + 2 * n1 + ((size_t)D.E * 16 + 255) / 256 * 256)) return false;
+      D.wBuf = (uint4 *)raw;
+      uint8_t *p = raw + ((size_t)D.E * 16 + 255) / 256 * 256;
+      D.wResT = (int32_t *)p;
+      D.wCnt = (uint32_t *)(p + n4);
+      D.wArr = p + 2 * n4;
+      D.wForced = D.wArr + n1;
+      I.windowClear = false;
+    }
+    if (!I.windowClear) {  // fresh, or what a failed pass left
+      const size_t n1 = ((size_t)D.N + 255) / 256 * 256;
+      if (cudaMemcpyAsync(D.wCnt, D.cscPtr, (size_t)D.N * 4, cudaMemcpyDeviceToDevice, b->st) != cudaSuccess ||
+          cudaMemsetAsync(D.wArr, 0, 2 * n1, b->st) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+      }
+      I.windowClear = true;
+    }
+    if (I.histRows < h) {
+      float *f = nullptr;
+      if (!try_talloc(b, &f, (size_t)2 * h * D.N)) return false;
+      D.wE = f;
+      D.wI = f + (size_t)h * D.N;
+      I.histRows = h;
+    }
+  }
+  return true;
+}
+
+template <typename R>
+void window_replay_t(fb_diff_batch *b, const DP<R> &P, int32_t t0, int32_t t1, int32_t row) {
+  k_wdeliver<R><<<arrival_grid(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, row, b->B == 1 ? 4 : 1);
+  if (b->in[0].D.coba) k_wreplay<R, false><<<neuron_grid(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, row);
+  else k_wreplay<R, true><<<neuron_grid(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, row);
+}
+void window_replay(fb_diff_batch *b, int32_t t0, int32_t t1, int32_t row) {
+  if (b->f32) window_replay_t<float>(b, b->P32, t0, t1, row);
+  else window_replay_t<double>(b, b->P64, t0, t1, row);
+}
+template <typename R>
+void window_reverse_t(fb_diff_batch *b, const DP<R> &P, cudaStream_t st, int32_t t0, int32_t t1, int32_t row, int32_t lossFrom) {
+  if (b->in[0].D.coba) k_wbneuron<R, false><<<neuron_grid(b), kDB, 0, st>>>(b->dDevs, P, t0, t1, row, lossFrom);
+  else k_wbneuron<R, true><<<neuron_grid(b), kDB, 0, st>>>(b->dDevs, P, t0, t1, row, lossFrom);
+  k_wbarrival<R><<<arrival_grid(b), kDB, 0, st>>>(b->dDevs, P, t0, t1, row);
+}
+void window_reverse(fb_diff_batch *b, cudaStream_t st, int32_t t0, int32_t t1, int32_t row, int32_t lossFrom) {
+  if (b->f32) window_reverse_t<float>(b, b->P32, st, t0, t1, row, lossFrom);
+  else window_reverse_t<double>(b, b->P64, st, t0, t1, row, lossFrom);
 }
 
 int set_readout(fb_diff_batch *b, Inst &I, int32_t nro, const int32_t *ro) {
@@ -2245,6 +2337,8 @@ extern "C" int fb_diff_batch_backward(fb_diff_batch *b, const float *const *dL, 
     }
     D.steps = (int32_t)steps;
   }
+  int win = window_steps(b);
+  if (win && !window_buffers(b, win)) win = 0;
   if ((rc = push_devs(b))) return rc;
   const dim3 ng = neuron_grid(b);
   k_zero_adjoint<<<ng, kDB, 0, b->st>>>(b->dDevs);
@@ -2254,7 +2348,7 @@ extern "C" int fb_diff_batch_backward(fb_diff_batch *b, const float *const *dL, 
   const int nseg = (steps + K - 1) / K;
   b->arenaBufs = bufs;
   PassKey key = pass_key(b, 'B');
-  key.add(steps).add(K).add(truncate).add(loss_from).add(bufs);
+  key.add(steps).add(K).add(truncate).add(loss_from).add(bufs).add(win).add(b->in[0].D.coba);
   // Segments are replayed on the main stream (one after another: they share the forward state)
   // and swept in reverse on the reverse stream (one after another: they share the adjoint
   // state). With two arena halves, segment sg's replay writes half sg & 1 and may run while the
@@ -2269,7 +2363,10 @@ extern "C" int fb_diff_batch_backward(fb_diff_batch *b, const float *const *dL, 
       // replay the segment from its checkpoint (src/lifdiff.js:390-464)
       if (bufs == 2 && sg + 2 < nseg) ev_wait(b, b->st, b->evRev[sg & 1]);
       k_ckpt<<<ng, kDB, 0, b->st>>>(b->dDevs, from, 0);
-      for (int32_t t = from; t < to; t++) run_step(b, t, 1, half + t - from);
+      if (win)
+        for (int32_t t = from; t < to; t += win) window_replay(b, t, std::min(to, t + win), half + t - from);
+      else
+        for (int32_t t = from; t < to; t++) run_step(b, t, 1, half + t - from);
       cudaStream_t rs = b->st;
       if (bufs == 2) {
         ev_record(b, b->evRep[sg & 1], b->st);
@@ -2277,14 +2374,24 @@ extern "C" int fb_diff_batch_backward(fb_diff_batch *b, const float *const *dL, 
         rs = b->rev;
       }
       // reverse sweep of the segment (src/lifdiff.js:540-667)
-      for (int32_t t = to - 1; t >= from; t--) {
+      for (int32_t t1 = to; win && t1 > from;) {
+        // a truncation restarts the adjoint before the window's first (latest) step, never inside
+        int32_t t0 = std::max(from, t1 - win);
+        if (truncate > 0) {
+          t0 = std::max(t0, (t1 - 1) / truncate * truncate);
+          if (t1 % truncate == 0) k_truncate<<<ng, kDB, 0, rs>>>(b->dDevs, t1 - 1, truncate);
+        }
+        window_reverse(b, rs, t0, t1, half + t0 - from, loss_from);
+        t1 = t0;
+      }
+      for (int32_t t = to - 1; !win && t >= from; t--) {
         if (truncate > 0) k_truncate<<<ng, kDB, 0, rs>>>(b->dDevs, t, truncate);
         reverse_step(b, rs, t, half + t - from, t >= loss_from ? 1 : 0);
       }
       if (bufs == 2) ev_record(b, b->evRev[sg & 1], b->rev);
     }
     if (steps > 0) {
-      join_side(b);
+      if (!win) join_side(b);
       if (bufs == 2) {
         ev_record(b, b->evRevJoin, b->rev);
         ev_wait(b, b->st, b->evRevJoin);

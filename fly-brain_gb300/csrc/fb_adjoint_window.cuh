@@ -1,0 +1,513 @@
+// The adjoint's replay and reverse sweep in windows of the synaptic delay (included by
+// fb_adjoint.cu). One launch of each kernel covers h steps instead of one:
+//
+//  - A spike arrives D = nslots - 1 steps after it is emitted, so with h <= D everything that
+//    arrives in steps [t0, t0 + h) is on the tape before them: one k_wdeliver pushes the window's
+//    contributions, one k_wupdate runs every neuron through the window with its state in registers.
+//  - In the reverse sweep the adjoint of a spike reaches the neuron's step D steps earlier: the
+//    window's h reverse neuron steps need only arrivals of later windows (k_wbneuron), and the
+//    window's arrivals only the conductance adjoints those steps leave (kept per step), so one
+//    k_wbarrival follows.
+// h is also at most the steps a neuron stays silent after a spike, so a neuron spikes, and its row
+// arrives, at most once in a window: a target's contributions fit in a region of its in-degree, and
+// every edge and presynaptic accumulator still has one writer per kernel, in time order. Hard
+// spikes only (a soft neuron spikes in every step); the per-step kernels run the rest.
+//
+// Arithmetic and its order are the per-step kernels'. What a step leaves for its reverse is less:
+// the integrated potential u instead of v, gE, gI (current-based), no adaptation where it is 0,
+// the spike in a bit of the mode -- 5 bytes per neuron and step instead of 21 in the current-based
+// float case. The res adjoint, which only its own arrivals read, decays when one does.
+#pragma once
+
+namespace fb {
+
+constexpr int kWSort = 8;          // contributions per target sorted in shared memory
+constexpr int kWindowMax = 31;     // steps per window (five key bits)
+constexpr uint32_t kWNone = 0xffffffffu;
+
+// A contribution: key {step << 27 | arrival rank << 1 | inhibitory}, edge, the amount (float bits,
+// or a double's two words).
+__device__ __forceinline__ bool w_before(const uint4 &p, const uint4 &q) { return p.x < q.x || (p.x == q.x && p.y < q.y); }
+
+// Sort in place by (key, edge), one warp: each lane counts the entries before its own (up to 4 of
+// them); longer lists by insertion, lane 0.
+__device__ __noinline__ void w_warp_sort(uint4 *e, uint32_t n) {
+  constexpr int kM = 4;
+  const uint32_t lane = threadIdx.x & 31u;
+  if (n > 32 * kM) {
+    if (lane == 0)
+      for (uint32_t gap = n / 2; gap > 0; gap /= 2)  // Shell sort
+        for (uint32_t u = gap; u < n; u++) {
+          const uint4 x = e[u];
+          uint32_t w = u;
+          while (w >= gap) {
+            const uint4 y = e[w - gap];
+            if (w_before(y, x)) break;
+            e[w] = y;
+            w -= gap;
+          }
+          e[w] = x;
+        }
+    __syncwarp();
+    return;
+  }
+  uint4 x[kM];
+  uint32_t rank[kM];
+#pragma unroll
+  for (int m = 0; m < kM; m++) {
+    const uint32_t k = lane + 32 * m;
+    x[m] = k < n ? e[k] : make_uint4(kWNone, kWNone, 0, 0);
+    rank[m] = 0;
+  }
+#pragma unroll
+  for (int g = 0; g < kM; g++) {
+    if (32u * g >= n) break;
+    for (int l = 0; l < 32; l++) {
+      uint4 y = x[g];
+      y.x = __shfl_sync(0xffffffffu, y.x, l);
+      y.y = __shfl_sync(0xffffffffu, y.y, l);
+#pragma unroll
+      for (int m = 0; m < kM; m++) rank[m] += w_before(y, x[m]);
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int m = 0; m < kM; m++)
+    if (lane + 32 * m < n) e[rank[m]] = x[m];
+  __syncwarp();
+}
+
+// A target's contributions of the window in order.
+struct WList {
+  const uint4 *p;
+  int stride;
+  uint32_t left;
+  uint4 c;  // the current one (key kWNone: none)
+};
+__device__ __forceinline__ void wl_next(WList &l) {
+  if (l.left) {
+    l.p += l.stride;
+    l.left--;
+    l.c = *l.p;
+  } else {
+    l.c.x = kWNone;
+  }
+}
+// Every lane its own target's; stage: this lane's column of shared memory (entries 32 apart).
+__device__ __forceinline__ WList wl_make(uint4 *e, uint32_t n, uint4 *stage) {
+  for (uint32_t big = __ballot_sync(0xffffffffu, n > (uint32_t)kWSort); big; big &= big - 1) {
+    const int src = __ffs(big) - 1;
+    uint4 *p = (uint4 *)__shfl_sync(0xffffffffu, (unsigned long long)e, src);
+    w_warp_sort(p, __shfl_sync(0xffffffffu, n, src));
+  }
+  WList l;
+  l.p = e;
+  l.stride = 1;
+  l.left = n ? n - 1 : 0;
+  l.c = make_uint4(kWNone, 0, 0, 0);
+  if (n > 1 && n <= (uint32_t)kWSort) {
+    for (uint32_t u = 0; u < n; u++) {
+      const uint4 x = e[u];
+      uint32_t w = u;
+      while (w > 0) {
+        const uint4 y = stage[(w - 1) * 32];
+        if (w_before(y, x)) break;
+        stage[w * 32] = y;
+        w--;
+      }
+      stage[w * 32] = x;
+    }
+    l.p = stage;
+    l.stride = 32;
+  }
+  if (n) l.c = *l.p;
+  return l;
+}
+
+// The instance's steps of window [t0, t1), and its arrivals: tape entries [a0, a1) with the first
+// entry of each emission step (off[k]: step e0 + k).
+struct WSpan {
+  int h, e0, ne;
+  int64_t a0, a1;
+};
+__device__ __forceinline__ WSpan w_span(const DiffDev &D, int t0, int t1, int64_t *off) {
+  WSpan s;
+  s.h = min(t1, D.steps) - t0;
+  const int d = D.nslots - 1;
+  s.e0 = max(0, t0 - d);
+  s.ne = s.h > 0 ? max(0, t0 + s.h - d - s.e0) : 0;
+  if (s.ne > 0 && (int)threadIdx.x <= s.ne) off[threadIdx.x] = min(D.tOff[s.e0 + threadIdx.x], D.tapeCap);
+  __syncthreads();
+  s.a0 = s.ne ? off[0] : 0;
+  s.a1 = s.ne ? off[s.ne] : 0;
+  return s;
+}
+__device__ __forceinline__ int w_step_of(const WSpan &s, const int64_t *off, int64_t a) {  // k with off[k] <= a < off[k+1]
+  int lo = 0, hi = s.ne;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (off[mid] <= a) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// Delivery of the window's arrivals (k_deliver for h steps), `parts` warps per arrival; in a replay
+// (row >= 0) also the forced spikes' marks from the tape. The amplitude's res is the window's first
+// one recovered to the arrival step.
+template <typename R>
+__global__ void __launch_bounds__(kDB, 4) k_wdeliver(const DiffDev *Ds, DP<R> P, int32_t t0, int32_t t1, int32_t row,
+                                                    int32_t parts) {
+  __shared__ DiffDev D;
+  __shared__ int64_t off[kWindowMax + 1];
+  load_dev(Ds, D);
+  const WSpan S = w_span(D, t0, t1, off);
+  if (S.h <= 0) return;
+  const bool ex = row < 0 && D.exact32;
+  const int lane = threadIdx.x & 31, d = D.nslots - 1;
+  const int64_t th = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (int64_t)gridDim.x * blockDim.x;
+  if (row >= 0)
+    for (int j = 0; j < S.h; j++) {
+      const int64_t base = D.tOff[t0 + j], nf = tape_count(D, base, base + D.tForced[t0 + j]);
+      for (int64_t k = th; k < nf; k += nth) D.wForced[D.tIdx[base + k]] = (uint8_t)(j + 1);
+    }
+  const int64_t work = (S.a1 - S.a0) * parts;
+  for (int64_t w = th >> 5; w < work; w += nth >> 5) {
+    const int64_t a = S.a0 + w / parts;
+    const int part = (int)(w % parts);
+    const int ek = w_step_of(S, off, a), j = S.e0 + ek + d - t0;
+    const uint32_t k = (uint32_t)(a - off[ek]);
+    const int32_t pre = D.tIdx[a];
+    const float sg = ex ? D.signW32[pre] : D.sign[pre];
+    float r = D.res[pre];
+    R eff = 0;
+    float sv = 0.f;
+    if (ex) {
+      for (int q = 0; q < j; q++) r = r + (1.f - r) * P.xkRec;
+      const float amp = D.tAmp[a];
+      sv = sg * r;
+      if (amp != 1.f) sv = sv * amp;
+      if (sv == 0.f) continue;
+    } else {
+      if (sg == 0) continue;
+      for (int q = 0; q < j; q++) r = (float)((R)r + (R(1) - (R)r) * P.kRec);
+      if (row >= 0 && part == 0 && lane == 0) D.resAt[(int64_t)(row + j) * D.maxArr + k] = r;
+      eff = (R)sg * P.wSyn * d_out<R>(D, pre) * exp((R)D.logGain[pre]) * (R)r * (R)D.tAmp[a];
+    }
+    if (part == 0 && lane == 0) D.wArr[pre] = (uint8_t)(j + 1);
+    const bool inh = ex ? !(sv > 0.f) : !(eff > 0);
+    const uint32_t key = ((uint32_t)j << 27) | (k << 1) | (inh ? 1u : 0u);
+    const uint32_t lo = D.indptr[pre], hi = D.indptr[pre + 1];
+    for (uint32_t j0 = lo + 32u * kEdgeILP * part + lane; j0 < hi; j0 += 32u * kEdgeILP * parts) {
+      bool on[kEdgeILP];
+      uint32_t q[kEdgeILP], pos[kEdgeILP];
+      uint4 c[kEdgeILP];
+#pragma unroll
+      for (int u = 0; u < kEdgeILP; u++) {
+        const uint32_t e = j0 + 32u * u;
+        on[u] = e < hi && D.gate[e];
+        if (!on[u]) continue;
+        q[u] = D.indices[e];
+        c[u] = make_uint4(key, e, 0u, 0u);
+        if (ex) {
+          const float dlt = D.W32[e] * sv;
+          on[u] = dlt != 0.f;
+          c[u].z = __float_as_uint(dlt);
+        } else if (sizeof(R) == 8) {
+          const R p = (R)D.P[e], x = inh ? p * P.inhGain * eff : p * eff;
+          const long long b = __double_as_longlong((double)x);
+          c[u].z = (uint32_t)b;
+          c[u].w = (uint32_t)(b >> 32);
+        } else {
+          const R p = (R)D.Pf[e];
+          c[u].z = __float_as_uint((float)(inh ? p * P.inhGain * eff : p * eff));
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kEdgeILP; u++)
+        if (on[u]) pos[u] = atomicAdd(D.wCnt + q[u], 1u);  // the counter starts at the target's region
+#pragma unroll
+      for (int u = 0; u < kEdgeILP; u++)
+        if (on[u] && (int64_t)pos[u] < D.E) D.wBuf[pos[u]] = c[u];
+    }
+  }
+}
+
+// Integrate and spike for the window (k_update for h steps), a neuron per lane. Replay: forced steps
+// from wForced, what the reverse needs into the arena. CUBA: current-based (u alone is kept).
+template <typename R, bool CUBA>
+__global__ void __launch_bounds__(kDB, 4) k_wreplay(const DiffDev *Ds, DP<R> P, int32_t t0, int32_t t1, int32_t row) {
+  __shared__ DiffDev D;
+  __shared__ uint4 stage[kDB / 32][kWSort * 32];
+  load_dev(Ds, D);
+  const int h = min(t1, D.steps) - t0;
+  if (h <= 0) return;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const int N = D.N, nW = (N + 31) / 32;
+  R *aU = (R *)D.aV;
+  const bool hasAd = P.adaptInc != 0;
+  for (int wt = blockIdx.x * (kDB / 32) + warp; wt < nW; wt += gridDim.x * (kDB / 32)) {
+    const int i0 = wt * 32 + (int)lane, i = i0 < N ? i0 : N - 1;
+    const bool own = i0 < N;
+    const uint32_t o = D.cscPtr[i], end = D.cscPtr[i + 1], cnt = D.wCnt[i];
+    float v = D.v[i], geF = D.gE[i], giF = D.gI[i], refr = D.refr[i], ad = D.adapt[i], res = D.res[i];
+    const float thrO = D.thrOffset[i];
+    const int arr = (int)D.wArr[i] - 1, frc = (int)D.wForced[i] - 1;
+    const R bias = d_bias<R>(D, P, i, nullptr), kc = d_kc<R>(D, P, i);
+    uint32_t n = own ? cnt - o : 0u;
+    if (n > end - o) {
+      atomicCAS(D.err, 0, FB_EOVERFLOW);
+      n = 0;
+    }
+    WList l = wl_make(D.wBuf + o, n, stage[warp] + lane);
+    __syncwarp();
+    for (int j = 0; j < h; j++) {
+      while ((l.c.x >> 27) == (uint32_t)j) {
+        const R x = sizeof(R) == 8 ? (R)__longlong_as_double((long long)(((unsigned long long)l.c.w << 32) | l.c.z))
+                                   : (R)__uint_as_float(l.c.z);
+        if (l.c.x & 1u) giF = (float)((R)giF + x);
+        else geF = (float)((R)geF + x);
+        wl_next(l);
+      }
+      if (arr == j) res = (float)((R)res - P.depU * (R)res);
+      int md = 0, s = 0;
+      if (frc == j) {
+        refr = (float)(P.tRef + P.dt);
+        ad = (float)((R)ad + P.adaptInc);
+      }
+      const R ge = geF, gi = giF;
+      const int64_t at = (int64_t)(row + j) * N + i;
+      R vi = v;
+      const bool wasRefr = refr > 0;
+      if (wasRefr) {
+        refr = (float)((R)refr - P.dt);
+        vi = P.vReset;
+        md = frc == j ? 2 : 1;
+      } else {
+        vi = d_u<R>(D, P, vi, ge, gi, bias);
+        if (own) {
+          if (CUBA) {
+            aU[at] = vi;
+          } else {
+            D.aV[at] = v;
+            D.aGE[at] = geF;
+            D.aGI[at] = giF;
+          }
+        }
+      }
+      geF = (float)(ge * P.dE);
+      giF = (float)(gi * P.dE);
+      ad = (float)((R)ad * P.dA);
+      res = (float)((R)res + (R(1) - (R)res) * P.kRec);
+      if (own && hasAd && !wasRefr) D.aAd[at] = ad;
+      if (!wasRefr) {
+        const R thr = P.vThresh + (R)ad + kc + (R)thrO;
+        if (vi >= thr) {
+          s = 1;
+          vi = R(1) * P.vReset + (R(1) - R(1)) * vi;
+          refr = (float)P.tRef;
+          ad = (float)((R)ad + R(1) * P.adaptInc);
+        }
+      }
+      if (own) D.aMode[at] = (uint8_t)(md | s << 2);
+      v = (float)vi;
+    }
+    if (!own) continue;
+    D.v[i] = v;
+    D.gE[i] = geF;
+    D.gI[i] = giF;
+    D.refr[i] = refr;
+    D.adapt[i] = ad;
+    D.res[i] = res;
+    if (n) D.wCnt[i] = o;
+    if (arr >= 0) D.wArr[i] = 0;
+    if (frc >= 0) D.wForced[i] = 0;
+  }
+}
+
+// The reverse neuron pass of the window's steps, last first (bneuron for h steps), a neuron per
+// lane; the conductance adjoints after each step go to wE / wI for the window's arrivals.
+template <typename R, bool CUBA>
+__global__ void __launch_bounds__(kDB, 3) k_wbneuron(const DiffDev *Ds, DP<R> P, int32_t t0, int32_t t1, int32_t row,
+                                                    int32_t lossFrom) {
+  __shared__ DiffDev D;
+  load_dev(Ds, D);
+  const int h = min(t1, D.steps) - t0;
+  if (h <= 0) return;
+  const int N = D.N;
+  const R *aU = (const R *)D.aV;
+  const bool hasAd = P.adaptInc != 0;
+  const R c = P.adjClip;
+  auto cl = [c](float x) { return c > 0 ? (float)((R)x > c ? c : ((R)x < -c ? -c : (R)x)) : x; };
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+    float lv = D.lv[i], lgE = D.lgE[i], lgI = D.lgI[i], lad = D.lad[i];
+    double accA = D.accA[i], accV = D.accV[i], gB = D.gBias[i];
+    const bool masked = D.thrMask && D.thrMask[i];
+    double accKc = masked ? D.accKc[i] : 0.0, accEI = CUBA ? 0.0 : D.accEI[i];
+    R lam;
+    const R bias = d_bias<R>(D, P, i, &lam), kc = d_kc<R>(D, P, i), beta = d_beta<R>(D, P, i);
+    double accLa = lam != 0 ? D.accLa[i] : 0.0;
+    const float thrO = D.thrOffset[i];
+    const int ro = D.dL && D.roMap ? D.roMap[i] : -1;
+    const int slotD = D.gDrive ? D.dSlot[i] : -1;
+    for (int j = h - 1; j >= 0; j--) {
+      const int t = t0 + j;
+      const int64_t at = (int64_t)(row + j) * N + i;
+      const int m = D.aMode[at], md = m & 3;
+      const R lpA = lad;
+      const R lE = (R)lgE * P.dE, lI = (R)lgI * P.dE, lA = lpA * P.dA;
+      float lgEF = (float)lE, lgIF = (float)lI, ladF = (float)lA;
+      if (md == 1) {
+        lv = 0.f;
+      } else {
+        float *ls = D.lsRing + (int64_t)(t % D.nslots) * N + i;
+        const float lsv = *ls;
+        R dl = 0;
+        if (t >= lossFrom && D.dL) dl = D.roMap ? (ro >= 0 ? D.dL[(int64_t)t * D.nro + ro] : 0.f) : D.dL[i];
+        float *gDrv = slotD >= 0 ? D.gDrive + (int64_t)(t / D.driveEpoch) * D.nDS + slotD : nullptr;
+        if (__float_as_uint(lsv) != 0u) *ls = 0.f;
+        if (md == 2) {
+          accA = accA + (double)lA;
+          if (gDrv) *gDrv = (float)((R)*gDrv + (lA * P.adaptInc + ((R)lsv + dl)) * P.dtS);
+          lv = 0.f;
+        } else {
+          R vv = 0, gEv = 0, gIv = 0, uu;
+          if (CUBA) {
+            uu = aU[at];
+          } else {
+            vv = D.aV[at];
+            gEv = D.aGE[at];
+            gIv = D.aGI[at];
+            uu = d_u<R>(D, P, vv, gEv, gIv, bias);
+          }
+          const R thr = P.vThresh + (R)(hasAd ? D.aAd[at] : 0.f) + kc + (R)thrO;
+          const R d = uu - thr;
+          const R s = (m & 4) ? R(1) : R(0);
+          const R tt = R(1) + fabs(d) / beta;
+          const R sg = R(1) / (beta * tt * tt);
+          const R lspike = (R)lsv + dl;
+          const R lvNew = lv;
+          const R lsTot = (P.vReset - uu) * lvNew + lpA * P.adaptInc + lspike;
+          const R lt = lsTot * (R(1) - R(0)) * sg;
+          const R lu = lvNew * (R(1) - s) + lt;
+          const R lthr = -lt;
+          if (gDrv) *gDrv = (float)((R)*gDrv + lsTot * (R(1) - s) * P.dtS);
+          accA = accA + (double)(lpA * s);
+          accV = accV + (double)lthr;
+          if (masked) accKc += (double)lthr;
+          ladF = (float)(lA + lthr * P.dA);
+          if (CUBA) {
+            lv = (float)(lu * (R(1) - P.kM));
+            lgEF = (float)(lE + lu * P.kM);
+            lgIF = (float)(lI + lu * P.kM);
+          } else {
+            lv = (float)(lu * (R(1) + P.kM * (R(-1) - gEv * P.cE + gIv * P.cI)));
+            lgEF = (float)(lE + lu * P.kM * (P.eExc - vv) * P.cE);
+            lgIF = (float)(lI + lu * P.kM * (vv - P.eInh) * P.cI);
+            accEI += (double)(lu * P.kM * gIv * P.cI * (R(-1) + (vv - P.eInh) * P.cI));
+          }
+          if (lam != 0) accLa += (double)(lu * P.kM);
+          gB = gB + (double)(lu * P.kM);
+        }
+      }
+      lv = cl(lv);
+      lgE = cl(lgEF);
+      lgI = cl(lgIF);
+      lad = cl(ladF);
+      D.wE[(int64_t)j * N + i] = lgE;
+      D.wI[(int64_t)j * N + i] = lgI;
+    }
+    D.lv[i] = lv;
+    D.lgE[i] = lgE;
+    D.lgI[i] = lgI;
+    D.lad[i] = lad;
+    D.accA[i] = accA;
+    D.accV[i] = accV;
+    D.gBias[i] = gB;
+    if (masked) D.accKc[i] = accKc;
+    if (!CUBA) D.accEI[i] = accEI;
+    if (lam != 0) D.accLa[i] = accLa;
+  }
+}
+
+// Reverse of the window's deliveries (k_barrival for h steps), warp per arrival.
+template <typename R>
+__global__ void __launch_bounds__(kDB, 2) k_wbarrival(const DiffDev *Ds, DP<R> P, int32_t t0, int32_t t1, int32_t row) {
+  __shared__ DiffDev D;
+  __shared__ int64_t off[kWindowMax + 1];
+  load_dev(Ds, D);
+  const WSpan S = w_span(D, t0, t1, off);
+  if (S.h <= 0) return;
+  const int lane = threadIdx.x & 31, dd = D.nslots - 1;
+  const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t a = S.a0 + w0; a < S.a1; a += nw) {
+    const int ek = w_step_of(S, off, a), e = S.e0 + ek, t = e + dd, j = t - t0;
+    const int32_t pre = D.tIdx[a];
+    const R sgn = D.sign[pre];
+    if (sgn == 0) continue;
+    const R amp = D.tAmp[a];
+    const R resAtv = D.resAt[(int64_t)(row + j) * D.maxArr + (a - off[ek])];
+    const R gain = exp((R)D.logGain[pre]) * d_out<R>(D, pre);
+    const R base = sgn * P.wSyn * gain * resAtv;
+    const R eff = base * amp;
+    const bool exc = eff > 0;
+    const float *lg0 = (exc ? D.wE : D.wI) + (int64_t)j * D.N;
+    const uint32_t lo = D.indptr[pre], hi = D.indptr[pre + 1];
+    R lraw = 0;
+    for (uint32_t j0 = lo + lane; j0 < hi; j0 += 32 * kEdgeILP) {
+      bool on[kEdgeILP];
+      uint32_t q[kEdgeILP];
+      float cnt[kEdgeILP], eg[kEdgeILP], lgv[kEdgeILP], ins[kEdgeILP];
+      double old[kEdgeILP];
+#pragma unroll
+      for (int u = 0; u < kEdgeILP; u++) {
+        const uint32_t ed = j0 + 32u * u;
+        on[u] = ed < hi && D.gate[ed];
+        if (on[u]) {
+          q[u] = D.indices[ed];
+          cnt[u] = D.counts[ed];
+          eg[u] = D.edgeGain ? D.edgeGain[ed] : 1.f;
+          old[u] = D.gEdge[ed];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kEdgeILP; u++) {
+        if (on[u]) {
+          lgv[u] = lg0[q[u]];
+          ins[u] = D.inScale[q[u]];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kEdgeILP; u++) {
+        if (on[u]) {
+          const R lg = lgv[u];
+          const R cw = (R)cnt[u] * (R)eg[u];
+          lraw += exc ? lg * cw * (R)ins[u] : lg * cw * (R)ins[u] * P.inhGain;
+          D.gEdge[j0 + 32u * u] = old[u] + (double)(lg * eff);
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) lraw += __shfl_xor_sync(0xffffffffu, lraw, o);
+    if (lane == 0) {
+      float *target = D.lsRing + (int64_t)(e % D.nslots) * D.N;
+      D.accW[pre] += (double)(lraw * sgn * gain * resAtv * amp);
+      D.gLog[pre] += (double)(lraw * eff);
+      float x = (float)((R)target[pre] + lraw * base);
+      if (P.adjClip > 0) x = (float)fmin(P.adjClip, fmax(-P.adjClip, (R)x));
+      target[pre] = x;
+      // the res adjoint decays once per step down to this one (its clip bounds what an arrival left)
+      float lr = D.lres[pre];
+      if (lr != 0.f)
+        for (int s = D.wResT[pre] - t; s > 0; s--) lr = (float)((R)lr * (R(1) - P.kRec));
+      const R lresAfter = lr;
+      D.accD[pre] += (double)(-lresAfter * resAtv);
+      float y = (float)(lresAfter * (R(1) - P.depU) + lraw * sgn * P.wSyn * gain * amp);
+      if (P.adjClip > 0) y = (float)fmin(P.adjClip, fmax(-P.adjClip, (R)y));
+      D.lres[pre] = y;
+      D.wResT[pre] = t;
+    }
+  }
+}
+
+}  // namespace fb

@@ -1,0 +1,60 @@
+"""The adjoint's windowed kernels (fly-brain_gb300/csrc/fb_adjoint_window.cuh) where their parts meet
+their limits, against the oracle's restatement of LIFDiff: checkpoint intervals, truncations and lengths that do
+not divide a window; targets with more contributions than a lane (8) or a warp (128) sorts; both
+membrane models; refractory times below the three steps a window needs. Tape and spike counts
+identical, gradients within the tolerance of tests/test_adjoint_gpu.py (the same arithmetic)."""
+import numpy as np
+import pytest
+
+from test_adjoint_gpu import _compare_grads, _pair
+
+pytestmark = pytest.mark.gpu
+
+
+def hub_net(N, hub, seed, deg=6):
+    rng = np.random.default_rng(seed)
+    rows = [np.unique(np.concatenate([np.arange(hub), rng.integers(0, N, deg)])) for _ in range(N)]
+    indptr = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.uint32)
+    idx = np.concatenate(rows).astype(np.uint32)
+    return dict(N=N, indptr=indptr, indices=idx, counts=rng.integers(1, 9, idx.shape[0]).astype(np.float32),
+                sign=np.where(rng.random(N) < 0.7, 1.0, -1.0).astype(np.float32))
+
+
+CUBA = dict(dt=0.1, coba=False, soft=False, surrogateBeta=0.5, wSyn=0.2, minSyn=2.0, adjClip=50.0)
+COBA = dict(dt=0.1, coba=True, soft=False, surrogateBeta=2.0, wSyn=0.4, minSyn=2.0, adaptInc=0.4, depU=0.15, inhGain=1.3)
+
+
+@pytest.mark.parametrize("model", [CUBA, COBA])
+@pytest.mark.parametrize("N,hub,hz", [(60, 3, 900.0), (300, 4, 4000.0)])
+@pytest.mark.parametrize("K,truncate,steps", [(7, 0, 61), (18, 0, 90), (100, 23, 130), (16, 16, 64), (1, 0, 20)])
+def test_windows_match_oracle(model, N, hub, hz, K, truncate, steps):
+    ins = hub_net(N, hub, N)
+    rng = np.random.default_rng(3)
+    driven = rng.permutation(N)[: N * 3 // 4].astype(np.int32)
+    p = dict(model, checkpoint=K)
+    prob, net = _pair(ins, p, driven, np.full(driven.shape[0], hz))
+    sc0, tape = prob.forward(steps, seed=5, checkpoint=K)
+    sc1 = net.forward(steps, seed=5)
+    assert sc0.tobytes() == sc1.tobytes()
+    off, idx, amp = net.tape()
+    np.testing.assert_array_equal(off, tape["off"])
+    np.testing.assert_array_equal(idx, tape["idx"])
+    dL = rng.normal(0, 1, N).astype(np.float32)
+    g0 = prob.backward(tape, dL, truncate=truncate, lossFrom=steps // 3)
+    g1 = net.backward(dL, truncate=truncate, lossFrom=steps // 3)
+    _compare_grads(g0, g1)
+    assert np.abs(g1["edge"]).sum() > 0
+
+
+@pytest.mark.parametrize("tref", [0.05, 0.25, 0.45])
+def test_short_refractory_times(tref):
+    ins = hub_net(80, 2, 9)
+    driven = np.arange(0, 80, 2, dtype=np.int32)
+    p = dict(COBA, tRef=tref, checkpoint=10, vThresh=-50.0)
+    prob, net = _pair(ins, p, driven, np.full(40, 500.0))
+    sc0, tape = prob.forward(70, seed=2, checkpoint=10)
+    assert sc0.tobytes() == net.forward(70, seed=2).tobytes()
+    off, idx, _ = net.tape()
+    np.testing.assert_array_equal(idx, tape["idx"])
+    dL = np.ones(80, np.float32)
+    _compare_grads(prob.backward(tape, dL), net.backward(dL))
