@@ -137,6 +137,15 @@ struct DiffDev {
   uint8_t *wArr, *wForced;
   float *wE, *wI;
   int32_t *wResT;
+  // a forward's windows: places in the live drivenSet (N); per driven entry its live steps, 1 + the
+  // step of its own spike, its forced step, its adaptation at the window's start; spikes per step
+  // as bits [N / 32][32 steps], and their number
+  int32_t *wDrv;
+  uint32_t *wLive;
+  uint8_t *wOwn, *wFs;
+  float *wAd0;
+  uint32_t *wBits;
+  int32_t *wSpikes;
   int32_t *err;
   const uint32_t *jump;
 };
@@ -1250,6 +1259,7 @@ struct fb_diff_batch {
   DP<float> P32;
   int32_t *err = nullptr, *nonfinite = nullptr;
   uint32_t *jump = nullptr;
+  uint32_t *winJump = nullptr;  // window_jump_tables of the forward's chain
   double *partial = nullptr;
 };
 
@@ -1778,31 +1788,46 @@ int window_steps(const fb_diff_batch *b) { return b->f32 ? window_steps_t(b, b->
 
 // The windows' buffers of every instance; false where memory is short (the pass then goes step by
 // step).
-bool window_buffers(fb_diff_batch *b, int h) {
+bool window_buffers(fb_diff_batch *b, int h, bool back) {
   for (Inst &I : b->in) {
     DiffDev &D = I.D;
     if (!D.wCnt) {
       uint8_t *raw = nullptr;
       const size_t n4 = ((size_t)D.N * 4 + 255) / 256 * 256, n1 = ((size_t)D.N + 255) / 256 * 256;
-      if (!try_talloc(b, &raw, 2 * n4 + 2 * n1 + ((size_t)D.E * 16 + 255) / 256 * 256)) return false;
+      const size_t nb = ((size_t)D.N + 31) / 32 * 32 * 4 + 255 & ~(size_t)255;
+      if (!try_talloc(b, &raw, 5 * n4 + 4 * n1 + nb + 256 + ((size_t)D.E * 16 + 255) / 256 * 256)) return false;
       D.wBuf = (uint4 *)raw;
       uint8_t *p = raw + ((size_t)D.E * 16 + 255) / 256 * 256;
       D.wResT = (int32_t *)p;
       D.wCnt = (uint32_t *)(p + n4);
       D.wArr = p + 2 * n4;
       D.wForced = D.wArr + n1;
+      p += 2 * n4 + 2 * n1;
+      D.wBits = (uint32_t *)p;
+      p += nb;
+      D.wSpikes = (int32_t *)p;
+      p += 256;
+      D.wDrv = (int32_t *)p;
+      p += n4;
+      D.wLive = (uint32_t *)p;
+      p += n4;
+      D.wAd0 = (float *)p;
+      p += n4;
+      D.wOwn = p;
+      D.wFs = p + n1;
       I.windowClear = false;
     }
     if (!I.windowClear) {  // fresh, or what a failed pass left
       const size_t n1 = ((size_t)D.N + 255) / 256 * 256;
       if (cudaMemcpyAsync(D.wCnt, D.cscPtr, (size_t)D.N * 4, cudaMemcpyDeviceToDevice, b->st) != cudaSuccess ||
-          cudaMemsetAsync(D.wArr, 0, 2 * n1, b->st) != cudaSuccess) {
+          cudaMemsetAsync(D.wArr, 0, 2 * n1, b->st) != cudaSuccess ||
+          cudaMemsetAsync(D.wBits, 0, ((size_t)D.N + 31) / 32 * 32 * 4, b->st) != cudaSuccess) {
         cudaGetLastError();
         return false;
       }
       I.windowClear = true;
     }
-    if (I.histRows < h) {
+    if (I.histRows < h && back) {
       float *f = nullptr;
       if (!try_talloc(b, &f, (size_t)2 * h * D.N)) return false;
       D.wE = f;
@@ -1811,6 +1836,62 @@ bool window_buffers(fb_diff_batch *b, int h) {
     }
   }
   return true;
+}
+
+// Steps per window of a forward (0: step by step): no spike train, not exact32, the driven lists and
+// their draws of a window within a block's shared memory.
+int forward_window_steps(const fb_diff_batch *b, const fb_diff_params *p) {
+  int h = window_steps(b);
+  if (!h || p->exact32) return 0;
+  size_t n = 1;
+  bool sched = false;
+  for (const Inst &I : b->in) {
+    if (I.D.trainOff) return 0;
+    sched = sched || I.D.driveAt;
+    n = std::max(n, I.driven0.size() + (I.D.epOff ? I.driveIdx.size() : 0));
+  }
+  if (n > (size_t)kChainDriven) return 0;
+  h = std::min<int>(h, (int)((kWinStream) / n));
+  if (sched) h = std::min(h, b->in[0].D.driveEpoch);  // a window lies within an epoch
+  return h >= kWindowMin ? h : 0;
+}
+size_t chain_smem(const fb_diff_batch *b) {  // lane tables, 2 words per driven neuron, the draws
+  size_t n = 1;
+  for (const Inst &I : b->in) n = std::max(n, I.driven0.size() + I.driveIdx.size());
+  return (kWinJumpWords + 2 * std::min<size_t>(n, kChainDriven) + std::min<size_t>(kWinStream, n * kWindowMax) + 64) * 4;
+}
+int chain_setup(fb_diff_batch *b) {
+  const int bytes = (int)chain_smem(b);
+  DCU(cudaFuncSetAttribute(k_wchain<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((kWinJumpWords + 2 * kChainDriven + kWinStream + 64) * 4)));
+  DCU(cudaFuncSetAttribute(k_wchain<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((kWinJumpWords + 2 * kChainDriven + kWinStream + 64) * 4)));
+  (void)bytes;
+  if (!b->winJump) {
+    std::vector<uint32_t> tab(kWinJumpWords);
+    window_jump_tables(kChainThreads, tab.data());
+    int rc = talloc(b, &b->winJump, tab.size());
+    if (rc) return rc;
+    DCU(cudaMemcpy(b->winJump, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice));
+  }
+  return FB_OK;
+}
+
+// One window of a forward. The driven list's part runs on the side stream beside the other neurons;
+// the tape of the window follows both.
+template <typename R>
+void window_forward_t(fb_diff_batch *b, const DP<R> &P, int32_t t0, int32_t t1) {
+  k_wdeliver<R><<<arrival_grid(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, -1, b->B == 1 ? 4 : 1);
+  ev_record(b, b->evFork, b->st);
+  ev_wait(b, b->side, b->evFork);
+  k_wforward<R><<<dim3(b->B == 1 ? 64 : 8, b->B), kDB, 0, b->side>>>(b->dDevs, P, t0, t1, 1);
+  k_wchain<R><<<dim3(1, b->B), kChainThreads, chain_smem(b), b->side>>>(b->dDevs, P, t0, t1, b->winJump);
+  ev_record(b, b->evForced, b->side);
+  k_wforward<R><<<neuron_grid(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, 0);
+  ev_wait(b, b->st, b->evForced);
+  k_wemit<<<dim3(t1 - t0, b->B), 1024, 0, b->st>>>(b->dDevs, t0, t1);
+}
+void window_forward(fb_diff_batch *b, int32_t t0, int32_t t1) {
+  if (b->f32) window_forward_t<float>(b, b->P32, t0, t1);
+  else window_forward_t<double>(b, b->P64, t0, t1);
 }
 
 template <typename R>
@@ -2151,6 +2232,9 @@ extern "C" int fb_diff_batch_forward_ex(fb_diff_batch *b, const fb_diff_params *
   }
   bool edits = false;
   for (int k = 0; k < b->B; k++) edits = edits || b->in[k].D.epOff;
+  int win = forward_window_steps(b, p);
+  if (win && (!window_buffers(b, win, false))) win = 0;
+  if (win && (rc = chain_setup(b))) return rc;
   if ((rc = push_devs(b)) || (rc = prepare(b, p))) return rc;
   if (p->exact32) {
     k_prepare_w32<<<dim3(256, b->B), kDB, 0, b->st>>>(b->dDevs, p->wSyn, p->inhGain);
@@ -2160,9 +2244,27 @@ extern "C" int fb_diff_batch_forward_ex(fb_diff_batch *b, const fb_diff_params *
   const float vRest = (float)p->vRest;
   const int32_t ck = p->checkpoint;
   PassKey key = pass_key(b, 'F');
-  key.add(maxSteps).add(record).add(ck).add(edits).add(ep).add(vRest);
+  key.add(maxSteps).add(record).add(ck).add(edits).add(ep).add(vRest).add(win);
+  bool sched = false;
+  for (const Inst &I : b->in) sched = sched || I.D.driveAt;
+  key.add(sched);
   rc = run_pass(b, key, [&] {
     k_reset<<<neuron_grid(b), kDB, 0, b->st>>>(b->dDevs, vRest);
+    if (win) {
+      const dim3 pg(std::max(1, 304 / b->B), b->B);
+      for (int32_t t = 0, t1; t < maxSteps; t = t1) {
+        if (record && t % ck == 0) k_ckpt<<<neuron_grid(b), kDB, 0, b->st>>>(b->dDevs, t, 1);
+        if (edits && t % ep == 0) k_epoch<<<dim3(1, b->B), 1024, 0, b->st>>>(b->dDevs, t);
+        if (t == 0 || (edits && t % ep == 0))
+          for (int set = 0; set < 2; set++) k_wplaces<<<pg, kDB, 0, b->st>>>(b->dDevs, set);
+        // up to the next checkpoint and epoch
+        t1 = std::min(maxSteps, t + win);
+        if (record) t1 = std::min(t1, (t / ck + 1) * ck);
+        if (sched) t1 = std::min(t1, (t / ep + 1) * ep);
+        window_forward(b, t, t1);
+      }
+      return;
+    }
     for (int32_t t = 0; t < maxSteps; t++) {
       if (record && t % ck == 0) k_ckpt<<<neuron_grid(b), kDB, 0, b->st>>>(b->dDevs, t, 1);
       run_step(b, t, 0, -1, edits && t % ep == 0);
@@ -2338,7 +2440,7 @@ extern "C" int fb_diff_batch_backward(fb_diff_batch *b, const float *const *dL, 
     D.steps = (int32_t)steps;
   }
   int win = window_steps(b);
-  if (win && !window_buffers(b, win)) win = 0;
+  if (win && !window_buffers(b, win, true)) win = 0;
   if ((rc = push_devs(b))) return rc;
   const dim3 ng = neuron_grid(b);
   k_zero_adjoint<<<ng, kDB, 0, b->st>>>(b->dDevs);

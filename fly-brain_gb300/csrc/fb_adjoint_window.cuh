@@ -1,4 +1,4 @@
-// The adjoint's replay and reverse sweep in windows of the synaptic delay (included by
+// The adjoint's forward, replay and reverse sweep in windows of the synaptic delay (included by
 // fb_adjoint.cu). One launch of each kernel covers h steps instead of one:
 //
 //  - A spike arrives D = nslots - 1 steps after it is emitted, so with h <= D everything that
@@ -18,6 +18,7 @@
 // the spike in a bit of the mode -- 5 bytes per neuron and step instead of 21 in the current-based
 // float case. The res adjoint, which only its own arrivals read, decays when one does.
 #pragma once
+#include "fb_window.cuh"
 
 namespace fb {
 
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(kDB, 4) k_wdeliver(const DiffDev *Ds, DP<R> P,
   const bool ex = row < 0 && D.exact32;
   const int lane = threadIdx.x & 31, d = D.nslots - 1;
   const int64_t th = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (int64_t)gridDim.x * blockDim.x;
+  if (row < 0 && th < kWindowMax) D.wSpikes[th] = 0;  // a forward's spike counts of the window
   if (row >= 0)
     for (int j = 0; j < S.h; j++) {
       const int64_t base = D.tOff[t0 + j], nf = tape_count(D, base, base + D.tForced[t0 + j]);
@@ -233,8 +235,109 @@ __global__ void __launch_bounds__(kDB, 4) k_wdeliver(const DiffDev *Ds, DP<R> P,
   }
 }
 
-// Integrate and spike for the window (k_update for h steps), a neuron per lane. Replay: forced steps
-// from wForced, what the reverse needs into the arena. CUBA: current-based (u alone is kept).
+// A neuron's state and its window. REPLAY: its forced step `frc` comes from the tape, and what the
+// reverse needs goes to the arena (CUBA: current-based, u alone is kept); otherwise the window runs
+// without a forced spike, and the steps it is live in (not refractory, so that a driven neuron draws)
+// and the step it fires in (-1) are returned.
+struct WNeuron {
+  float v, ge, gi, refr, ad, res;
+};
+__device__ __forceinline__ WNeuron wn_load(const DiffDev &D, int i) {
+  WNeuron x;
+  x.v = D.v[i];
+  x.ge = D.gE[i];
+  x.gi = D.gI[i];
+  x.refr = D.refr[i];
+  x.ad = D.adapt[i];
+  x.res = D.res[i];
+  return x;
+}
+__device__ __forceinline__ void wn_store(const DiffDev &D, int i, const WNeuron &x) {
+  D.v[i] = x.v;
+  D.gE[i] = x.ge;
+  D.gI[i] = x.gi;
+  D.refr[i] = x.refr;
+  D.adapt[i] = x.ad;
+  D.res[i] = x.res;
+}
+template <typename R, bool REPLAY, bool CUBA>
+__device__ __forceinline__ int wn_run(const DiffDev &D, const DP<R> &P, int i, bool own, int h, int row, WNeuron &x, WList &l,
+                                      int arr, int frc, uint32_t *live) {
+  const int N = D.N;
+  const float thrO = D.thrOffset[i];
+  const R bias = d_bias<R>(D, P, i, nullptr), kc = d_kc<R>(D, P, i);
+  R *aU = (R *)D.aV;
+  const bool hasAd = P.adaptInc != 0;
+  int fired = -1;
+  for (int j = 0; j < h; j++) {
+    while ((l.c.x >> 27) == (uint32_t)j) {
+      const R c = sizeof(R) == 8 ? (R)__longlong_as_double((long long)(((unsigned long long)l.c.w << 32) | l.c.z))
+                                 : (R)__uint_as_float(l.c.z);
+      if (l.c.x & 1u) x.gi = (float)((R)x.gi + c);
+      else x.ge = (float)((R)x.ge + c);
+      wl_next(l);
+    }
+    if (arr == j) x.res = (float)((R)x.res - P.depU * (R)x.res);
+    if (REPLAY && frc == j) {
+      x.refr = (float)(P.tRef + P.dt);
+      x.ad = (float)((R)x.ad + P.adaptInc);
+    }
+    const R ge = x.ge, gi = x.gi;
+    const int64_t at = REPLAY ? (int64_t)(row + j) * N + i : 0;
+    R vi = x.v;
+    int md = 0, s = 0;
+    const bool wasRefr = x.refr > 0;
+    if (wasRefr) {
+      x.refr = (float)((R)x.refr - P.dt);
+      vi = P.vReset;
+      md = frc == j ? 2 : 1;
+    } else {
+      if (!REPLAY) *live |= 1u << j;
+      vi = d_u<R>(D, P, vi, ge, gi, bias);
+      if (REPLAY && own) {
+        if (CUBA) {
+          aU[at] = vi;
+        } else {
+          D.aV[at] = x.v;
+          D.aGE[at] = x.ge;
+          D.aGI[at] = x.gi;
+        }
+      }
+    }
+    x.ge = (float)(ge * P.dE);
+    x.gi = (float)(gi * P.dE);
+    x.ad = (float)((R)x.ad * P.dA);
+    x.res = (float)((R)x.res + (R(1) - (R)x.res) * P.kRec);
+    if (REPLAY && own && hasAd && !wasRefr) D.aAd[at] = x.ad;
+    if (!wasRefr) {
+      const R thr = P.vThresh + (R)x.ad + kc + (R)thrO;
+      if (vi >= thr) {
+        s = 1;
+        fired = j;
+        vi = R(1) * P.vReset + (R(1) - R(1)) * vi;
+        x.refr = (float)P.tRef;
+        x.ad = (float)((R)x.ad + R(1) * P.adaptInc);
+      }
+    }
+    if (REPLAY && own) D.aMode[at] = (uint8_t)(md | s << 2);
+    x.v = (float)vi;
+  }
+  return fired;
+}
+
+// The window's contributions of neuron i (none unless own).
+__device__ __forceinline__ uint32_t wn_count(const DiffDev &D, int i, bool own, uint32_t &o) {
+  o = D.cscPtr[i];
+  const uint32_t end = D.cscPtr[i + 1];
+  uint32_t n = own ? D.wCnt[i] - o : 0u;
+  if (n > end - o) {  // two spikes of one neuron in a window
+    atomicCAS(D.err, 0, FB_EOVERFLOW);
+    n = 0;
+  }
+  return n;
+}
+
+// Replay of the window (k_update for h steps of a replay), a neuron per lane.
 template <typename R, bool CUBA>
 __global__ void __launch_bounds__(kDB, 4) k_wreplay(const DiffDev *Ds, DP<R> P, int32_t t0, int32_t t1, int32_t row) {
   __shared__ DiffDev D;
@@ -244,85 +347,271 @@ __global__ void __launch_bounds__(kDB, 4) k_wreplay(const DiffDev *Ds, DP<R> P, 
   if (h <= 0) return;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const int N = D.N, nW = (N + 31) / 32;
-  R *aU = (R *)D.aV;
-  const bool hasAd = P.adaptInc != 0;
   for (int wt = blockIdx.x * (kDB / 32) + warp; wt < nW; wt += gridDim.x * (kDB / 32)) {
     const int i0 = wt * 32 + (int)lane, i = i0 < N ? i0 : N - 1;
     const bool own = i0 < N;
-    const uint32_t o = D.cscPtr[i], end = D.cscPtr[i + 1], cnt = D.wCnt[i];
-    float v = D.v[i], geF = D.gE[i], giF = D.gI[i], refr = D.refr[i], ad = D.adapt[i], res = D.res[i];
-    const float thrO = D.thrOffset[i];
+    uint32_t o;
+    WNeuron x = wn_load(D, i);
     const int arr = (int)D.wArr[i] - 1, frc = (int)D.wForced[i] - 1;
-    const R bias = d_bias<R>(D, P, i, nullptr), kc = d_kc<R>(D, P, i);
-    uint32_t n = own ? cnt - o : 0u;
-    if (n > end - o) {
-      atomicCAS(D.err, 0, FB_EOVERFLOW);
-      n = 0;
-    }
+    const uint32_t n = wn_count(D, i, own, o);
     WList l = wl_make(D.wBuf + o, n, stage[warp] + lane);
     __syncwarp();
-    for (int j = 0; j < h; j++) {
-      while ((l.c.x >> 27) == (uint32_t)j) {
-        const R x = sizeof(R) == 8 ? (R)__longlong_as_double((long long)(((unsigned long long)l.c.w << 32) | l.c.z))
-                                   : (R)__uint_as_float(l.c.z);
-        if (l.c.x & 1u) giF = (float)((R)giF + x);
-        else geF = (float)((R)geF + x);
-        wl_next(l);
-      }
-      if (arr == j) res = (float)((R)res - P.depU * (R)res);
-      int md = 0, s = 0;
-      if (frc == j) {
-        refr = (float)(P.tRef + P.dt);
-        ad = (float)((R)ad + P.adaptInc);
-      }
-      const R ge = geF, gi = giF;
-      const int64_t at = (int64_t)(row + j) * N + i;
-      R vi = v;
-      const bool wasRefr = refr > 0;
-      if (wasRefr) {
-        refr = (float)((R)refr - P.dt);
-        vi = P.vReset;
-        md = frc == j ? 2 : 1;
-      } else {
-        vi = d_u<R>(D, P, vi, ge, gi, bias);
-        if (own) {
-          if (CUBA) {
-            aU[at] = vi;
-          } else {
-            D.aV[at] = v;
-            D.aGE[at] = geF;
-            D.aGI[at] = giF;
-          }
-        }
-      }
-      geF = (float)(ge * P.dE);
-      giF = (float)(gi * P.dE);
-      ad = (float)((R)ad * P.dA);
-      res = (float)((R)res + (R(1) - (R)res) * P.kRec);
-      if (own && hasAd && !wasRefr) D.aAd[at] = ad;
-      if (!wasRefr) {
-        const R thr = P.vThresh + (R)ad + kc + (R)thrO;
-        if (vi >= thr) {
-          s = 1;
-          vi = R(1) * P.vReset + (R(1) - R(1)) * vi;
-          refr = (float)P.tRef;
-          ad = (float)((R)ad + R(1) * P.adaptInc);
-        }
-      }
-      if (own) D.aMode[at] = (uint8_t)(md | s << 2);
-      v = (float)vi;
-    }
+    wn_run<R, true, CUBA>(D, P, i, own, h, row, x, l, arr, frc, nullptr);
     if (!own) continue;
-    D.v[i] = v;
-    D.gE[i] = geF;
-    D.gI[i] = giF;
-    D.refr[i] = refr;
-    D.adapt[i] = ad;
-    D.res[i] = res;
+    wn_store(D, i, x);
     if (n) D.wCnt[i] = o;
     if (arr >= 0) D.wArr[i] = 0;
     if (frc >= 0) D.wForced[i] = 0;
   }
+}
+
+// ---- the forward ----------------------------------------------------------------------------------
+// As in the brain step's windows (fb_window.cu): the driven neurons first run the window as if
+// nothing were drawn for them (k_wforward, its driven part), one block per instance follows the chain
+// of draws (k_wchain), the other neurons run beside it (k_wforward), and the window's spikes go to
+// the tape from per-step bitmaps (k_wemit). A window lies within a checkpoint interval and a drive
+// epoch.
+
+// Places in the live drivenSet (wDrv, -1: not driven), at the start of a pass and after an epoch's edits.
+__global__ void k_wplaces(const DiffDev *Ds, int32_t set) {
+  __shared__ DiffDev D;
+  load_dev(Ds, D);
+  const int n = set ? *D.nLive : D.N;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    if (set) D.wDrv[D.drivenLive[k]] = k;
+    else D.wDrv[k] = -1;
+  }
+}
+
+// driven 0: the neurons that are not driven; 1: the driven list, without its draws.
+template <typename R>
+__global__ void __launch_bounds__(kDB, 4) k_wforward(const DiffDev *Ds, DP<R> P, int32_t t0, int32_t t1, int32_t driven) {
+  __shared__ DiffDev D;
+  __shared__ uint4 stage[kDB / 32][kWSort * 32];
+  load_dev(Ds, D);
+  const int h = min(t1, D.steps) - t0;
+  if (h <= 0) return;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const int M = driven ? *D.nLive : D.N, nW = (M + 31) / 32;
+  for (int wt = blockIdx.x * (kDB / 32) + warp; wt < nW; wt += gridDim.x * (kDB / 32)) {
+    const int k = wt * 32 + (int)lane, kk = k < M ? k : M - 1;
+    const int i = driven ? D.drivenLive[kk] : kk;
+    const bool own = k < M && (driven || D.wDrv[i] < 0);
+    uint32_t o, live = 0;
+    WNeuron x = wn_load(D, i);
+    const float ad0 = x.ad;
+    const int arr = (int)D.wArr[i] - 1;
+    const uint32_t n = wn_count(D, i, own, o);
+    WList l = wl_make(D.wBuf + o, n, stage[warp] + lane);
+    __syncwarp();
+    int fired = wn_run<R, false, false>(D, P, i, own, h, 0, x, l, arr, -1, &live);
+    if (!own) fired = -1;
+    if (own) {
+      wn_store(D, i, x);
+      if (n) D.wCnt[i] = o;
+      if (arr >= 0) D.wArr[i] = 0;
+    }
+    if (driven) {
+      if (own) {
+        D.wLive[k] = live;
+        D.wOwn[k] = (uint8_t)(fired + 1);
+        D.wAd0[k] = ad0;
+      }
+      continue;
+    }
+    if (fired >= 0) {
+      atomicOr(D.wBits + (int64_t)wt * 32 + fired, 1u << lane);
+      atomicAdd(D.wSpikes + fired, 1);
+      D.spikeCount[i] = (float)((R)D.spikeCount[i] + R(1));
+    }
+  }
+}
+
+constexpr int kChainThreads = kWinNarrow;
+constexpr int kChainRun = window_run(kChainThreads);
+constexpr int kChainDriven = 8 * kChainThreads;  // driven neurons per instance at most
+
+// For each step the live entries' ranks, their draws, the forced spikes (draw_chain of fb_window.cu:
+// a warp owns M words of 32 entries and publishes a byte per four of them and step). sm: the
+// window's draws; returns the number used.
+template <int M>
+__device__ __forceinline__ uint32_t wc_chain(int n, int h, uint32_t *sLive, const uint32_t *sLim, const uint32_t *sm,
+                                             uint4 (*cnt)[2]) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+  constexpr int kBytes = M > 4 ? 2 : 1, V = kBytes;
+  uint32_t below[4 * V];
+#pragma unroll
+  for (int q = 0; q < 4 * V; q++) {
+    const int m = min(max((int)warp * kBytes - 4 * q, 0), 4);
+    below[q] = m == 0 ? 0u : 0x01010101u >> (32 - 8 * m);
+  }
+  uint32_t mask[M], lim[M], f[M];
+#pragma unroll
+  for (int m = 0; m < M; m++) {
+    const int k = (int)(warp * M + m) * 32 + (int)lane;
+    mask[m] = k < n ? sLive[k] : 0u;
+    lim[m] = k < n ? sLim[k] : 0u;
+    f[m] = 255u;
+  }
+  uint32_t base = 0;
+  for (int j = 0; j < h; j++) {
+    uint32_t live[M], mine[2] = {0, 0};
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+      live[m] = __ballot_sync(0xffffffffu, mask[m] & 1u);
+      mine[m / 4] += (uint32_t)__popc(live[m]);
+    }
+    if (lane < kBytes) ((uint8_t *)cnt[j & 1])[warp * kBytes + lane] = (uint8_t)(lane ? mine[1] : mine[0]);
+    __syncthreads();
+    uint32_t at = base;
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+      const uint4 c = cnt[j & 1][v];
+      at = __dp4a(c.x, below[4 * v], at);
+      at = __dp4a(c.y, below[4 * v + 1], at);
+      at = __dp4a(c.z, below[4 * v + 2], at);
+      at = __dp4a(c.w, below[4 * v + 3], at);
+      base = __dp4a(c.x, 0x01010101u, base);
+      base = __dp4a(c.y, 0x01010101u, base);
+      base = __dp4a(c.z, 0x01010101u, base);
+      base = __dp4a(c.w, 0x01010101u, base);
+    }
+    uint32_t x[M];
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+      x[m] = sm[at + (uint32_t)__popc(live[m] & lt)];
+      at += (uint32_t)__popc(live[m]);
+    }
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+      const bool hit = (mask[m] & 1u) && x[m] <= lim[m];
+      f[m] = hit ? (uint32_t)j : f[m];
+      mask[m] = hit ? 0u : mask[m] >> 1;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < M; m++) {
+    const int k = (int)(warp * M + m) * 32 + (int)lane;
+    if (k < n) sLive[k] = f[m];  // the forced step from here on
+  }
+  return base;
+}
+
+// The window's draws and forced spikes of one instance per block; the forced neurons' state and the
+// driven ones' own spikes.
+template <typename R>
+__global__ void __launch_bounds__(kChainThreads, 1) k_wchain(const DiffDev *Ds, DP<R> P, int32_t t0, int32_t t1,
+                                                            const uint32_t *jumpTab) {
+  extern __shared__ __align__(16) uint32_t pool[];  // lane tables, live bits, draw limits, draws
+  __shared__ DiffDev D;
+  __shared__ uint4 cnt[2][2];
+  __shared__ int nForced[kWindowMax];
+  load_dev(Ds, D);
+  const int h = min(t1, D.steps) - t0;
+  if (h <= 0) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n = *D.nLive;
+  uint32_t *jump = pool, *sLive = pool + kWinJumpWords, *sLim = sLive + n, *sm = sLim + n;
+  for (int k = tid; k < kWinJumpWords; k += kChainThreads) jump[k] = jumpTab[k];
+  if (tid < 4) cnt[tid >> 1][tid & 1] = make_uint4(0, 0, 0, 0);
+  if (tid < kWindowMax) nForced[tid] = 0;
+  for (int k = tid; k < n; k += kChainThreads) {
+    sLive[k] = D.wLive[k];
+    // x <= lim for u < p: u = (x >> 8) 2^-24, p = drive dt/1000 in R; a draw x is never 0
+    const R p = (R)d_drive(D, D.drivenLive[k], t0) * P.dtS;
+    const uint32_t t = p >= R(1) ? 1u << 24 : (uint32_t)ceil((double)p * 16777216.0);
+    sLim[k] = t ? (t << 8) - 1u : 0u;
+  }
+  const uint32_t s0 = *D.rng;
+  __syncthreads();
+  const uint32_t need = (uint32_t)n * (uint32_t)h;  // the host keeps it within the pool
+  if ((uint32_t)warp * 32 * kChainRun < need) {
+    uint32_t b = s0, x = 0;
+    for (int q = 0; q < 5; q++)
+      if ((warp >> q) & 1) b = xs_apply(jump + q * 128, b);
+    const uint32_t *off = jump + 5 * 128;
+#pragma unroll
+    for (int q = 0; q < 8; q++) x ^= off[((uint32_t)q * 16 + ((b >> (4 * q)) & 15u)) * 32 + lane];
+    for (uint32_t k = (uint32_t)tid * kChainRun, e = min(need, k + kChainRun); k < e; k++) {
+      x = xs_next(x);
+      sm[k] = x;
+    }
+  }
+  __syncthreads();
+  uint32_t used;
+  if (n <= kChainThreads) used = wc_chain<1>(n, h, sLive, sLim, sm, cnt);
+  else if (n <= 4 * kChainThreads) used = wc_chain<4>(n, h, sLive, sLim, sm, cnt);
+  else used = wc_chain<8>(n, h, sLive, sLim, sm, cnt);
+  __syncthreads();
+  if (tid == 0 && used) *D.rng = sm[used - 1];
+  for (int k = tid; k < n; k += kChainThreads) {
+    const uint32_t f = sLive[k];
+    const int own = (int)D.wOwn[k] - 1;
+    D.wFs[k] = (uint8_t)f;
+    if (f == 255u && own < 0) continue;
+    const int i = D.drivenLive[k];
+    D.spikeCount[i] = (float)((R)D.spikeCount[i] + R(1));
+    if (f == 255u) {
+      atomicOr(D.wBits + (int64_t)(i >> 5) * 32 + own, 1u << (i & 31));
+      atomicAdd(D.wSpikes + own, 1);
+      continue;
+    }
+    atomicAdd(&nForced[f], 1);
+    // refractory from the forced spike to the window's end
+    float r = (float)(P.tRef + P.dt), ad = D.wAd0[k];
+    for (int j = 0; j < h; j++) {
+      if (j >= (int)f && r > 0) r = (float)((R)r - P.dt);
+      if (j == (int)f) ad = (float)((R)ad + P.adaptInc);
+      ad = (float)((R)ad * P.dA);
+    }
+    D.v[i] = (float)P.vReset;
+    D.refr[i] = r;
+    D.adapt[i] = ad;
+  }
+  __syncthreads();
+  if (tid < h) D.tForced[t0 + tid] = nForced[tid];
+}
+
+// The tape of step t0 + blockIdx.x: its forced spikes in list order, then its threshold spikes
+// ascending, after the window's steps before it.
+__global__ void __launch_bounds__(1024) k_wemit(const DiffDev *Ds, int32_t t0, int32_t t1) {
+  __shared__ DiffDev D;
+  __shared__ uint32_t scan[33];
+  load_dev(Ds, D);
+  const int h = min(t1, D.steps) - t0, j = blockIdx.x, tid = threadIdx.x;
+  if (j >= h) return;
+  int64_t o = D.tOff[t0];
+  for (int q = 0; q < j; q++) o += D.tForced[t0 + q] + D.wSpikes[q];
+  auto put = [&](int64_t at, int32_t i) {
+    if (at < D.tapeCap) {
+      D.tIdx[at] = i;
+      D.tAmp[at] = 1.f;
+    } else {
+      atomicCAS(D.err, 0, FB_EOVERFLOW);
+    }
+  };
+  const int n = *D.nLive;
+  for (int k0 = 0; k0 < n; k0 += 1024) {
+    const int k = k0 + tid;
+    const uint32_t on = k < n && D.wFs[k] == j ? 1u : 0u;
+    uint32_t tot;
+    const uint32_t at = block_exclusive_scan(on, &tot, scan);
+    if (on) put(o + at, D.drivenLive[k]);
+    o += tot;
+  }
+  const int nW = (D.N + 31) / 32, per = (nW + 1023) / 1024, w0 = min(nW, tid * per), w1 = min(nW, w0 + per);
+  uint32_t c = 0, tot;
+  for (int w = w0; w < w1; w++) c += (uint32_t)__popc(D.wBits[(int64_t)w * 32 + j]);
+  int64_t at = o + block_exclusive_scan(c, &tot, scan);
+  if (c)
+    for (int w = w0; w < w1; w++) {
+      uint32_t bits = D.wBits[(int64_t)w * 32 + j];
+      if (!bits) continue;
+      D.wBits[(int64_t)w * 32 + j] = 0;
+      for (; bits; bits &= bits - 1) put(at++, w * 32 + __ffs(bits) - 1);
+    }
+  if (tid == 0) D.tOff[t0 + j + 1] = o + tot;
 }
 
 // The reverse neuron pass of the window's steps, last first (bneuron for h steps), a neuron per

@@ -58,3 +58,19 @@ def test_short_refractory_times(tref):
     np.testing.assert_array_equal(idx, tape["idx"])
     dL = np.ones(80, np.float32)
     _compare_grads(prob.backward(tape, dL), net.backward(dL))
+
+
+@pytest.mark.parametrize("nD", [1, 512, 513, 2048, 2049, 4096, 4097])
+def test_driven_list_sizes(nD):
+    """The chain's layouts; 2,049 and more also shorten the windows (their draws); 4,097 goes step by
+    step. Drawn often enough that a step forces hundreds of spikes."""
+    ins = hub_net(4500, 1, nD, deg=5)
+    rng = np.random.default_rng(nD)
+    driven = rng.permutation(4500)[:nD].astype(np.int32)
+    hz = rng.uniform(100, 2500, nD)
+    prob, net = _pair(ins, dict(CUBA, checkpoint=50, adaptInc=0.3), driven, hz)
+    sc0, tape = prob.forward(57, seed=4, checkpoint=50)
+    assert sc0.tobytes() == net.forward(57, seed=4).tobytes()
+    off, idx, _ = net.tape()
+    np.testing.assert_array_equal(off, tape["off"])
+    np.testing.assert_array_equal(idx, tape["idx"])
