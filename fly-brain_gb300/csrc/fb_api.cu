@@ -1179,6 +1179,7 @@ static int win_setup(fb_brains *br) {
   WinRes &R = br->win;
   int rc;
   if (!R.ready && (rc = win_create(br, false))) return rc;
+  bool moved = false;
   for (int b = 0; b < br->B; b++) {
     const Trial &T = br->host[b];
     WinBrain &W = R.host[b];
@@ -1187,15 +1188,10 @@ static int win_setup(fb_brains *br) {
       CU(cudaMemsetAsync(W.bgHit, 0, (size_t)T.N * std::min(T.nslots - 1, kWinMax) * 4, br->stream));
       CU(cudaMemcpyAsync(&R.win[b].bgHit, &W.bgHit, sizeof(void *), cudaMemcpyHostToDevice, br->stream));
     }
-    const DrivenSet &ds = br->driven[b];
-    if (ds.version != R.drivenVersion[b]) {
-      const int nD = (int)ds.order.size();
-      CU(launch_driven_pos(T.driven, nD, T.N, W.drvPos, br->stream));
-      W.hasDriven = nD > 0;
-      CU(cudaMemcpyAsync(&R.win[b].hasDriven, &W.hasDriven, 4, cudaMemcpyHostToDevice, br->stream));
-      R.drivenVersion[b] = ds.version;
-    }
+    moved = moved || br->driven[b].version != R.drivenVersion[b];
+    R.drivenVersion[b] = br->driven[b].version;
   }
+  if (moved) CU(launch_driven_pos(br->trials, R.win, br->B, br->stream));
   return FB_OK;
 }
 
@@ -1205,18 +1201,19 @@ static int win_launch(fb_brains *br, const std::vector<int32_t> &steps, int hCap
   WinArgs a;
   memset(&a, 0, sizeof a);
   a.allPlain = 1;
+  bool changed = false;  // some brain's window
   for (int b = 0; b < br->B; b++) {
     const Trial &T = br->host[b];
     const int32_t H = std::min(window_steps(T, (int64_t)br->driven[b].order.size()), hCap);
-    if (H != R.host[b].H) {
-      R.host[b].H = H;
-      CU(cudaMemcpyAsync(&R.win[b].H, &R.host[b].H, 4, cudaMemcpyHostToDevice, br->stream));
-    }
+    changed = changed || H != R.host[b].H;
+    R.host[b].H = H;
     a.nWin = std::max(a.nWin, (steps[b] + H - 1) / H);
     if (steps[b] > 0 && (T.flags & kHasBg)) a.anyBg = 1;
     if ((T.flags & (kAdaptZero | kResRest | kHasBg | kHasDep)) != (kAdaptZero | kResRest) || T.coba) a.allPlain = 0;
   }
   if (a.nWin == 0) return FB_OK;
+  if (changed)
+    CU(cudaMemcpy2DAsync(&R.win[0].H, sizeof(WinBrain), &R.host[0].H, sizeof(WinBrain), 4, br->B, cudaMemcpyHostToDevice, br->stream));
   if (br->stepsUploaded != steps) {  // the last launch's counts stay on the device otherwise
     std::memcpy(br->h_steps, steps.data(), sizeof(int32_t) * br->B);
     CU(cudaMemcpyAsync(br->d_steps, br->h_steps, sizeof(int32_t) * br->B, cudaMemcpyHostToDevice, br->stream));

@@ -39,6 +39,7 @@
 // Not covered (the grid kernel runs these): presynaptic inhibition, sequential and fast delivery.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "fb_window.cuh"
@@ -1499,9 +1500,16 @@ __global__ void __launch_bounds__(1024) exclusive_prefix_kernel(uint32_t *off, i
     carry += tot;
   }
 }
-__global__ void driven_pos_kernel(const int32_t *driven, int32_t nD, int32_t *pos) {
-  const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < nD) pos[driven[k]] = k;
+// Places in the driven lists of all brains: first none, then each entry's.
+__global__ void driven_pos_kernel(const Trial *trials, WinBrain *win, int set) {
+  const Trial &T = trials[blockIdx.y];
+  WinBrain &W = win[blockIdx.y];
+  const int n = set ? T.nDriven : T.N;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    if (set) W.drvPos[T.driven[k]] = k;
+    else W.drvPos[k] = -1;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) W.hasDriven = T.nDriven > 0;
 }
 
 // ---- launch glue ---------------------------------------------------------------------------------
@@ -1589,10 +1597,10 @@ cudaError_t launch_in_offsets(const uint32_t *indices, int32_t N, int64_t E, uin
   return cudaGetLastError();
 }
 
-cudaError_t launch_driven_pos(const int32_t *driven, int32_t nD, int32_t N, int32_t *pos, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(pos, 0xff, (size_t)N * 4, st);
-  if (e != cudaSuccess || nD == 0) return e;
-  driven_pos_kernel<<<(nD + 255) / 256, 256, 0, st>>>(driven, nD, pos);
+cudaError_t launch_driven_pos(const Trial *trials, WinBrain *win, int B, cudaStream_t st) {
+  const dim3 grid(std::max(1, 1216 / B), B);
+  driven_pos_kernel<<<grid, 256, 0, st>>>(trials, win, 0);
+  driven_pos_kernel<<<grid, 256, 0, st>>>(trials, win, 1);
   return cudaGetLastError();
 }
 

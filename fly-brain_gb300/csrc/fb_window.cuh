@@ -84,8 +84,8 @@ const void *window_kernel_wide();
 const void *window_kernel_narrow();
 // In-degree prefix of a topology (off: [N+1]).
 cudaError_t launch_in_offsets(const uint32_t *indices, int32_t N, int64_t E, uint32_t *off, cudaStream_t st);
-// drvPos from the driven list.
-cudaError_t launch_driven_pos(const int32_t *driven, int32_t nD, int32_t N, int32_t *pos, cudaStream_t st);
+// drvPos and hasDriven of every brain from its driven list.
+cudaError_t launch_driven_pos(const Trial *trials, WinBrain *win, int B, cudaStream_t st);
 // The ring's spikes in flight into the log (import), the log's into the ring (export: every slot
 // in flight, or the last step's list only), the log emptied (brains b0 .. b1-1).
 cudaError_t launch_log_import(Trial *trials, WinBrain *win, int B, cudaStream_t st);
