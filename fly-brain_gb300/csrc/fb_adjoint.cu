@@ -44,7 +44,7 @@ void host_jump_tables(std::vector<uint32_t> &tab);
 constexpr int kDB = 256;      // threads per block of the per-neuron kernels
 constexpr int kDBucket = 8;   // bucket slots per target and step
 constexpr int kDSortMax = 64; // contributions per target sorted in local memory
-constexpr int kRB = 128;      // blocks per instance of the final reduction
+constexpr int kRB = 256;      // blocks per instance of the final reduction
 constexpr int kNSums = 9;     // scalar sums per instance
 constexpr int32_t kClaimFree = 0x7f7f7f7f;  // spike-train claim slots between steps
 constexpr double kDriveMax = 0.999;         // a soft drive's largest expected spike (src/lifdiff.js:72)
@@ -64,7 +64,7 @@ struct DiffDev {
   int64_t E;
   // graph and per-neuron structure
   const uint32_t *indptr, *indices;
-  const uint32_t *cscPtr, *cscEdge, *cscSrc;  // in-edges of each target, ascending edge id
+  const uint32_t *cscPtr;  // in-degree prefix
   const float *counts, *edgeGain, *sign, *logGain, *outScale, *thrOffset, *betaArr, *biasArr, *sizeLog;
   const uint8_t *thrMask, *biasMask;
   const float *drive;     // the drive as set (Hz)
@@ -124,6 +124,7 @@ struct DiffDev {
   double *accA, *accV, *accKc, *accLa, *accEI, *accW, *accD, *gLog, *gBias, *gEdge;
   float *gLogF;  // log-gain gradient as returned (non-finite -> 0)
   double *gOut;  // outScale gradient
+  double *sizeW; // the sizeAlpha term's factor of each target (k_size_weights)
   float *gDrive; // [epochs][nDS] dLoss/d(scheduled drive), float as the reference accumulates it
   const float *dL;       // flat [N], or per step over the readout set [steps][nro]
   const int32_t *roMap;  // neuron -> readout column, -1 elsewhere (per-step dL)
@@ -138,8 +139,8 @@ struct DiffDev {
   float *wE, *wI;
   int32_t *wResT;
   // a forward's windows: places in the live drivenSet (N); per driven entry its live steps, 1 + the
-  // step of its own spike, its forced step, its adaptation at the window's start; spikes per step
-  // as bits [N / 32][32 steps], and their number
+  // step of its own spike, its forced step, its adaptation at the window's start; threshold spikes
+  // as bits [kWindowMax steps][N / 32], and their number per step
   int32_t *wDrv;
   uint32_t *wLive;
   uint8_t *wOwn, *wFs;
@@ -225,14 +226,14 @@ __global__ void k_prepare(int32_t N, float *inScale, const float *sizeLog, const
 // of the delivered amount (:281-282), in double and in float.
 __global__ void k_prepare_edges(int64_t E, const uint32_t *indices, const float *counts, const float *edgeGain,
                                 const float *inScale, const uint8_t *sensory, double minSyn, uint8_t *gate,
-                                double *P, float *Pf) {
+                                double *P, float *Pf) {  // P or Pf may be null
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
   for (int64_t j = tid; j < E; j += nt) {
     const uint32_t q = indices[j];
     const double c = (double)counts[j];
     gate[j] = (c >= minSyn && !(sensory && sensory[q])) ? 1 : 0;
-    P[j] = c * (edgeGain ? (double)edgeGain[j] : 1.0) * (double)inScale[q];
-    Pf[j] = counts[j] * (edgeGain ? edgeGain[j] : 1.f) * inScale[q];
+    if (P) P[j] = c * (edgeGain ? (double)edgeGain[j] : 1.0) * (double)inScale[q];
+    if (Pf) Pf[j] = counts[j] * (edgeGain ? edgeGain[j] : 1.f) * inScale[q];
   }
 }
 
@@ -1068,14 +1069,16 @@ __global__ void __launch_bounds__(kDB, 2) k_barrival(const DiffDev *Ds, DP<R> P,
 namespace fb {
 
 // Per instance, kRB blocks of fixed-order partial sums: the seven per-neuron accumulators
-// (W EI V Kc La A D), the sizeAlpha term through inScale (src/lifdiff.js:650-655, 676-680:
-// gInScale[q] summed over q's in-edges in edge order) and the inhibitory-gain term.
-__global__ void k_reduce(const DiffDev *Ds, double inhGain, double sizeAlpha, double boostCap,
-                         double maxSizeScale, double *partial) {
+// (W EI V Kc La A D), the sizeAlpha term through inScale (src/lifdiff.js:650-655, 676-680: each
+// edge's gradient times its weight and its target's (-sizeLog) exp(-sizeAlpha sizeLog), where that is
+// inside the clamp) and the inhibitory-gain term. Edges are dealt to warps in order, so the per-edge
+// arrays stream; gathered by target (in-edges in edge order, a thread each) the kernel took 862 us at
+// 11M edges.
+__global__ void k_reduce(const DiffDev *Ds, double inhGain, double *partial) {
   __shared__ DiffDev D;
   __shared__ double sm[kNSums][kDB];
   load_dev(Ds, D);
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31;
   double acc[kNSums];
 #pragma unroll
   for (int k = 0; k < kNSums; k++) acc[k] = 0;
@@ -1087,19 +1090,47 @@ __global__ void k_reduce(const DiffDev *Ds, double inhGain, double sizeAlpha, do
     acc[4] += D.accLa[i];
     acc[5] += D.accA[i];
     acc[6] += D.accD[i];
-    double gis = 0, ginh = 0;
-    for (uint32_t e = D.cscPtr[i]; e < D.cscPtr[i + 1]; e++) {
-      const uint32_t j = D.cscEdge[e];
-      if (!D.gate[j]) continue;
-      const bool inh = D.sign[D.cscSrc[e]] < 0;  // eff's sign follows the presynaptic sign
-      const double cw = (double)D.counts[j] * (D.edgeGain ? (double)D.edgeGain[j] : 1.0);
-      gis += cw * (inh ? inhGain : 1.0) * D.gEdge[j];
-      if (inh) ginh += cw * (double)D.inScale[i] * D.gEdge[j];
+  }
+  // a warp takes a contiguous run of edges, four per lane in flight; each lane follows its row
+  const int64_t nw = (int64_t)(gridDim.x * blockDim.x) >> 5, w = ((int64_t)blockIdx.x * blockDim.x + tid) >> 5;
+  const int64_t run = (D.E + 128 * nw - 1) / (128 * nw) * 128, e0 = w * run, e1 = min(D.E, e0 + run);
+  int row = 0;  // the row of edge e0 + lane
+  if (e0 + lane < e1) {
+    int hi = D.N;
+    while (hi - row > 1) {
+      const int mid = (row + hi) >> 1;
+      if ((int64_t)D.indptr[mid] <= e0 + lane) row = mid;
+      else hi = mid;
     }
-    const double sl = (double)D.sizeLog[i];
-    const double raw = exp(-sizeAlpha * sl);
-    if (raw < boostCap && raw > 1 / maxSizeScale) acc[7] += gis * (-sl) * raw;
-    acc[8] += ginh;
+  }
+  for (int64_t e = e0 + lane; e < e1; e += 128) {
+    bool on[4];
+    uint32_t q[4];
+    float cn[4], eg[4], ins[4];
+    double g[4], sz[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int64_t j = e + 32 * u;
+      on[u] = j < e1 && D.gate[j];
+      q[u] = on[u] ? D.indices[j] : 0u;
+      cn[u] = on[u] ? D.counts[j] : 0.f;
+      eg[u] = on[u] && D.edgeGain ? D.edgeGain[j] : 1.f;
+      g[u] = on[u] ? D.gEdge[j] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      ins[u] = D.inScale[q[u]];
+      sz[u] = D.sizeW[q[u]];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      if (!on[u]) continue;
+      while ((int64_t)D.indptr[row + 1] <= e + 32 * u) row++;
+      const bool inh = D.sign[row] < 0;  // eff's sign follows the presynaptic sign
+      const double cw = (double)cn[u] * (double)eg[u];
+      if (sz[u] == sz[u]) acc[7] += cw * (inh ? inhGain : 1.0) * g[u] * sz[u];  // NaN: outside the clamp
+      if (inh) acc[8] += cw * (double)ins[u] * g[u];
+    }
   }
 #pragma unroll
   for (int k = 0; k < kNSums; k++) sm[k][tid] = acc[k];
@@ -1111,6 +1142,17 @@ __global__ void k_reduce(const DiffDev *Ds, double inhGain, double sizeAlpha, do
   }
   if (tid == 0)
     for (int k = 0; k < kNSums; k++) partial[((int64_t)blockIdx.y * kRB + blockIdx.x) * kNSums + k] = sm[k][0];
+}
+
+// The sizeAlpha term's factor of each target: (-sizeLog) exp(-sizeAlpha sizeLog) inside the clamp, NaN
+// outside.
+__global__ void k_size_weights(const DiffDev *Ds, double sizeAlpha, double boostCap, double maxSizeScale) {
+  __shared__ DiffDev D;
+  load_dev(Ds, D);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < D.N; i += gridDim.x * blockDim.x) {
+    const double sl = (double)D.sizeLog[i], raw = exp(-sizeAlpha * sl);
+    D.sizeW[i] = raw < boostCap && raw > 1 / maxSizeScale ? (-sl) * raw : __longlong_as_double(0x7ff8000000000000ll);
+  }
 }
 
 // Log-gain gradient as float with non-finite values zeroed and counted (src/lifdiff.js:681-684),
@@ -1236,7 +1278,7 @@ struct fb_diff_batch {
   std::vector<Inst> in;
   std::vector<EdgeGroup> groups;
   std::map<std::pair<const void *, int>, std::pair<void *, size_t>> shared;
-  std::map<std::pair<const void *, const void *>, std::vector<uint32_t *>> csc;  // (indptr, indices) -> CSC
+  std::map<std::pair<const void *, const void *>, uint32_t *> csc;  // (indptr, indices) -> in-degree prefix
   std::map<int64_t, float *> zeros;  // read-only zero arrays by length
   DiffDev *dDevs = nullptr;
   cudaStream_t st = nullptr;
@@ -1259,6 +1301,7 @@ struct fb_diff_batch {
   DP<float> P32;
   int32_t *err = nullptr, *nonfinite = nullptr;
   uint32_t *jump = nullptr;
+  double prepared[6] = {0, 0, 0, 0, 0, 0};  // what prepare() last ran for (last entry 0: nothing)
   uint32_t *winJump = nullptr;  // window_jump_tables of the forward's chain
   double *partial = nullptr;
 };
@@ -1334,17 +1377,15 @@ struct Carver {
   }
 };
 
-// In-edges of every target in ascending edge id (a stable counting sort of the CSR by target).
+// The graph checked, and its in-degree prefix.
 int build_csc(fb_diff_batch *b, DiffDev &D) {
   auto it = b->csc.find(std::make_pair((const void *)D.indptr, (const void *)D.indices));
   if (it != b->csc.end()) {
-    D.cscPtr = it->second[0];
-    D.cscEdge = it->second[1];
-    D.cscSrc = it->second[2];
+    D.cscPtr = it->second;
     return FB_OK;
   }
   const int64_t N = D.N, E = D.E;
-  std::vector<uint32_t> ip(N + 1), ix(E), cp(N + 1, 0), ce(E), cs(E);
+  std::vector<uint32_t> ip(N + 1), ix(E), cp(N + 1, 0);
   DCU(cudaMemcpy(ip.data(), D.indptr, (N + 1) * 4, cudaMemcpyDeviceToHost));
   if (E) DCU(cudaMemcpy(ix.data(), D.indices, E * 4, cudaMemcpyDeviceToHost));
   if (ip[0] != 0 || (int64_t)ip[N] != E)
@@ -1355,25 +1396,12 @@ int build_csc(fb_diff_batch *b, DiffDev &D) {
     if (ix[j] >= (uint32_t)N) return dfail(FB_EINVAL, "fb_diff: indices[%lld]=%u >= N", (long long)j, ix[j]);
   for (int64_t j = 0; j < E; j++) cp[ix[j] + 1]++;
   for (int64_t q = 0; q < N; q++) cp[q + 1] += cp[q];
-  std::vector<uint32_t> fill(cp.begin(), cp.end() - 1);
-  for (int64_t s = 0; s < N; s++)
-    for (uint32_t j = ip[s]; j < ip[s + 1]; j++) {
-      const uint32_t o = fill[ix[j]]++;
-      ce[o] = j;
-      cs[o] = (uint32_t)s;
-    }
-  uint32_t *a, *e, *s;
+  uint32_t *a;
   int rc;
-  if ((rc = talloc(b, &a, N + 1)) || (rc = talloc(b, &e, E)) || (rc = talloc(b, &s, E))) return rc;
+  if ((rc = talloc(b, &a, N + 1))) return rc;
   DCU(cudaMemcpy(a, cp.data(), (N + 1) * 4, cudaMemcpyHostToDevice));
-  if (E) {
-    DCU(cudaMemcpy(e, ce.data(), E * 4, cudaMemcpyHostToDevice));
-    DCU(cudaMemcpy(s, cs.data(), E * 4, cudaMemcpyHostToDevice));
-  }
-  b->csc[std::make_pair((const void *)D.indptr, (const void *)D.indices)] = {a, e, s};
+  b->csc[std::make_pair((const void *)D.indptr, (const void *)D.indices)] = a;
   D.cscPtr = a;
-  D.cscEdge = e;
-  D.cscSrc = s;
   return FB_OK;
 }
 
@@ -1492,7 +1520,7 @@ int create_instance(fb_diff_batch *b, Inst &I, const fb_diff_net *net, int64_t t
   c.add(&D.lv, N); c.add(&D.lgE, N); c.add(&D.lgI, N); c.add(&D.lad, N); c.add(&D.lres, N);
   c.add(&D.accA, N); c.add(&D.accV, N); c.add(&D.accKc, N); c.add(&D.accLa, N); c.add(&D.accEI, N);
   c.add(&D.accW, N); c.add(&D.accD, N); c.add(&D.gLog, N); c.add(&D.gBias, N); c.add(&D.gEdge, E);
-  c.add(&D.gLogF, N); c.add(&D.gOut, N); c.add(&D.nonfinite, 2);
+  c.add(&D.gLogF, N); c.add(&D.gOut, N); c.add(&D.sizeW, N); c.add(&D.nonfinite, 2);
   c.add(&D.tIdx, D.tapeCap); c.add(&D.tAmp, D.tapeCap);
   c.add(&D.drivenLive, N); c.add(&D.nLive, 1); c.add(&D.rmFlag, N); c.add(&D.claim, N);
   if ((rc = c.commit(b))) return rc;
@@ -1595,15 +1623,20 @@ int push_devs(fb_diff_batch *b) {
   return FB_OK;
 }
 
+// inScale, the gate and the products, in the pass's precision: again only after a field was set
+// or the parameters changed.
 int prepare(fb_diff_batch *b, const fb_diff_params *p) {
+  const double q[6] = {p->sizeAlpha, p->maxSizeScale, p->boostCap, p->minSyn, (double)b->f32, 1.0};
+  if (!memcmp(q, b->prepared, sizeof q)) return FB_OK;
   for (const EdgeGroup &G : b->groups) {
     const Inst &I = b->in[G.rep];
     k_prepare<<<256, kDB, 0, b->st>>>(I.D.N, G.inScale, I.sizeLogSrc, I.inScaleSrc, p->sizeAlpha,
                                        p->maxSizeScale, p->boostCap);
     k_prepare_edges<<<1024, kDB, 0, b->st>>>(I.D.E, I.D.indices, I.D.counts, I.D.edgeGain, G.inScale, I.sensory,
-                                              p->minSyn, G.gate, G.P, G.Pf);
+                                              p->minSyn, G.gate, b->f32 ? nullptr : G.P, b->f32 ? G.Pf : nullptr);
   }
   DCU(cudaGetLastError());
+  memcpy(b->prepared, q, sizeof q);
   return FB_OK;
 }
 
@@ -1794,7 +1827,7 @@ bool window_buffers(fb_diff_batch *b, int h, bool back) {
     if (!D.wCnt) {
       uint8_t *raw = nullptr;
       const size_t n4 = ((size_t)D.N * 4 + 255) / 256 * 256, n1 = ((size_t)D.N + 255) / 256 * 256;
-      const size_t nb = ((size_t)D.N + 31) / 32 * 32 * 4 + 255 & ~(size_t)255;
+      const size_t nb = (((size_t)D.N + 31) / 32 * kWindowMax * 4 + 255) / 256 * 256;
       if (!try_talloc(b, &raw, 5 * n4 + 4 * n1 + nb + 256 + ((size_t)D.E * 16 + 255) / 256 * 256)) return false;
       D.wBuf = (uint4 *)raw;
       uint8_t *p = raw + ((size_t)D.E * 16 + 255) / 256 * 256;
@@ -1821,7 +1854,7 @@ bool window_buffers(fb_diff_batch *b, int h, bool back) {
       const size_t n1 = ((size_t)D.N + 255) / 256 * 256;
       if (cudaMemcpyAsync(D.wCnt, D.cscPtr, (size_t)D.N * 4, cudaMemcpyDeviceToDevice, b->st) != cudaSuccess ||
           cudaMemsetAsync(D.wArr, 0, 2 * n1, b->st) != cudaSuccess ||
-          cudaMemsetAsync(D.wBits, 0, ((size_t)D.N + 31) / 32 * 32 * 4, b->st) != cudaSuccess) {
+          cudaMemsetAsync(D.wBits, 0, ((size_t)D.N + 31) / 32 * kWindowMax * 4, b->st) != cudaSuccess) {
         cudaGetLastError();
         return false;
       }
@@ -2169,6 +2202,7 @@ extern "C" int fb_diff_batch_set(fb_diff_batch *b, int32_t inst, int32_t field, 
     default: return dfail(FB_EINVAL, "fb_diff_set: unknown field %d", field);
   }
   if (!dst) return dfail(FB_ESTATE, "fb_diff_set: field %d was not given at creation", field);
+  b->prepared[5] = 0;
   DCU(cudaMemcpyAsync((void *)dst, values, n * 4, cudaMemcpyDefault, b->st));
   DCU(cudaStreamSynchronize(b->st));
   return FB_OK;
@@ -2504,8 +2538,8 @@ extern "C" int fb_diff_batch_backward(fb_diff_batch *b, const float *const *dL, 
   if ((rc = check_err(b, "fb_diff_backward"))) return rc;
   // fixed-order reductions of the scalar terms
   const fb_diff_params &P = b->lastP;
-  k_reduce<<<dim3(kRB, b->B), kDB, 0, b->st>>>(b->dDevs, P.inhGain, P.sizeAlpha, P.boostCap, P.maxSizeScale,
-                                                b->partial);
+  k_size_weights<<<dim3(32, b->B), kDB, 0, b->st>>>(b->dDevs, P.sizeAlpha, P.boostCap, P.maxSizeScale);
+  k_reduce<<<dim3(kRB, b->B), kDB, 0, b->st>>>(b->dDevs, P.inhGain, b->partial);
   k_finalize<<<ng, kDB, 0, b->st>>>(b->dDevs);
   DCU(cudaGetLastError());
   std::vector<double> part((size_t)b->B * kRB * kNSums);

@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kDB, 4) k_wforward(const DiffDev *Ds, DP<R> P,
       continue;
     }
     if (fired >= 0) {
-      atomicOr(D.wBits + (int64_t)wt * 32 + fired, 1u << lane);
+      atomicOr(D.wBits + (int64_t)fired * nW + wt, 1u << lane);
       atomicAdd(D.wSpikes + fired, 1);
       D.spikeCount[i] = (float)((R)D.spikeCount[i] + R(1));
     }
@@ -507,6 +507,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_wchain(const DiffDev *Ds, 
   __shared__ DiffDev D;
   __shared__ uint4 cnt[2][2];
   __shared__ int nForced[kWindowMax];
+  __shared__ uint32_t nEvents;
   load_dev(Ds, D);
   const int h = min(t1, D.steps) - t0;
   if (h <= 0) return;
@@ -516,6 +517,8 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_wchain(const DiffDev *Ds, 
   for (int k = tid; k < kWinJumpWords; k += kChainThreads) jump[k] = jumpTab[k];
   if (tid < 4) cnt[tid >> 1][tid & 1] = make_uint4(0, 0, 0, 0);
   if (tid < kWindowMax) nForced[tid] = 0;
+  if (tid == 0) nEvents = 0;
+#pragma unroll 4
   for (int k = tid; k < n; k += kChainThreads) {
     sLive[k] = D.wLive[k];
     // x <= lim for u < p: u = (x >> 8) 2^-24, p = drive dt/1000 in R; a draw x is never 0
@@ -545,15 +548,33 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_wchain(const DiffDev *Ds, 
   else used = wc_chain<8>(n, h, sLive, sLim, sm, cnt);
   __syncthreads();
   if (tid == 0 && used) *D.rng = sm[used - 1];
-  for (int k = tid; k < n; k += kChainThreads) {
-    const uint32_t f = sLive[k];
-    const int own = (int)D.wOwn[k] - 1;
-    D.wFs[k] = (uint8_t)f;
-    if (f == 255u && own < 0) continue;
+  // the entries that fire, gathered so that one pass serves them (in the place of the limits)
+  uint32_t *event = sLim;
+  for (int k0 = 0; k0 < n; k0 += kChainThreads) {
+    const int k = k0 + tid;
+    uint32_t f = 255u;
+    int own = -1;
+    if (k < n) {
+      f = sLive[k];
+      own = (int)D.wOwn[k] - 1;
+      D.wFs[k] = (uint8_t)f;
+    }
+    const bool on = f != 255u || own >= 0;
+    const uint32_t m = __ballot_sync(0xffffffffu, on);
+    uint32_t at = 0;
+    if (m && lane == 0) at = atomicAdd(&nEvents, (uint32_t)__popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0) + (uint32_t)__popc(m & ((1u << lane) - 1u));
+    if (on) event[at] = (uint32_t)k | (f << 16) | ((uint32_t)(own + 1) << 24);
+  }
+  __syncthreads();
+  const uint32_t nE = nEvents;
+  for (uint32_t q = tid; q < nE; q += kChainThreads) {
+    const uint32_t ev = event[q], f = (ev >> 16) & 255u;
+    const int k = (int)(ev & 0xffffu), own = (int)(ev >> 24) - 1;
     const int i = D.drivenLive[k];
     D.spikeCount[i] = (float)((R)D.spikeCount[i] + R(1));
     if (f == 255u) {
-      atomicOr(D.wBits + (int64_t)(i >> 5) * 32 + own, 1u << (i & 31));
+      atomicOr(D.wBits + (int64_t)own * ((D.N + 31) / 32) + (i >> 5), 1u << (i & 31));
       atomicAdd(D.wSpikes + own, 1);
       continue;
     }
@@ -602,13 +623,14 @@ __global__ void __launch_bounds__(1024) k_wemit(const DiffDev *Ds, int32_t t0, i
   }
   const int nW = (D.N + 31) / 32, per = (nW + 1023) / 1024, w0 = min(nW, tid * per), w1 = min(nW, w0 + per);
   uint32_t c = 0, tot;
-  for (int w = w0; w < w1; w++) c += (uint32_t)__popc(D.wBits[(int64_t)w * 32 + j]);
+  uint32_t *words = D.wBits + (int64_t)j * nW;
+  for (int w = w0; w < w1; w++) c += (uint32_t)__popc(words[w]);
   int64_t at = o + block_exclusive_scan(c, &tot, scan);
   if (c)
     for (int w = w0; w < w1; w++) {
-      uint32_t bits = D.wBits[(int64_t)w * 32 + j];
+      uint32_t bits = words[w];
       if (!bits) continue;
-      D.wBits[(int64_t)w * 32 + j] = 0;
+      words[w] = 0;
       for (; bits; bits &= bits - 1) put(at++, w * 32 + __ffs(bits) - 1);
     }
   if (tid == 0) D.tOff[t0 + j + 1] = o + tot;
@@ -639,37 +661,56 @@ __global__ void __launch_bounds__(kDB, 3) k_wbneuron(const DiffDev *Ds, DP<R> P,
     const float thrO = D.thrOffset[i];
     const int ro = D.dL && D.roMap ? D.roMap[i] : -1;
     const int slotD = D.gDrive ? D.dSlot[i] : -1;
-    for (int j = h - 1; j >= 0; j--) {
+    const bool lossAll = D.dL && !D.roMap, lossRo = ro >= 0;
+    // a step's inputs, loaded a step ahead: mode, spike adjoint, potential, loss gradient
+    struct In {
+      int m;
+      float ls, v, ge, gi, ad, dl;
+      R u;
+    };
+    auto load = [&](int j) {
+      In x;
       const int t = t0 + j;
       const int64_t at = (int64_t)(row + j) * N + i;
-      const int m = D.aMode[at], md = m & 3;
+      x.m = D.aMode[at];
+      x.ls = D.lsRing[(int64_t)(t % D.nslots) * N + i];
+      x.v = x.ge = x.gi = 0.f;
+      x.u = 0;
+      if (CUBA) {
+        x.u = aU[at];
+      } else {
+        x.v = D.aV[at];
+        x.ge = D.aGE[at];
+        x.gi = D.aGI[at];
+      }
+      x.ad = hasAd ? D.aAd[at] : 0.f;
+      x.dl = t >= lossFrom && (lossAll || lossRo) ? (lossRo ? D.dL[(int64_t)t * D.nro + ro] : D.dL[i]) : 0.f;
+      return x;
+    };
+    In next = load(h - 1);
+    for (int j = h - 1; j >= 0; j--) {
+      const int t = t0 + j;
+      const In in = next;
+      if (j > 0) next = load(j - 1);
+      const int m = in.m, md = m & 3;
       const R lpA = lad;
       const R lE = (R)lgE * P.dE, lI = (R)lgI * P.dE, lA = lpA * P.dA;
       float lgEF = (float)lE, lgIF = (float)lI, ladF = (float)lA;
       if (md == 1) {
         lv = 0.f;
       } else {
-        float *ls = D.lsRing + (int64_t)(t % D.nslots) * N + i;
-        const float lsv = *ls;
-        R dl = 0;
-        if (t >= lossFrom && D.dL) dl = D.roMap ? (ro >= 0 ? D.dL[(int64_t)t * D.nro + ro] : 0.f) : D.dL[i];
+        const float lsv = in.ls;
+        const R dl = in.dl;
         float *gDrv = slotD >= 0 ? D.gDrive + (int64_t)(t / D.driveEpoch) * D.nDS + slotD : nullptr;
-        if (__float_as_uint(lsv) != 0u) *ls = 0.f;
+        if (__float_as_uint(lsv) != 0u) D.lsRing[(int64_t)(t % D.nslots) * N + i] = 0.f;
         if (md == 2) {
           accA = accA + (double)lA;
           if (gDrv) *gDrv = (float)((R)*gDrv + (lA * P.adaptInc + ((R)lsv + dl)) * P.dtS);
           lv = 0.f;
         } else {
-          R vv = 0, gEv = 0, gIv = 0, uu;
-          if (CUBA) {
-            uu = aU[at];
-          } else {
-            vv = D.aV[at];
-            gEv = D.aGE[at];
-            gIv = D.aGI[at];
-            uu = d_u<R>(D, P, vv, gEv, gIv, bias);
-          }
-          const R thr = P.vThresh + (R)(hasAd ? D.aAd[at] : 0.f) + kc + (R)thrO;
+          const R vv = in.v, gEv = in.ge, gIv = in.gi;
+          const R uu = CUBA ? in.u : d_u<R>(D, P, vv, gEv, gIv, bias);
+          const R thr = P.vThresh + (R)in.ad + kc + (R)thrO;
           const R d = uu - thr;
           const R s = (m & 4) ? R(1) : R(0);
           const R tt = R(1) + fabs(d) / beta;
@@ -681,9 +722,13 @@ __global__ void __launch_bounds__(kDB, 3) k_wbneuron(const DiffDev *Ds, DP<R> P,
           const R lu = lvNew * (R(1) - s) + lt;
           const R lthr = -lt;
           if (gDrv) *gDrv = (float)((R)*gDrv + lsTot * (R(1) - s) * P.dtS);
-          accA = accA + (double)(lpA * s);
-          accV = accV + (double)lthr;
-          if (masked) accKc += (double)lthr;
+          // a zero leaves a sum as it is (no sum is ever -0), and the double pipes are the scarce ones
+          const R aA = lpA * s, aB = lu * P.kM;
+          if (aA != R(0)) accA = accA + (double)aA;
+          if (lthr != R(0)) {
+            accV = accV + (double)lthr;
+            if (masked) accKc += (double)lthr;
+          }
           ladF = (float)(lA + lthr * P.dA);
           if (CUBA) {
             lv = (float)(lu * (R(1) - P.kM));
@@ -693,10 +738,13 @@ __global__ void __launch_bounds__(kDB, 3) k_wbneuron(const DiffDev *Ds, DP<R> P,
             lv = (float)(lu * (R(1) + P.kM * (R(-1) - gEv * P.cE + gIv * P.cI)));
             lgEF = (float)(lE + lu * P.kM * (P.eExc - vv) * P.cE);
             lgIF = (float)(lI + lu * P.kM * (vv - P.eInh) * P.cI);
-            accEI += (double)(lu * P.kM * gIv * P.cI * (R(-1) + (vv - P.eInh) * P.cI));
+            const R aE = lu * P.kM * gIv * P.cI * (R(-1) + (vv - P.eInh) * P.cI);
+            if (aE != R(0)) accEI += (double)aE;
           }
-          if (lam != 0) accLa += (double)(lu * P.kM);
-          gB = gB + (double)(lu * P.kM);
+          if (aB != R(0)) {
+            if (lam != 0) accLa += (double)aB;
+            gB = gB + (double)aB;
+          }
         }
       }
       lv = cl(lv);
