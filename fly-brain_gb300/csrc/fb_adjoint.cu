@@ -46,6 +46,7 @@ constexpr int kDBucket = 8;   // bucket slots per target and step
 constexpr int kDSortMax = 64; // contributions per target sorted in local memory
 constexpr int kRB = 256;      // blocks per instance of the final reduction
 constexpr int kNSums = 9;     // scalar sums per instance
+constexpr int kWSumRows = 12; // rows of the float passes' sums in windows (three of four accumulators)
 constexpr int32_t kClaimFree = 0x7f7f7f7f;  // spike-train claim slots between steps
 constexpr double kDriveMax = 0.999;         // a soft drive's largest expected spike (src/lifdiff.js:72)
 
@@ -137,6 +138,7 @@ struct DiffDev {
   uint4 *wBuf;
   uint8_t *wArr, *wForced;
   float *wE, *wI;
+  float *wSum;            // the float passes' sums: kWSumRows rows of N
   int32_t *wResT;
   // a forward's windows: places in the live drivenSet (N); per driven entry its live steps, 1 + the
   // step of its own spike, its forced step, its adaptation at the window's start; threshold spikes
@@ -816,6 +818,8 @@ __global__ void k_zero_adjoint(const DiffDev *Ds) {
     D.lv[i] = D.lgE[i] = D.lgI[i] = D.lad[i] = D.lres[i] = 0.f;
     D.accA[i] = D.accV[i] = D.accKc[i] = D.accLa[i] = D.accEI[i] = D.accW[i] = D.accD[i] = 0.0;
     D.gLog[i] = D.gBias[i] = 0.0;
+    if (D.wSum)
+      for (int k = 0; k < kWSumRows; k++) D.wSum[k * N + i] = 0.f;
   }
   for (int64_t i = s0; i < (int64_t)D.nslots * N; i += ns) D.lsRing[i] = 0.f;
   for (int64_t j = s0; j < D.E; j += ns) D.gEdge[j] = 0.0;
@@ -1862,9 +1866,10 @@ bool window_buffers(fb_diff_batch *b, int h, bool back) {
     }
     if (I.histRows < h && back) {
       float *f = nullptr;
-      if (!try_talloc(b, &f, (size_t)2 * h * D.N)) return false;
+      if (!try_talloc(b, &f, (size_t)(2 * h + kWSumRows) * D.N)) return false;
       D.wE = f;
       D.wI = f + (size_t)h * D.N;
+      D.wSum = D.wI + (size_t)h * D.N;
       I.histRows = h;
     }
   }
@@ -2536,6 +2541,8 @@ extern "C" int fb_diff_batch_backward(fb_diff_batch *b, const float *const *dL, 
   }, "fb_diff_backward");
   if (rc) return rc;
   if ((rc = check_err(b, "fb_diff_backward"))) return rc;
+  if (win && b->f32) k_wsums<float><<<ng, kDB, 0, b->st>>>(b->dDevs, b->P32);
+  else if (win) k_wsums<double><<<ng, kDB, 0, b->st>>>(b->dDevs, b->P64);
   // fixed-order reductions of the scalar terms
   const fb_diff_params &P = b->lastP;
   k_size_weights<<<dim3(32, b->B), kDB, 0, b->st>>>(b->dDevs, P.sizeAlpha, P.boostCap, P.maxSizeScale);

@@ -636,6 +636,64 @@ __global__ void __launch_bounds__(1024) k_wemit(const DiffDev *Ds, int32_t t0, i
   if (tid == 0) D.tOff[t0 + j + 1] = o + tot;
 }
 
+// A gradient accumulator over a window's steps (kWA..kWEI). A double runs at two lanes per clock and
+// SM here, so the sums of floats are kept as three floats, in wSum from window to window, whose sum
+// is exact but for the last one's rounding (TwoSum: Knuth, The Art of Computer Programming,
+// 4.2.2): 72 bits against a double's 53. Addends past 2^100, infinities and NaN go to the double;
+// k_wsums adds the floats to it at the pass's end.
+enum { kWA, kWV, kWB, kWEI, kWSums };
+static_assert(3 * kWSums == kWSumRows, "three floats per accumulator");
+__device__ __forceinline__ double *w_acc(const DiffDev &D, int k) {
+  return k == kWA ? D.accA : k == kWV ? D.accV : k == kWB ? D.gBias : D.accEI;
+}
+template <typename R, int k>
+struct WSum {
+  double s;
+  __device__ void load(const DiffDev &D, int i) { s = w_acc(D, k)[i]; }
+  __device__ void add(const DiffDev &, int, R x) { s += x; }
+  __device__ void store(const DiffDev &D, int i) const { w_acc(D, k)[i] = s; }
+};
+template <int k>
+struct WSum<float, k> {
+  float a, b, c;
+  __device__ void load(const DiffDev &D, int i) {
+    const float *p = D.wSum + (int64_t)3 * k * D.N + i;
+    a = p[0], b = p[D.N], c = p[2 * (int64_t)D.N];
+  }
+  __device__ static float two(float &s, float x) {  // s + x as s and what it lost
+    const float t = s + x, z = t - s, e = (s - (t - z)) + (x - z);
+    s = t;
+    return e;
+  }
+  __device__ void add(const DiffDev &D, int i, float x) {
+    if (!(fabsf(x) <= 0x1p100f)) w_acc(D, k)[i] += (double)x;
+    else c += two(b, two(a, x));
+  }
+  __device__ void store(const DiffDev &D, int i) const {
+    float *p = D.wSum + (int64_t)3 * k * D.N + i;
+    p[0] = a, p[D.N] = b, p[2 * (int64_t)D.N] = c;
+  }
+};
+// The accumulators complete: the floats' part, and the two that are sums of the same addends over
+// part of the neurons (kcThreshold, laminaBias).
+template <typename R>
+__global__ void k_wsums(const DiffDev *Ds, DP<R> P) {
+  __shared__ DiffDev D;
+  load_dev(Ds, D);
+  const int64_t N = D.N;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+    if (sizeof(R) == 4)
+      for (int k = 0; k < kWSums; k++) {
+        const float *p = D.wSum + 3 * k * N + i;
+        w_acc(D, k)[i] += (double)p[0] + ((double)p[N] + (double)p[2 * N]);
+      }
+    if (D.thrMask && D.thrMask[i]) D.accKc[i] = D.accV[i];
+    R lam;
+    d_bias<R>(D, P, i, &lam);
+    if (lam != 0) D.accLa[i] = D.gBias[i];
+  }
+}
+
 // The reverse neuron pass of the window's steps, last first (bneuron for h steps), a neuron per
 // lane; the conductance adjoints after each step go to wE / wI for the window's arrivals.
 template <typename R, bool CUBA>
@@ -652,12 +710,15 @@ __global__ void __launch_bounds__(kDB, 3) k_wbneuron(const DiffDev *Ds, DP<R> P,
   auto cl = [c](float x) { return c > 0 ? (float)((R)x > c ? c : ((R)x < -c ? -c : (R)x)) : x; };
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
     float lv = D.lv[i], lgE = D.lgE[i], lgI = D.lgI[i], lad = D.lad[i];
-    double accA = D.accA[i], accV = D.accV[i], gB = D.gBias[i];
-    const bool masked = D.thrMask && D.thrMask[i];
-    double accKc = masked ? D.accKc[i] : 0.0, accEI = CUBA ? 0.0 : D.accEI[i];
-    R lam;
-    const R bias = d_bias<R>(D, P, i, &lam), kc = d_kc<R>(D, P, i), beta = d_beta<R>(D, P, i);
-    double accLa = lam != 0 ? D.accLa[i] : 0.0;
+    WSum<R, kWA> sA;
+    WSum<R, kWV> sV;
+    WSum<R, kWB> sB;
+    WSum<R, kWEI> sEI;
+    sA.load(D, i);
+    sV.load(D, i);
+    sB.load(D, i);
+    if (!CUBA) sEI.load(D, i);
+    const R bias = d_bias<R>(D, P, i, nullptr), kc = d_kc<R>(D, P, i), beta = d_beta<R>(D, P, i);
     const float thrO = D.thrOffset[i];
     const int ro = D.dL && D.roMap ? D.roMap[i] : -1;
     const int slotD = D.gDrive ? D.dSlot[i] : -1;
@@ -704,7 +765,7 @@ __global__ void __launch_bounds__(kDB, 3) k_wbneuron(const DiffDev *Ds, DP<R> P,
         float *gDrv = slotD >= 0 ? D.gDrive + (int64_t)(t / D.driveEpoch) * D.nDS + slotD : nullptr;
         if (__float_as_uint(lsv) != 0u) D.lsRing[(int64_t)(t % D.nslots) * N + i] = 0.f;
         if (md == 2) {
-          accA = accA + (double)lA;
+          if (lA != R(0)) sA.add(D, i, lA);
           if (gDrv) *gDrv = (float)((R)*gDrv + (lA * P.adaptInc + ((R)lsv + dl)) * P.dtS);
           lv = 0.f;
         } else {
@@ -722,13 +783,9 @@ __global__ void __launch_bounds__(kDB, 3) k_wbneuron(const DiffDev *Ds, DP<R> P,
           const R lu = lvNew * (R(1) - s) + lt;
           const R lthr = -lt;
           if (gDrv) *gDrv = (float)((R)*gDrv + lsTot * (R(1) - s) * P.dtS);
-          // a zero leaves a sum as it is (no sum is ever -0), and the double pipes are the scarce ones
           const R aA = lpA * s, aB = lu * P.kM;
-          if (aA != R(0)) accA = accA + (double)aA;
-          if (lthr != R(0)) {
-            accV = accV + (double)lthr;
-            if (masked) accKc += (double)lthr;
-          }
+          if (aA != R(0)) sA.add(D, i, aA);
+          if (lthr != R(0)) sV.add(D, i, lthr);
           ladF = (float)(lA + lthr * P.dA);
           if (CUBA) {
             lv = (float)(lu * (R(1) - P.kM));
@@ -739,12 +796,9 @@ __global__ void __launch_bounds__(kDB, 3) k_wbneuron(const DiffDev *Ds, DP<R> P,
             lgEF = (float)(lE + lu * P.kM * (P.eExc - vv) * P.cE);
             lgIF = (float)(lI + lu * P.kM * (vv - P.eInh) * P.cI);
             const R aE = lu * P.kM * gIv * P.cI * (R(-1) + (vv - P.eInh) * P.cI);
-            if (aE != R(0)) accEI += (double)aE;
+            if (aE != R(0)) sEI.add(D, i, aE);
           }
-          if (aB != R(0)) {
-            if (lam != 0) accLa += (double)aB;
-            gB = gB + (double)aB;
-          }
+          if (aB != R(0)) sB.add(D, i, aB);
         }
       }
       lv = cl(lv);
@@ -758,12 +812,10 @@ __global__ void __launch_bounds__(kDB, 3) k_wbneuron(const DiffDev *Ds, DP<R> P,
     D.lgE[i] = lgE;
     D.lgI[i] = lgI;
     D.lad[i] = lad;
-    D.accA[i] = accA;
-    D.accV[i] = accV;
-    D.gBias[i] = gB;
-    if (masked) D.accKc[i] = accKc;
-    if (!CUBA) D.accEI[i] = accEI;
-    if (lam != 0) D.accLa[i] = accLa;
+    sA.store(D, i);
+    sV.store(D, i);
+    sB.store(D, i);
+    if (!CUBA) sEI.store(D, i);
   }
 }
 

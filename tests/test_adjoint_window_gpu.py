@@ -74,3 +74,28 @@ def test_driven_list_sizes(nD):
     off, idx, _ = net.tape()
     np.testing.assert_array_equal(off, tape["off"])
     np.testing.assert_array_equal(idx, tape["idx"])
+
+
+@pytest.mark.parametrize("model", [CUBA, COBA])
+@pytest.mark.parametrize("power", [50, 100, 112])
+def test_float_sums_scale(model, power):
+    """Every operation of the reverse sweep is linear in dL, so with dL times 2^power the gradients
+    are the same times 2^power: at 0 every accumulator is summed in floats, at 100 part of them and
+    at 112 nearly all go to the double. Each sum of at most 200 terms is off by at most 200 * 2^-53 of its
+    terms' magnitudes; a float result rounds by 2^-24."""
+    ins = hub_net(300, 4, 11)
+    rng = np.random.default_rng(6)
+    driven = rng.permutation(300)[:200].astype(np.int32)
+    p = dict(model, checkpoint=40, precision="f32", adjClip=0.0, surrogateBeta=5.0)
+    _, net = _pair(ins, p, driven, np.full(200, 900.0))
+    net.forward(120, seed=5)
+    dL = rng.normal(0, 1, 300).astype(np.float32)
+    g0 = net.backward(dL)
+    net.forward(120, seed=5)
+    g1 = net.backward(np.ldexp(dL, power).astype(np.float32))
+    for k in ("logGain", "bias", "edge"):
+        a, b = np.asarray(g0[k], np.float64), np.ldexp(np.asarray(g1[k], np.float64), -power)
+        assert np.isfinite(b).all() and np.abs(a).max() > 0
+        assert np.abs(a - b).max() <= 1e-9 * np.abs(a).max() + 2.0 ** -23 * np.abs(a).max(), k
+    for k, v in g0["params"].items():
+        assert abs(v - np.ldexp(g1["params"][k], -power)) <= 1e-6 * abs(v) + 1e-9, k
