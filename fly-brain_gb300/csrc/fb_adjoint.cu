@@ -1669,6 +1669,19 @@ dim3 arrival_grid(const fb_diff_batch *b) {
   return dim3(std::max(2, 304 / b->B), b->B);
 }
 
+// The window kernels' grids. Neurons: a thread each, so that no block runs a second window-long pass
+// (a grid of 1,216 blocks over a batch of 12 uneven brains left a third of them a second one: its
+// training step 13.0 -> 11.6 ms). Arrivals: 608 blocks fill the chip at the delivery's four per SM,
+// and kWParts warps share a row, a window having fewer spikes than the chip has warps: 8 per row
+// gives one brain 1% and costs batches 2%; 304 or 1,216 blocks cost 1%.
+constexpr int kWParts = 4;
+dim3 window_neurons(const fb_diff_batch *b) {
+  return dim3(b->tuneNeuron > 0 ? std::min(b->maxTiles, b->tuneNeuron) : b->maxTiles, b->B);
+}
+dim3 window_arrivals(const fb_diff_batch *b) {
+  return dim3(b->tuneArrival > 0 ? b->tuneArrival : std::max(4, 608 / b->B), b->B);
+}
+
 // Stream ordering inside a pass: the first failure of an event record or wait is kept and
 // reported by run_pass (the launches' own errors are read there too).
 void order_note(fb_diff_batch *b, cudaError_t e) {
@@ -1729,6 +1742,7 @@ PassKey pass_key(const fb_diff_batch *b, char kind) {
   // the ring depth shapes a forward's stream order (a one-step delay orders the tape before the
   // next delivery) and is not among the scalars below (it follows from delay / dt)
   k.add(kind).add(b->f32).add(ng.x).add(ng.y).add(ag.x).add(ag.y).add(b->in[0].D.nslots);
+  k.add(window_neurons(b).x).add(window_arrivals(b).x);
   // the typed parameters without the struct's trailing padding
   if (b->f32) {
     const uint8_t *q = (const uint8_t *)&b->P32;
@@ -1917,13 +1931,13 @@ int chain_setup(fb_diff_batch *b) {
 // the tape of the window follows both.
 template <typename R>
 void window_forward_t(fb_diff_batch *b, const DP<R> &P, int32_t t0, int32_t t1) {
-  k_wdeliver<R><<<arrival_grid(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, -1, b->B == 1 ? 4 : 1);
+  k_wdeliver<R><<<window_arrivals(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, -1, kWParts);
   ev_record(b, b->evFork, b->st);
   ev_wait(b, b->side, b->evFork);
   k_wforward<R><<<dim3(b->B == 1 ? 64 : 8, b->B), kDB, 0, b->side>>>(b->dDevs, P, t0, t1, 1);
   k_wchain<R><<<dim3(1, b->B), kChainThreads, chain_smem(b), b->side>>>(b->dDevs, P, t0, t1, b->winJump);
   ev_record(b, b->evForced, b->side);
-  k_wforward<R><<<neuron_grid(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, 0);
+  k_wforward<R><<<window_neurons(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, 0);
   ev_wait(b, b->st, b->evForced);
   k_wemit<<<dim3(t1 - t0, b->B), 1024, 0, b->st>>>(b->dDevs, t0, t1);
 }
@@ -1934,9 +1948,9 @@ void window_forward(fb_diff_batch *b, int32_t t0, int32_t t1) {
 
 template <typename R>
 void window_replay_t(fb_diff_batch *b, const DP<R> &P, int32_t t0, int32_t t1, int32_t row) {
-  k_wdeliver<R><<<arrival_grid(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, row, b->B == 1 ? 4 : 1);
-  if (b->in[0].D.coba) k_wreplay<R, false><<<neuron_grid(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, row);
-  else k_wreplay<R, true><<<neuron_grid(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, row);
+  k_wdeliver<R><<<window_arrivals(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, row, kWParts);
+  if (b->in[0].D.coba) k_wreplay<R, false><<<window_neurons(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, row);
+  else k_wreplay<R, true><<<window_neurons(b), kDB, 0, b->st>>>(b->dDevs, P, t0, t1, row);
 }
 void window_replay(fb_diff_batch *b, int32_t t0, int32_t t1, int32_t row) {
   if (b->f32) window_replay_t<float>(b, b->P32, t0, t1, row);
@@ -1944,9 +1958,9 @@ void window_replay(fb_diff_batch *b, int32_t t0, int32_t t1, int32_t row) {
 }
 template <typename R>
 void window_reverse_t(fb_diff_batch *b, const DP<R> &P, cudaStream_t st, int32_t t0, int32_t t1, int32_t row, int32_t lossFrom) {
-  if (b->in[0].D.coba) k_wbneuron<R, false><<<neuron_grid(b), kDB, 0, st>>>(b->dDevs, P, t0, t1, row, lossFrom);
-  else k_wbneuron<R, true><<<neuron_grid(b), kDB, 0, st>>>(b->dDevs, P, t0, t1, row, lossFrom);
-  k_wbarrival<R><<<arrival_grid(b), kDB, 0, st>>>(b->dDevs, P, t0, t1, row);
+  if (b->in[0].D.coba) k_wbneuron<R, false><<<window_neurons(b), kDB, 0, st>>>(b->dDevs, P, t0, t1, row, lossFrom);
+  else k_wbneuron<R, true><<<window_neurons(b), kDB, 0, st>>>(b->dDevs, P, t0, t1, row, lossFrom);
+  k_wbarrival<R><<<window_arrivals(b), kDB, 0, st>>>(b->dDevs, P, t0, t1, row);
 }
 void window_reverse(fb_diff_batch *b, cudaStream_t st, int32_t t0, int32_t t1, int32_t row, int32_t lossFrom) {
   if (b->f32) window_reverse_t<float>(b, b->P32, st, t0, t1, row, lossFrom);

@@ -697,7 +697,7 @@ __global__ void k_wsums(const DiffDev *Ds, DP<R> P) {
 // The reverse neuron pass of the window's steps, last first (bneuron for h steps), a neuron per
 // lane; the conductance adjoints after each step go to wE / wI for the window's arrivals.
 template <typename R, bool CUBA>
-__global__ void __launch_bounds__(kDB, 3) k_wbneuron(const DiffDev *Ds, DP<R> P, int32_t t0, int32_t t1, int32_t row,
+__global__ void __launch_bounds__(kDB, 4) k_wbneuron(const DiffDev *Ds, DP<R> P, int32_t t0, int32_t t1, int32_t row,
                                                     int32_t lossFrom) {
   __shared__ DiffDev D;
   load_dev(Ds, D);
