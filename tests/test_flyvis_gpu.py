@@ -73,3 +73,35 @@ def test_set_input_and_reset():
     from flybrain import _native as nat
     with pytest.raises(nat.FlyBrainError):
         fv.set_input([m["N"]], [1.0], 0)
+
+
+@pytest.mark.parametrize("finite", [True, False])
+@pytest.mark.parametrize("N", [1, 37, 3000])
+@pytest.mark.parametrize("B", [1, 2, 3, 4, 6, 63, 66, 132])
+def test_vectors_chunks_and_weights(B, N, finite):
+    """Rows of whole and of padded vectors, one and several chunks of them, lists that end within a
+    group of four or are empty, several calls of one and more steps; weights that are not finite
+    (an inactive source must not meet them)."""
+    from oracle import oracle as O
+    from flybrain.flyvis import FlyVis
+    rng = np.random.default_rng(B * 7 + N)
+    deg = rng.integers(0, 12, N) * (rng.random(N) < 0.8)
+    indptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    E = int(indptr[-1])
+    w = rng.normal(0, 0.3, E).astype(np.float32)
+    if not finite and E:
+        w[:: max(1, E // 5)] = np.inf
+    m = dict(N=N, E=E, indptr=indptr, target=rng.integers(0, N, E).astype(np.int32), weight=w,
+             bias=rng.normal(0, 0.5, N).astype(np.float32), tau=rng.uniform(0.02, 0.2, N).astype(np.float32), dt=0.02)
+    x = rng.normal(0.0, 0.6, (B, N)).astype(np.float32)
+    fv = FlyVis(m, B=B)
+    v = np.tile(m["bias"], (B, 1)).astype(np.float32)
+    for b in range(B):
+        fv.write("x", b, x[b])
+    for steps in (1, 4, 1):
+        fv.step(steps)
+        O.fv_run(m, v, x, steps)
+        for b in range(B):
+            np.testing.assert_array_equal(fv.v(b), v[b])
+        v[0] = -v[0]
+        fv.write("v", 0, v[0])
