@@ -105,3 +105,31 @@ def test_vectors_chunks_and_weights(B, N, finite):
             np.testing.assert_array_equal(fv.v(b), v[b])
         v[0] = -v[0]
         fv.write("v", 0, v[0])
+
+
+@pytest.mark.parametrize("n", [1, 1024, 1025, 8192, 8193])
+def test_input_lists(n):
+    """Lists that a block holds in registers and longer ones, each index several times (its last
+    value stays), a bad index among them (an error, the rest written)."""
+    from flybrain import _native as nat
+    from flybrain.flyvis import FlyVis, synth_flyvis
+    m = synth_flyvis(N=700, seed=3, columns=12)
+    rng = np.random.default_rng(n)
+    fv = FlyVis(m, B=3)
+    for k in range(2):
+        idx = rng.integers(0, 700, n).astype(np.int32)
+        val = rng.normal(0, 1, n).astype(np.float32)
+        bad = k == 1 and n > 1
+        if bad:
+            idx[n // 2] = 700
+        ref = fv.read("x", 1)
+        ok = idx < 700
+        for i, y in zip(idx[ok], val[ok]):
+            ref[i] = y
+        if bad:
+            with pytest.raises(nat.FlyBrainError):
+                fv.set_input(idx, val, 1)
+        else:
+            fv.set_input(idx, val, 1)
+        np.testing.assert_array_equal(fv.read("x", 1), ref)
+    assert not fv.read("x", 0).any() and not fv.read("x", 2).any()
