@@ -1113,7 +1113,7 @@ static int win_create(fb_brains *br, bool early) {
   if (window_blocks_per_sm(B, R.smem) < 1) return fail(FB_EINVAL, "fb_step: the windowed kernel does not fit on an SM (%zu bytes)", R.smem);
   auto n4 = [&](int b) { return align256((size_t)br->host[b].N * 4); };
   // what must start at zero comes first: per brain drvPos, bgMask and arr (wcnt from the offsets)
-  size_t zero = align256(sizeof(WinBrain) * B) + align256(256 * 4), rest = 0;
+  size_t zero = align256(sizeof(WinBrain) * B) + align256(256 * 4 + (size_t)B * kWarpBrainBytes), rest = 0;
   std::vector<uint64_t> cap(B, 1024);
   for (int b = 0; b < B; b++) {
     const Trial &T = br->host[b];
@@ -1142,7 +1142,7 @@ static int win_create(fb_brains *br, bool early) {
   };
   CU(cudaMemsetAsync(R.arena, 0, zero, br->stream));
   R.win = (WinBrain *)take(sizeof(WinBrain) * B);
-  R.sync = (uint32_t *)take(256 * 4);
+  R.sync = (uint32_t *)take(256 * 4 + (size_t)B * kWarpBrainBytes);
   R.barBase = 0;
   for (int b = 0; b < B; b++) {
     const Trial &T = br->host[b];
@@ -1227,6 +1227,7 @@ static int win_launch(fb_brains *br, const std::vector<int32_t> &steps, int hCap
   a.jump = br->jump + kJumpWords + (window_threads(br->B) == kWinNarrow ? kWinJumpWords : 0);
   a.barCount = R.sync;
   a.uNext = R.sync + 64;
+  a.brains = (char *)(R.sync + 256);
   a.err = br->d_err;
   a.timeoutNs = br->timeoutNs;
   a.tripStep = br->tripStep;

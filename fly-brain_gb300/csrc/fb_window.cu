@@ -389,7 +389,7 @@ struct WinShared {
       uint32_t pre[kWinSpikes + 1];
     };
   };
-  WarpBrain wb[kWT / 32][2];
+  WarpBrain wb[kWT > 512 ? kWT / 32 : 1][2];
   WinArgs a;
   WinCtx ctx;
   Trial tr;  // a single brain's headers
@@ -422,10 +422,11 @@ __device__ __forceinline__ int find_brain(const uint32_t *pre, int B, uint32_t x
 // ---- U: the other neurons, the whole window ---------------------------------------------------
 //
 // A warp takes tiles of 32 neurons, and the steps between two contributions to any of them run
-// without looking at the lists: about 18 instructions per neuron and step. Measured on 96 full
-// brains, a window's U: 769 us when a warp also loaded its next tile ahead (the registers for it
-// spill, and the block's shared memory leaves little L1 to spill to), 634 us with a tile at a time
-// and the other 31 warps to hide its loads.
+// without looking at the lists: about 14 instructions per neuron and step. Bound by instructions
+// (72% of the issue slots). Measured on 96 full brains, a window's U: 769 us when a warp also loaded
+// its next tile ahead (the registers for it spill, and the block's shared memory leaves little L1 to
+// spill to), 641 us with a tile at a time and the other 31 warps to hide its loads, 592 us now; with
+// the next two tiles copied to shared memory ahead no less.
 struct Tile {
   int32_t i;  // this lane's neuron (0 where it has none)
   int32_t pos;  // its place in the driven list (-1: not driven)
@@ -435,40 +436,46 @@ struct Tile {
   uint32_t ar;
 };
 
-__device__ __forceinline__ void warp_brain(WarpBrain &B, const WinArgs &a, const WinCtx &c, int w, int b) {
+// By one thread, before the window's first barrier.
+__device__ __forceinline__ void make_brain(WarpBrain &B, const WinArgs &a, const WinCtx &c, int w, int b) {
+  const Trial &T = c.tr[b];
+  const WinBrain &C = c.win[b];
+  B.v = T.v;
+  B.f = (uint32_t)(T.gE - T.v);
+  B.N = T.N;
+  B.flags = T.flags;
+  B.nD = a.B == 1 ? T.nDriven : ldcg(&a.trials[b].nDriven);
+  B.h = c.h(b, w);
+  B.t0 = c.t0(b, w);
+  B.steps = c.steps[b];
+  B.e0 = (uint32_t)(c.done[b] + B.t0);
+  B.logMask = C.logMask;
+  B.dTr = T.dTr;
+  B.vThresh = T.vThresh;
+  B.K = model_of<1>(T);
+  B.inOff = C.inOff;
+  B.indptr = T.indptr;
+  B.drvPos = C.drvPos;
+  B.wcnt = C.wcnt;
+  B.spikeCount = T.spikeCount;
+  B.bgMask = C.bgMask;
+  B.bgHit = C.bgHit;
+  B.wbuf = C.wbuf;
+  B.log = C.log;
+  B.arr = C.arr;
+  B.sign = T.sign;
+  B.logTop = &a.win[b].logTop;
+  B.nFired = &a.trials[b].nFired;
+}
+// Into the warp's own words: a thread that reads the headers one by one takes microseconds.
+__device__ __forceinline__ void copy_brain(WarpBrain &B, const WarpBrain *src) {
+  static_assert(sizeof(WarpBrain) <= kWarpBrainBytes && sizeof(WarpBrain) % 4 == 0, "room in the launch's table");
   __syncwarp();
-  if ((threadIdx.x & 31u) == 0) {
-    const Trial &T = c.tr[b];
-    const WinBrain &C = c.win[b];
-    B.v = T.v;
-    B.f = (uint32_t)(T.gE - T.v);
-    B.N = T.N;
-    B.flags = T.flags;
-    B.nD = a.B == 1 ? T.nDriven : ldcg(&a.trials[b].nDriven);
-    B.h = c.h(b, w);
-    B.t0 = c.t0(b, w);
-    B.steps = c.steps[b];
-    B.e0 = (uint32_t)(c.done[b] + B.t0);
-    B.logMask = C.logMask;
-    B.dTr = T.dTr;
-    B.vThresh = T.vThresh;
-    B.K = model_of<1>(T);
-    B.inOff = C.inOff;
-    B.indptr = T.indptr;
-    B.drvPos = C.drvPos;
-    B.wcnt = C.wcnt;
-    B.spikeCount = T.spikeCount;
-    B.bgMask = C.bgMask;
-    B.bgHit = C.bgHit;
-    B.wbuf = C.wbuf;
-    B.log = C.log;
-    B.arr = C.arr;
-    B.sign = T.sign;
-    B.logTop = &a.win[b].logTop;
-    B.nFired = &a.trials[b].nFired;
-  }
+#pragma unroll
+  for (uint32_t k = threadIdx.x & 31u; k < sizeof(WarpBrain) / 4; k += 32) ((uint32_t *)&B)[k] = ldcg((const uint32_t *)src + k);
   __syncwarp();
 }
+
 
 // Only loads: nothing here waits for one.
 template <int GEN>
@@ -522,9 +529,42 @@ __device__ __forceinline__ void tile_run(const WarpBrain &T, const Tile &t, bool
     }
   } else {
     int j = 0;
+    if (kWT > 512 && !__any_sync(0xffffffffu, K.vReset >= thB)) {
+      // The refractory count as the step it ends before: a neuron that fires stays refractory to the
+      // window's end, and while it is it cannot cross a threshold above vReset. Four instructions
+      // fewer per step, which U of a batch is bound by (96 brains 641 -> 617 us a window); one
+      // brain's is not (its warps have two tiles at most).
+      int silent = 0;
+      float r = x.r;
+      for (int q = 0; q < h && __any_sync(0xffffffffu, r > 0); q++)
+        if (r > 0) {
+          r = __fsub_rn(r, K.dt);
+          silent = q + 1;
+        }
+      while (j < h) {
+        neuron_inputs<0>(K, x, l, j, 0, false, 0.f);
+        // steps until any lane's next contribution
+        const int e = min(h, (int)__reduce_min_sync(0xffffffffu, l.key >> 27));
+        do {  // neuron_step<0>
+          const float acc = __fadd_rn(__fadd_rn(__fadd_rn(__fsub_rn(K.vRest, x.v), x.ge), x.gi), t.bias);
+          const float v = __fadd_rn(x.v, __fmul_rn(acc, K.kM));
+          const bool cross = j >= silent && v >= thB;
+          x.v = j < silent || cross ? K.vReset : v;
+          silent = cross ? kWinMax + 1 + j : silent;
+          x.ge = __fmul_rn(x.ge, K.dE);
+          x.gi = __fmul_rn(x.gi, K.dE);
+        } while (++j < e);
+      }
+      fired = silent - (kWinMax + 1);
+      x.r = r;
+      if (__any_sync(0xffffffffu, fired >= 0)) {
+        if (fired >= 0) x.r = K.tRef;
+        for (int q = 1; q < h; q++)
+          if (fired >= 0 && q > fired) x.r = __fsub_rn(x.r, K.dt);
+      }
+    }
     while (j < h) {
       neuron_inputs<0>(K, x, l, j, 0, false, 0.f);
-      // steps until any lane's next contribution
       const int e = min(h, (int)__reduce_min_sync(0xffffffffu, l.key >> 27));
       do {
         if (neuron_step<0>(K, x, t.bias, t.thr, thB)) fired = j;
@@ -566,30 +606,32 @@ __device__ __forceinline__ void tile_run(const WarpBrain &T, const Tile &t, bool
 
 // This warp's share of the tiles of all brains (`total`, numbered through the prefix c.pre). Few
 // tiles per warp: dealt. Many: three quarters dealt as runs of a warp (a run stays within few brains), the
-// rest taken four at a time from a counter, so blocks that come late from a driven list take fewer.
+// rest taken by tickets from a counter, so that blocks that come late from a driven list take fewer:
+// four tiles a ticket, the last ones singly, as the warps of a block take 6 us for a tile.
 // meet: where not 0, the target of the grid barrier that U waits at, after the first loads.
 template <int GEN>
 __device__ __noinline__ bool update_tiles(int w, uint32_t total, uint32_t first,
                                           uint32_t nWarps, uint32_t meet) {
   const WinArgs &a = s_win.a;
   const WinCtx &c = s_win.ctx;
-  WarpBrain *wb = s_win.wb[threadIdx.x >> 5];
+  WarpBrain *wb = s_win.wb[kWT > 512 ? threadIdx.x >> 5 : 0];  // one brain: one for the block
   uint2 *stage = sort_stage();
   const uint32_t lane = threadIdx.x & 31u;
   constexpr uint32_t kGrab = 4;
   const bool dyn = total >= 16 * nWarps;
   const uint32_t run = total / nWarps * 3 / 4, dealt = dyn ? run * nWarps : total;
+  const uint32_t grabs = (total - dealt) / kGrab - min((total - dealt) / kGrab, nWarps / kGrab);  // tickets of four
   uint32_t g = dyn ? first * run : first, end = dyn ? g + run : total;
   // tiles first + k nWarps of every brain's, or of a run: two brains at most are in use at a time
   uint32_t lo = 0, hi = 0, cur = 0;
   Tile t;
   auto load = [&](Tile &x) {
-    if (g < lo || g >= hi) {
+    if (kWT > 512 && (g < lo || g >= hi)) {
       const int b = find_brain(c.pre, a.B, g);
       lo = c.pre[b];
       hi = c.pre[b + 1];
       cur ^= 1u;
-      warp_brain(wb[cur], a, c, w, b);
+      copy_brain(wb[cur], (const WarpBrain *)(a.brains + (size_t)b * kWarpBrainBytes));
     }
     tile_load<GEN>(wb[cur], (int32_t)((g - lo) * 32 + lane), x);
   };
@@ -608,9 +650,10 @@ __device__ __noinline__ bool update_tiles(int w, uint32_t total, uint32_t first,
     g += dyn ? 1 : nWarps;
     if (dyn && g >= end) {
       uint32_t x = 0;
-      if (lane == 0) x = atomicAdd(a.uNext + (w & 1), kGrab);
-      g = dealt + __shfl_sync(0xffffffffu, x, 0);
-      end = min(total, g + kGrab);
+      if (lane == 0) x = atomicAdd(a.uNext + (w & 1), 1u);
+      x = __shfl_sync(0xffffffffu, x, 0);
+      g = dealt + (x < grabs ? x * kGrab : grabs * kGrab + (x - grabs));
+      end = min(total, g + (x < grabs ? kGrab : 1u));
     }
     const bool more = g < total;
     tile_run<GEN>(T, t, own, n, head, stage);
@@ -1286,11 +1329,13 @@ __global__ void __launch_bounds__(kWT, 1) window_kernel(const WinArgs args) {
         }
         if (t0 + h >= c.steps[b]) args.trials[b].nFired = 0;
       }
+      if (kWT > 512 && tid == kWT - 1) make_brain(*(WarpBrain *)(args.brains + (size_t)b * kWarpBrainBytes), a, c, w, b);
       if (own < nServe) {  // one brain, and P left to the others: its draws now
         __syncthreads();
         fill_stream(ldcg(&W->rng), stream_need(c.tr[b], driven_count(a, c, b), h));
       }
     }
+    if (kWT <= 512 && tid == kWT - 1) make_brain(sh.wb[0][0], a, c, w, 0);
     if (blockIdx.x == gridDim.x - 1 && tid == 0) args.uNext[w & 1] = 0;
     if (own >= nServe) {
       if (args.B == 1) {

@@ -17,6 +17,7 @@ constexpr int kWinSort = 16;        // contributions per target sorted in shared
 constexpr int kWinStream = 37888;   // draws of a window at most, in shared memory
 // Generator words per thread (odd: the threads' runs start in different banks).
 constexpr int window_run(int threads) { return (kWinStream + threads - 1) / threads | 1; }
+constexpr int kWarpBrainBytes = 384;
 constexpr int kWinPool = 44032;     // words of that memory: a window's draws and its driven entries
 // Words a driven list's entries take of it.
 __host__ __device__ constexpr int window_entry_words(int nD) { return 3 * nD + (3 * nD + 3) / 4; }
@@ -70,6 +71,7 @@ struct WinArgs {
   uint32_t barBase;
   unsigned long long *prof;
   uint32_t *dbg;
+  char *brains;              // [B] kWarpBrainBytes: what U's warps need of each brain (written per window)
 };
 
 // M^(32 run 2^i) for i < 5 (8 nibble tables of 16 words each), then M^(run l) for l < 32 as word
