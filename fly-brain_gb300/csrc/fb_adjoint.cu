@@ -1840,15 +1840,26 @@ int window_steps(const fb_diff_batch *b) { return b->f32 ? window_steps_t(b, b->
 // The windows' buffers of every instance; false where memory is short (the pass then goes step by
 // step).
 bool window_buffers(fb_diff_batch *b, int h, bool back) {
+  auto up = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+  auto size = [&](const DiffDev &D) {
+    const size_t n4 = up((size_t)D.N * 4), n1 = up(D.N), nb = up(((size_t)D.N + 31) / 32 * kWindowMax * 4);
+    return up((size_t)D.E * 16) + 5 * n4 + 4 * n1 + nb + 256;
+  };
+  // one allocation for all instances: each costs a first pass some 100 us
+  size_t need = 0, hist = 0;
+  for (const Inst &I : b->in) {
+    if (!I.D.wCnt) need += size(I.D);
+    if (I.histRows < h && back) hist += up((size_t)(2 * h + kWSumRows) * I.D.N * 4);
+  }
+  uint8_t *raw = nullptr, *rows = nullptr;
+  if (need && !try_talloc(b, &raw, need)) return false;
   for (Inst &I : b->in) {
     DiffDev &D = I.D;
     if (!D.wCnt) {
-      uint8_t *raw = nullptr;
-      const size_t n4 = ((size_t)D.N * 4 + 255) / 256 * 256, n1 = ((size_t)D.N + 255) / 256 * 256;
-      const size_t nb = (((size_t)D.N + 31) / 32 * kWindowMax * 4 + 255) / 256 * 256;
-      if (!try_talloc(b, &raw, 5 * n4 + 4 * n1 + nb + 256 + ((size_t)D.E * 16 + 255) / 256 * 256)) return false;
+      const size_t n4 = up((size_t)D.N * 4), n1 = up(D.N), nb = up(((size_t)D.N + 31) / 32 * kWindowMax * 4);
       D.wBuf = (uint4 *)raw;
-      uint8_t *p = raw + ((size_t)D.E * 16 + 255) / 256 * 256;
+      uint8_t *p = raw + up((size_t)D.E * 16);
+      raw += size(D);
       D.wResT = (int32_t *)p;
       D.wCnt = (uint32_t *)(p + n4);
       D.wArr = p + 2 * n4;
@@ -1868,6 +1879,10 @@ bool window_buffers(fb_diff_batch *b, int h, bool back) {
       D.wFs = p + n1;
       I.windowClear = false;
     }
+  }
+  if (hist && !try_talloc(b, &rows, hist)) return false;
+  for (Inst &I : b->in) {
+    DiffDev &D = I.D;
     if (!I.windowClear) {  // fresh, or what a failed pass left
       const size_t n1 = ((size_t)D.N + 255) / 256 * 256;
       if (cudaMemcpyAsync(D.wCnt, D.cscPtr, (size_t)D.N * 4, cudaMemcpyDeviceToDevice, b->st) != cudaSuccess ||
@@ -1879,8 +1894,8 @@ bool window_buffers(fb_diff_batch *b, int h, bool back) {
       I.windowClear = true;
     }
     if (I.histRows < h && back) {
-      float *f = nullptr;
-      if (!try_talloc(b, &f, (size_t)(2 * h + kWSumRows) * D.N)) return false;
+      float *f = (float *)rows;
+      rows += up((size_t)(2 * h + kWSumRows) * D.N * 4);
       D.wE = f;
       D.wI = f + (size_t)h * D.N;
       D.wSum = D.wI + (size_t)h * D.N;
