@@ -1096,6 +1096,7 @@ static int win_alloc(fb_brains *br, X **p, size_t n) {
   return FB_OK;
 }
 
+static size_t bg_hit_bytes(const Trial &T) { return align256((size_t)T.N * std::min(T.nslots - 1, kWinMax) * 4); }
 // The kernel's resources: one allocation for the batch. At the batch's creation (early) they wait
 // for the first launch if they would take much of the free memory.
 static int win_create(fb_brains *br, bool early) {
@@ -1120,7 +1121,7 @@ static int win_create(fb_brains *br, bool early) {
     // spikes of the last D + H steps: a neuron fires at most once in any H of them (H >= 1)
     const int D = T.nslots - 1, H = std::min(D, silent_steps(T));
     while (cap[b] < (uint64_t)T.N * ((D + H - 1) / H + 2)) cap[b] *= 2;
-    zero += 2 * n4(b) + align256(T.N);
+    zero += 2 * n4(b) + align256(T.N) + ((T.flags & kHasBg) ? bg_hit_bytes(T) : 0);
     rest += n4(b) + align256(cap[b] * 16) + align256((size_t)T.E * 8) + align256((size_t)kWinDriven * (4 + kWinSaved * 4 + 1));
   }
   if (early && zero + rest > ((size_t)8 << 30)) {
@@ -1150,6 +1151,7 @@ static int win_create(fb_brains *br, bool early) {
     W.bgMask = (uint32_t *)take(n4(b));
     W.drvPos = (int32_t *)take(n4(b));
     W.arr = (uint8_t *)take(T.N);
+    if (T.flags & kHasBg) W.bgHit = (uint32_t *)take(bg_hit_bytes(T));
   }
   for (int b = 0; b < B; b++) {
     const Trial &T = br->host[b];
@@ -1180,14 +1182,22 @@ static int win_setup(fb_brains *br) {
   int rc;
   if (!R.ready && (rc = win_create(br, false))) return rc;
   bool moved = false;
+  size_t need = 0;  // brains that draw background events since they were created (then in the arena)
+  for (int b = 0; b < br->B; b++)
+    if ((br->host[b].flags & kHasBg) && !R.host[b].bgHit) need += bg_hit_bytes(br->host[b]);
+  if (need) {
+    char *p = nullptr;
+    if ((rc = win_alloc(br, &p, need))) return rc;
+    CU(cudaMemsetAsync(p, 0, need, br->stream));
+    for (int b = 0; b < br->B; b++)
+      if ((br->host[b].flags & kHasBg) && !R.host[b].bgHit) {
+        R.host[b].bgHit = (uint32_t *)p;
+        p += bg_hit_bytes(br->host[b]);
+      }
+    CU(cudaMemcpy2DAsync(&R.win[0].bgHit, sizeof(WinBrain), &R.host[0].bgHit, sizeof(WinBrain), sizeof(void *), br->B,
+                         cudaMemcpyHostToDevice, br->stream));
+  }
   for (int b = 0; b < br->B; b++) {
-    const Trial &T = br->host[b];
-    WinBrain &W = R.host[b];
-    if ((T.flags & kHasBg) && !W.bgHit) {
-      if ((rc = win_alloc(br, &W.bgHit, (size_t)T.N * std::min(T.nslots - 1, kWinMax)))) return rc;
-      CU(cudaMemsetAsync(W.bgHit, 0, (size_t)T.N * std::min(T.nslots - 1, kWinMax) * 4, br->stream));
-      CU(cudaMemcpyAsync(&R.win[b].bgHit, &W.bgHit, sizeof(void *), cudaMemcpyHostToDevice, br->stream));
-    }
     moved = moved || br->driven[b].version != R.drivenVersion[b];
     R.drivenVersion[b] = br->driven[b].version;
   }
