@@ -51,17 +51,17 @@ L2_FLUSH_BYTES = 512 << 20
 # capture of a 100-step launch of each kernel (profiles/); traffic grows in proportion to steps.
 DRAM_BYTES_PER_STEP_SINGLE = {
     "grid": 16.826112e6 / 100,    # fb::step_kernel
-    "lagged": (52.875264e6 + 0.801792e6) / 100,   # fb::lagged_kernel
+    "lagged": (17.078784e6 + 0.124160e6) / 100,   # fb::narrow::window_kernel
 }
-# DRAM bytes (read + write) per trial-step of the batched grid kernel, from one ncu capture of a
-# 100-step launch over 32 full-scale trials (profiles/step_kernel_batched_32_trials.txt:
-# 12.51 GB read + 6.95 GB written over 3,200 trial-steps); the bench's launch is scaled by its
-# trial-steps (the update streams every trial's state, so traffic grows in proportion).
-DRAM_BYTES_PER_TRIAL_STEP_BATCHED = (12.51e9 + 6.95e9) / 3200
+# DRAM bytes (read + write) per trial-step of the batched windowed kernel, from one ncu capture of
+# the whole uneven launch over 32 full-scale trials (profiles/window_kernels.txt: 226.5 GB read +
+# 104.1 GB written over 351,925 trial-steps); the bench's launch is scaled by its trial-steps (the
+# update streams every trial's state once a window, so traffic grows in proportion).
+DRAM_BYTES_PER_TRIAL_STEP_BATCHED = (226.51e9 + 104.08e9) / 351925
 HIGH_ACTIVITY_BIAS_MV = 6.0
 KERNEL_NAME = {
     "grid": "fb::step_kernel (persistent, two grid barriers per step)",
-    "lagged": "fb::lagged_kernel (persistent, delay-scheduled)",
+    "lagged": "fb::narrow::window_kernel (persistent, windows of the synaptic delay)",
 }
 
 
@@ -326,8 +326,7 @@ def run_ours(args, rank, world):
         events=tot_events,
         e2e=dict(value=e2e_events / e2e_s, unit="synaptic events/s", h2d_bytes_per_step=h2d // args.steps,
                  d2h_bytes_per_step=d2h // args.steps, sim_s_per_wall_s=sim_s / e2e_s),
-        # the lagged schedule launches the step kernel and the ring bookkeeping kernel
-        gpu_launches=args.steps * (2 if sched == "lagged" else 1),
+        gpu_launches=args.steps,  # one persistent kernel each
         schedule=sched,
         roofline=dict(bound="hbm", achieved=achieved, peak=peak, unit="GB/s", frac=achieved / peak,
                       peak_kind=kind, traffic=DRAM_BYTES_PER_STEP_SINGLE[sched] * S,
@@ -430,7 +429,7 @@ def run_high_activity(g, idx, hz, args, bias_mv=HIGH_ACTIVITY_BIAS_MV, launches=
     return dict(bias_mv=bias_mv, launches=launches, brain_steps=launches * S, events_per_s=events / secs,
                 ms_per_1000_steps=1e3 * secs / (launches * S) * 1000, realtime_factor=sim_s / secs,
                 spikes_per_step=spikes / (launches * S), recurrent_fraction=1.0 - dspikes / max(spikes, 1.0),
-                events_per_step=events / (launches * S), schedule=sched, gpu_launches=launches * (2 if sched == "lagged" else 1),
+                events_per_step=events / (launches * S), schedule=sched, gpu_launches=launches,
                 roofline=dict(bound="hbm", achieved=ach, peak=peak, unit="GB/s", frac=ach / peak, peak_kind=kind,
                               traffic=None, kernel=KERNEL_NAME[sched], algorithmic_bytes_per_launch=byts),
                 clocks=clk.summary(),
