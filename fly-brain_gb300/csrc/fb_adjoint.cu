@@ -138,6 +138,9 @@ struct DiffDev {
   uint4 *wBuf;
   uint8_t *wArr, *wForced;
   float *wE, *wI;
+  int32_t wRows;          // rows of wE and of wI
+  uint8_t *wAct;          // neurons whose adjoint may not be zero
+  const int32_t *wild;    // some edge's factors are not finite
   float *wSum;            // the float passes' sums: kWSumRows rows of N
   int32_t *wResT;
   // a forward's windows: places in the live drivenSet (N); per driven entry its live steps, 1 + the
@@ -228,12 +231,16 @@ __global__ void k_prepare(int32_t N, float *inScale, const float *sizeLog, const
 // of the delivered amount (:281-282), in double and in float.
 __global__ void k_prepare_edges(int64_t E, const uint32_t *indices, const float *counts, const float *edgeGain,
                                 const float *inScale, const uint8_t *sensory, double minSyn, uint8_t *gate,
-                                double *P, float *Pf) {  // P or Pf may be null
+                                double *P, float *Pf, int32_t *wild) {  // P or Pf may be null
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
   for (int64_t j = tid; j < E; j += nt) {
     const uint32_t q = indices[j];
     const double c = (double)counts[j];
     gate[j] = (c >= minSyn && !(sensory && sensory[q])) ? 1 : 0;
+    if (gate[j]) {  // an edge whose products with zero need not be zero
+      const float w = counts[j] * (edgeGain ? edgeGain[j] : 1.f);
+      if (!isfinite(w) || !isfinite(inScale[q])) *wild = 1;
+    }
     if (P) P[j] = c * (edgeGain ? (double)edgeGain[j] : 1.0) * (double)inScale[q];
     if (Pf) Pf[j] = counts[j] * (edgeGain ? edgeGain[j] : 1.f) * inScale[q];
   }
@@ -1243,6 +1250,7 @@ struct EdgeGroup {
   uint8_t *gate;
   double *P;
   float *Pf;
+  int32_t *wild;  // some edge's factors are not finite
 };
 
 struct Inst {
@@ -1553,7 +1561,7 @@ int build_groups(fb_diff_batch *b) {
       const int64_t N = I.D.N, E = I.D.E;
       int rc;
       Carver c;
-      c.add(&G.inScale, N); c.add(&G.gate, E); c.add(&G.P, E); c.add(&G.Pf, E);
+      c.add(&G.inScale, N); c.add(&G.gate, E); c.add(&G.P, E); c.add(&G.Pf, E); c.add(&G.wild, 1);
       if ((rc = c.commit(b))) return rc;
       b->groups.push_back(G);
       g = (int)b->groups.size() - 1;
@@ -1563,6 +1571,7 @@ int build_groups(fb_diff_batch *b) {
     I.D.gate = b->groups[g].gate;
     I.D.P = b->groups[g].P;
     I.D.Pf = b->groups[g].Pf;
+    I.D.wild = b->groups[g].wild;
   }
   return FB_OK;
 }
@@ -1634,10 +1643,12 @@ int prepare(fb_diff_batch *b, const fb_diff_params *p) {
   if (!memcmp(q, b->prepared, sizeof q)) return FB_OK;
   for (const EdgeGroup &G : b->groups) {
     const Inst &I = b->in[G.rep];
+    DCU(cudaMemsetAsync(G.wild, 0, 4, b->st));
     k_prepare<<<256, kDB, 0, b->st>>>(I.D.N, G.inScale, I.sizeLogSrc, I.inScaleSrc, p->sizeAlpha,
                                        p->maxSizeScale, p->boostCap);
     k_prepare_edges<<<1024, kDB, 0, b->st>>>(I.D.E, I.D.indices, I.D.counts, I.D.edgeGain, G.inScale, I.sensory,
-                                              p->minSyn, G.gate, b->f32 ? nullptr : G.P, b->f32 ? G.Pf : nullptr);
+                                              p->minSyn, G.gate, b->f32 ? nullptr : G.P, b->f32 ? G.Pf : nullptr,
+                                              G.wild);
   }
   DCU(cudaGetLastError());
   memcpy(b->prepared, q, sizeof q);
@@ -1849,7 +1860,7 @@ bool window_buffers(fb_diff_batch *b, int h, bool back) {
   size_t need = 0, hist = 0;
   for (const Inst &I : b->in) {
     if (!I.D.wCnt) need += size(I.D);
-    if (I.histRows < h && back) hist += up((size_t)(2 * h + kWSumRows) * I.D.N * 4);
+    if (I.histRows < h && back) hist += up((size_t)(2 * h + kWSumRows) * I.D.N * 4) + up(I.D.N);
   }
   uint8_t *raw = nullptr, *rows = nullptr;
   if (need && !try_talloc(b, &raw, need)) return false;
@@ -1896,6 +1907,9 @@ bool window_buffers(fb_diff_batch *b, int h, bool back) {
     if (I.histRows < h && back) {
       float *f = (float *)rows;
       rows += up((size_t)(2 * h + kWSumRows) * D.N * 4);
+      D.wAct = rows;
+      rows += up(D.N);
+      D.wRows = h;
       D.wE = f;
       D.wI = f + (size_t)h * D.N;
       D.wSum = D.wI + (size_t)h * D.N;
@@ -1971,11 +1985,20 @@ void window_replay(fb_diff_batch *b, int32_t t0, int32_t t1, int32_t row) {
   if (b->f32) window_replay_t<float>(b, b->P32, t0, t1, row);
   else window_replay_t<double>(b, b->P64, t0, t1, row);
 }
+// A parameter that is not finite: the reverse sweep then leaves no zero out.
+template <typename R>
+int32_t not_finite(const DP<R> &P) {
+  const R all[] = {P.vThresh, P.vReset, P.wSyn, P.adaptInc, P.depU, P.eExc, P.eInh, P.inhGain, P.kcThreshold, P.laminaBias,
+              P.dE, P.dA, P.kRec, P.kM, P.dtS, P.cE, P.cI};
+  for (R x : all)
+    if (!std::isfinite(x)) return 1;
+  return 0;
+}
 template <typename R>
 void window_reverse_t(fb_diff_batch *b, const DP<R> &P, cudaStream_t st, int32_t t0, int32_t t1, int32_t row, int32_t lossFrom) {
   if (b->in[0].D.coba) k_wbneuron<R, false><<<window_neurons(b), kDB, 0, st>>>(b->dDevs, P, t0, t1, row, lossFrom);
   else k_wbneuron<R, true><<<window_neurons(b), kDB, 0, st>>>(b->dDevs, P, t0, t1, row, lossFrom);
-  k_wbarrival<R><<<window_arrivals(b), kDB, 0, st>>>(b->dDevs, P, t0, t1, row);
+  k_wbarrival<R><<<window_arrivals(b), kDB, 0, st>>>(b->dDevs, P, t0, t1, row, not_finite(P));
 }
 void window_reverse(fb_diff_batch *b, cudaStream_t st, int32_t t0, int32_t t1, int32_t row, int32_t lossFrom) {
   if (b->f32) window_reverse_t<float>(b, b->P32, st, t0, t1, row, lossFrom);
@@ -2512,6 +2535,8 @@ extern "C" int fb_diff_batch_backward(fb_diff_batch *b, const float *const *dL, 
   if ((rc = push_devs(b))) return rc;
   const dim3 ng = neuron_grid(b);
   k_zero_adjoint<<<ng, kDB, 0, b->st>>>(b->dDevs);
+  if (win && b->f32) k_wactive<float><<<ng, kDB, 0, b->st>>>(b->dDevs, b->P32, not_finite(b->P32));
+  else if (win) k_wactive<double><<<ng, kDB, 0, b->st>>>(b->dDevs, b->P64, not_finite(b->P64));
   for (int k = 0; k < b->B; k++) DCU(cudaMemsetAsync(b->in[k].D.nonfinite, 0, 8, b->st));
   if ((rc = prepare(b, &b->lastP))) return rc;
   const int32_t steps = b->maxSteps;

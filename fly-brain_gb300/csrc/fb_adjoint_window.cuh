@@ -269,6 +269,7 @@ __device__ __forceinline__ int wn_run(const DiffDev &D, const DP<R> &P, int i, b
   R *aU = (R *)D.aV;
   const bool hasAd = P.adaptInc != 0;
   int fired = -1;
+  bool wild = false;
   for (int j = 0; j < h; j++) {
     while ((l.c.x >> 27) == (uint32_t)j) {
       const R c = sizeof(R) == 8 ? (R)__longlong_as_double((long long)(((unsigned long long)l.c.w << 32) | l.c.z))
@@ -311,6 +312,7 @@ __device__ __forceinline__ int wn_run(const DiffDev &D, const DP<R> &P, int i, b
     if (REPLAY && own && hasAd && !wasRefr) D.aAd[at] = x.ad;
     if (!wasRefr) {
       const R thr = P.vThresh + (R)x.ad + kc + (R)thrO;
+      if (REPLAY) wild |= !(fabs(vi - thr) <= (R)3e38);
       if (vi >= thr) {
         s = 1;
         fired = j;
@@ -322,6 +324,7 @@ __device__ __forceinline__ int wn_run(const DiffDev &D, const DP<R> &P, int i, b
     if (REPLAY && own) D.aMode[at] = (uint8_t)(md | s << 2);
     x.v = (float)vi;
   }
+  if (REPLAY && own && wild) D.wAct[i] = 1;  // zero times infinity
   return fired;
 }
 
@@ -694,8 +697,29 @@ __global__ void k_wsums(const DiffDev *Ds, DP<R> P) {
   }
 }
 
-// The reverse neuron pass of the window's steps, last first (bneuron for h steps), a neuron per
-// lane; the conductance adjoints after each step go to wE / wI for the window's arrivals.
+// The reverse sweep leaves out what is zero. A neuron's adjoint is zero until a loss gradient or an
+// arrival reversed at one of its targets reaches it, and a step of the sweep keeps it so (every
+// term is a product with it). wAct marks the neurons that may have one: at the pass's start those
+// with a loss gradient, then those k_wbarrival hands one to; also every neuron whose products with
+// zero need not be zero (a potential, threshold or surrogate width that is not finite, `dense` for
+// the parameters). The others' rows of wE and wI stay zero. 1% of the neurons of a full brain with
+// 1,000 readouts are ever marked.
+template <typename R>
+__global__ void k_wactive(const DiffDev *Ds, DP<R> P, int32_t dense) {
+  __shared__ DiffDev D;
+  load_dev(Ds, D);
+  const int64_t N = D.N, s0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, ns = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = s0; i < N; i += ns) {
+    const bool loss = D.dL && (D.roMap ? D.roMap[i] >= 0 : !(D.dL[i] == 0.f));
+    const float thr = D.thrOffset[i];
+    D.wAct[i] = dense || loss || thr != thr || !(d_beta<R>(D, P, (int)i) > R(1e-30));
+  }
+  for (int64_t k = s0; k < 2 * D.wRows * N; k += ns) D.wE[k] = 0.f;  // and wI behind it
+}
+
+// The reverse neuron pass of the window's steps, last first (bneuron for h steps), over the marked
+// neurons of each tile of 256, gathered so that they fill warps; the conductance adjoints after
+// each step go to wE / wI for the window's arrivals.
 template <typename R, bool CUBA>
 __global__ void __launch_bounds__(kDB, 4) k_wbneuron(const DiffDev *Ds, DP<R> P, int32_t t0, int32_t t1, int32_t row,
                                                     int32_t lossFrom) {
@@ -708,7 +732,16 @@ __global__ void __launch_bounds__(kDB, 4) k_wbneuron(const DiffDev *Ds, DP<R> P,
   const bool hasAd = P.adaptInc != 0;
   const R c = P.adjClip;
   auto cl = [c](float x) { return c > 0 ? (float)((R)x > c ? c : ((R)x < -c ? -c : (R)x)) : x; };
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+  __shared__ uint16_t mark[kDB];
+  __shared__ uint32_t nMark;
+  for (int tile = blockIdx.x * kDB; tile < N; tile += gridDim.x * kDB) {
+    __syncthreads();
+    if (threadIdx.x == 0) nMark = 0;
+    __syncthreads();
+    if (tile + (int)threadIdx.x < N && D.wAct[tile + threadIdx.x]) mark[atomicAdd(&nMark, 1u)] = (uint16_t)threadIdx.x;
+    __syncthreads();
+    if (threadIdx.x >= nMark) continue;
+    const int i = tile + mark[threadIdx.x];
     float lv = D.lv[i], lgE = D.lgE[i], lgI = D.lgI[i], lad = D.lad[i];
     WSum<R, kWA> sA;
     WSum<R, kWV> sV;
@@ -821,12 +854,14 @@ __global__ void __launch_bounds__(kDB, 4) k_wbneuron(const DiffDev *Ds, DP<R> P,
 
 // Reverse of the window's deliveries (k_barrival for h steps), warp per arrival.
 template <typename R>
-__global__ void __launch_bounds__(kDB, 2) k_wbarrival(const DiffDev *Ds, DP<R> P, int32_t t0, int32_t t1, int32_t row) {
+__global__ void __launch_bounds__(kDB, 2) k_wbarrival(const DiffDev *Ds, DP<R> P, int32_t t0, int32_t t1, int32_t row,
+                                                      int32_t dense) {
   __shared__ DiffDev D;
   __shared__ int64_t off[kWindowMax + 1];
   load_dev(Ds, D);
   const WSpan S = w_span(D, t0, t1, off);
   if (S.h <= 0) return;
+  const bool wild = dense || *D.wild;
   const int lane = threadIdx.x & 31, dd = D.nslots - 1;
   const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t a = S.a0 + w0; a < S.a1; a += nw) {
@@ -842,6 +877,7 @@ __global__ void __launch_bounds__(kDB, 2) k_wbarrival(const DiffDev *Ds, DP<R> P
     const bool exc = eff > 0;
     const float *lg0 = (exc ? D.wE : D.wI) + (int64_t)j * D.N;
     const uint32_t lo = D.indptr[pre], hi = D.indptr[pre + 1];
+    const bool all = wild || !(fabs(eff) <= (R)3e38) || !(fabs(base) <= (R)3e38);
     R lraw = 0;
     for (uint32_t j0 = lo + lane; j0 < hi; j0 += 32 * kEdgeILP) {
       bool on[kEdgeILP];
@@ -852,17 +888,19 @@ __global__ void __launch_bounds__(kDB, 2) k_wbarrival(const DiffDev *Ds, DP<R> P
       for (int u = 0; u < kEdgeILP; u++) {
         const uint32_t ed = j0 + 32u * u;
         on[u] = ed < hi && D.gate[ed];
+        if (on[u]) q[u] = D.indices[ed];
+      }
+#pragma unroll
+      for (int u = 0; u < kEdgeILP; u++)
+        if (on[u]) lgv[u] = lg0[q[u]];
+#pragma unroll
+      for (int u = 0; u < kEdgeILP; u++) {  // a zero adjoint adds zeros
+        const uint32_t ed = j0 + 32u * u;
+        on[u] = on[u] && (all || lgv[u] != 0.f);
         if (on[u]) {
-          q[u] = D.indices[ed];
           cnt[u] = D.counts[ed];
           eg[u] = D.edgeGain ? D.edgeGain[ed] : 1.f;
           old[u] = D.gEdge[ed];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < kEdgeILP; u++) {
-        if (on[u]) {
-          lgv[u] = lg0[q[u]];
           ins[u] = D.inScale[q[u]];
         }
       }
@@ -878,13 +916,14 @@ __global__ void __launch_bounds__(kDB, 2) k_wbarrival(const DiffDev *Ds, DP<R> P
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) lraw += __shfl_xor_sync(0xffffffffu, lraw, o);
-    if (lane == 0) {
+    if (lane == 0 && (all || lraw != 0 || D.lres[pre] != 0.f)) {
       float *target = D.lsRing + (int64_t)(e % D.nslots) * D.N;
       D.accW[pre] += (double)(lraw * sgn * gain * resAtv * amp);
       D.gLog[pre] += (double)(lraw * eff);
       float x = (float)((R)target[pre] + lraw * base);
       if (P.adjClip > 0) x = (float)fmin(P.adjClip, fmax(-P.adjClip, (R)x));
       target[pre] = x;
+      if (x != 0.f) D.wAct[pre] = 1;  // NaN != 0
       // the res adjoint decays once per step down to this one (its clip bounds what an arrival left)
       float lr = D.lres[pre];
       if (lr != 0.f)

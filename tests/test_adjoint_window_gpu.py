@@ -99,3 +99,54 @@ def test_float_sums_scale(model, power):
         assert np.abs(a - b).max() <= 1e-9 * np.abs(a).max() + 2.0 ** -23 * np.abs(a).max(), k
     for k, v in g0["params"].items():
         assert abs(v - np.ldexp(g1["params"][k], -power)) <= 1e-6 * abs(v) + 1e-9, k
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("what", ["one", "edge inf", "threshold inf", "threshold nan", "bias inf", "readout"])
+def test_what_the_sweep_leaves_out(what, precision):
+    """Losses on few neurons, so that most adjoints stay zero, and values with which a product with
+    zero is not zero, somewhere in the network. Without them a sweep over every neuron (a loss of the least
+    float on each, which marks all of them) gives the same gradients up to that loss's own; with them the
+    oracle's double sweep and the kernels agree on which gradients are lost."""
+    N = 400
+    ins = hub_net(N, 2, 21, deg=8)
+    rng = np.random.default_rng(8)
+    thr = np.zeros(N, np.float32)
+    if what == "edge inf":
+        ins["counts"][np.nonzero(ins["indices"] == 77)[0][0]] = np.inf
+    if what == "threshold inf":
+        thr[50:60] = np.inf
+    if what == "threshold nan":
+        thr[50:52] = np.nan
+    bias = np.zeros(N, np.float32)
+    if what == "bias inf":
+        bias[90] = np.inf
+    driven = rng.permutation(N)[:250].astype(np.int32)
+    p = dict(CUBA, checkpoint=30, adjClip=0.0, precision=precision)
+    prob, net = _pair(dict(ins, thrOffset=thr), p, driven, np.full(250, 700.0))
+    if what == "bias inf":
+        from flybrain.diff import DiffNet
+        net = DiffNet(dict(N=N, indptr=ins["indptr"], indices=ins["indices"], weights=ins["counts"], sign=ins["sign"]),
+                      dict(p, bias=bias, thrOffset=thr))
+        for i in driven:
+            net.setDriveOne(int(i), 700.0)
+    dL = np.zeros(N, np.float32)
+    dL[[5, 123]] = 1.0, -2.0
+    every = np.where(dL == 0, np.float32(1e-45), dL)
+    got = []
+    for d in (dL, every):
+        net.forward(100, seed=9)
+        if what == "readout":
+            got.append(net.backward(np.tile(d[[5, 123]], (100, 1)), readout=np.array([5, 123], np.int32))
+                       if d is dL else net.backward(d))
+        else:
+            got.append(net.backward(d))
+    a, b = got
+    for k in ("logGain", "bias", "edge"):
+        x, y = np.asarray(a[k], np.float64), np.asarray(b[k], np.float64)
+        np.testing.assert_array_equal(np.isnan(x), np.isnan(y))
+        np.testing.assert_array_equal(np.isinf(x), np.isinf(y))
+        ok = np.isfinite(x)
+        scale = np.abs(x[ok]).max() if ok.any() else 0.0
+        assert np.abs(x[ok] - y[ok]).max() <= 1e-6 * scale + 1e-30, k
+    assert a["clamped"] == b["clamped"]
