@@ -140,6 +140,8 @@ struct DiffDev {
   float *wE, *wI;
   int32_t wRows;          // rows of wE and of wI
   uint8_t *wAct;          // neurons whose adjoint may not be zero
+  uint8_t *wNeed;         // neurons that a segment's replay runs
+  uint8_t *wWild;         // neurons whose potential was not finite in the forward
   const int32_t *wild;    // some edge's factors are not finite
   float *wSum;            // the float passes' sums: kWSumRows rows of N
   int32_t *wResT;
@@ -258,6 +260,7 @@ __global__ void k_reset(const DiffDev *Ds, float vRest) {
     D.cnt[i] = 0;
     D.ovfHead[i] = kNil;
     if (i < D.nDriven) D.drivenLive[i] = D.driven[i];
+    if (D.wWild) D.wWild[i] = 0;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *D.rng = D.seed0;
@@ -1304,6 +1307,7 @@ struct fb_diff_batch {
   cudaError_t orderErr = cudaSuccess;  // first failed event record or wait of the pass being issued
   std::vector<void *> allocs;
   fb_diff_params lastP;
+  int32_t recordedWin = 0;  // the recorded forward ran in windows, nothing was set since
   int32_t f32 = 0, recordedK = 0, recorded = 0, maxSteps = 0, maxTiles = 1, maxN = 1;
   int32_t tuneNeuron = 0, tuneArrival = 0;  // launch shape overrides (0: default)
   int32_t stepLaunches = 0;                   // 1: launch every step's kernels from the host
@@ -1854,13 +1858,13 @@ bool window_buffers(fb_diff_batch *b, int h, bool back) {
   auto up = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
   auto size = [&](const DiffDev &D) {
     const size_t n4 = up((size_t)D.N * 4), n1 = up(D.N), nb = up(((size_t)D.N + 31) / 32 * kWindowMax * 4);
-    return up((size_t)D.E * 16) + 5 * n4 + 4 * n1 + nb + 256;
+    return up((size_t)D.E * 16) + 5 * n4 + 5 * n1 + nb + 256;
   };
   // one allocation for all instances: each costs a first pass some 100 us
   size_t need = 0, hist = 0;
   for (const Inst &I : b->in) {
     if (!I.D.wCnt) need += size(I.D);
-    if (I.histRows < h && back) hist += up((size_t)(2 * h + kWSumRows) * I.D.N * 4) + up(I.D.N);
+    if (I.histRows < h && back) hist += up((size_t)(2 * h + kWSumRows) * I.D.N * 4) + 2 * up(I.D.N);
   }
   uint8_t *raw = nullptr, *rows = nullptr;
   if (need && !try_talloc(b, &raw, need)) return false;
@@ -1888,6 +1892,7 @@ bool window_buffers(fb_diff_batch *b, int h, bool back) {
       p += n4;
       D.wOwn = p;
       D.wFs = p + n1;
+      D.wWild = D.wFs + n1;
       I.windowClear = false;
     }
   }
@@ -1908,7 +1913,8 @@ bool window_buffers(fb_diff_batch *b, int h, bool back) {
       float *f = (float *)rows;
       rows += up((size_t)(2 * h + kWSumRows) * D.N * 4);
       D.wAct = rows;
-      rows += up(D.N);
+      D.wNeed = rows + up(D.N);
+      rows += 2 * up(D.N);
       D.wRows = h;
       D.wE = f;
       D.wI = f + (size_t)h * D.N;
@@ -2260,6 +2266,7 @@ extern "C" int fb_diff_batch_set(fb_diff_batch *b, int32_t inst, int32_t field, 
   }
   if (!dst) return dfail(FB_ESTATE, "fb_diff_set: field %d was not given at creation", field);
   b->prepared[5] = 0;
+  b->recordedWin = 0;  // a replay need no longer be the forward again
   DCU(cudaMemcpyAsync((void *)dst, values, n * 4, cudaMemcpyDefault, b->st));
   DCU(cudaStreamSynchronize(b->st));
   return FB_OK;
@@ -2374,6 +2381,7 @@ extern "C" int fb_diff_batch_forward_ex(fb_diff_batch *b, const fb_diff_params *
   }
   b->recorded = record ? 1 : 0;
   b->recordedK = p->checkpoint;
+  b->recordedWin = record && win ? 1 : 0;
   b->maxSteps = maxSteps;
   for (int k = 0; k < b->B; k++) b->in[k].recordedSteps = record ? steps[k] : 0;
   return FB_OK;
@@ -2535,15 +2543,15 @@ extern "C" int fb_diff_batch_backward(fb_diff_batch *b, const float *const *dL, 
   if ((rc = push_devs(b))) return rc;
   const dim3 ng = neuron_grid(b);
   k_zero_adjoint<<<ng, kDB, 0, b->st>>>(b->dDevs);
-  if (win && b->f32) k_wactive<float><<<ng, kDB, 0, b->st>>>(b->dDevs, b->P32, not_finite(b->P32));
-  else if (win) k_wactive<double><<<ng, kDB, 0, b->st>>>(b->dDevs, b->P64, not_finite(b->P64));
+  if (win && b->f32) k_wactive<float><<<ng, kDB, 0, b->st>>>(b->dDevs, b->P32, not_finite(b->P32), b->recordedWin);
+  else if (win) k_wactive<double><<<ng, kDB, 0, b->st>>>(b->dDevs, b->P64, not_finite(b->P64), b->recordedWin);
   for (int k = 0; k < b->B; k++) DCU(cudaMemsetAsync(b->in[k].D.nonfinite, 0, 8, b->st));
   if ((rc = prepare(b, &b->lastP))) return rc;
   const int32_t steps = b->maxSteps;
   const int nseg = (steps + K - 1) / K;
   b->arenaBufs = bufs;
   PassKey key = pass_key(b, 'B');
-  key.add(steps).add(K).add(truncate).add(loss_from).add(bufs).add(win).add(b->in[0].D.coba);
+  key.add(steps).add(K).add(truncate).add(loss_from).add(bufs).add(win).add(b->in[0].D.coba).add(b->recordedWin);
   // Segments are replayed on the main stream (one after another: they share the forward state)
   // and swept in reverse on the reverse stream (one after another: they share the adjoint
   // state). With two arena halves, segment sg's replay writes half sg & 1 and may run while the
@@ -2558,6 +2566,10 @@ extern "C" int fb_diff_batch_backward(fb_diff_batch *b, const float *const *dL, 
       // replay the segment from its checkpoint (src/lifdiff.js:390-464)
       if (bufs == 2 && sg + 2 < nseg) ev_wait(b, b->st, b->evRev[sg & 1]);
       k_ckpt<<<ng, kDB, 0, b->st>>>(b->dDevs, from, 0);
+      // what the sweep can read: without the windowed forward's marks, anything
+      for (int spikes = 0; win && spikes < 2; spikes++)
+        k_wneed<<<ng, kDB, 0, b->st>>>(b->dDevs, std::max(0, from - b->in[0].D.nslots + 1), std::min(steps, to + K),
+                                       !b->recordedWin, spikes);
       if (win)
         for (int32_t t = from; t < to; t += win) window_replay(b, t, std::min(to, t + win), half + t - from);
       else

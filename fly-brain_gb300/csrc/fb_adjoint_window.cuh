@@ -208,8 +208,15 @@ __global__ void __launch_bounds__(kDB, 4) k_wdeliver(const DiffDev *Ds, DP<R> P,
       for (int u = 0; u < kEdgeILP; u++) {
         const uint32_t e = j0 + 32u * u;
         on[u] = e < hi && D.gate[e];
+        if (on[u]) q[u] = D.indices[e];
+      }
+      if (row >= 0)
+#pragma unroll
+        for (int u = 0; u < kEdgeILP; u++) on[u] = on[u] && D.wNeed[q[u]];
+#pragma unroll
+      for (int u = 0; u < kEdgeILP; u++) {
+        const uint32_t e = j0 + 32u * u;
         if (!on[u]) continue;
-        q[u] = D.indices[e];
         c[u] = make_uint4(key, e, 0u, 0u);
         if (ex) {
           const float dlt = D.W32[e] * sv;
@@ -312,7 +319,7 @@ __device__ __forceinline__ int wn_run(const DiffDev &D, const DP<R> &P, int i, b
     if (REPLAY && own && hasAd && !wasRefr) D.aAd[at] = x.ad;
     if (!wasRefr) {
       const R thr = P.vThresh + (R)x.ad + kc + (R)thrO;
-      if (REPLAY) wild |= !(fabs(vi - thr) <= (R)3e38);
+      wild |= !(fabs(vi - thr) <= (R)3e38);
       if (vi >= thr) {
         s = 1;
         fired = j;
@@ -324,7 +331,7 @@ __device__ __forceinline__ int wn_run(const DiffDev &D, const DP<R> &P, int i, b
     if (REPLAY && own) D.aMode[at] = (uint8_t)(md | s << 2);
     x.v = (float)vi;
   }
-  if (REPLAY && own && wild) D.wAct[i] = 1;  // zero times infinity
+  if (own && wild) (REPLAY ? D.wAct : D.wWild)[i] = 1;  // zero times infinity
   return fired;
 }
 
@@ -340,19 +347,48 @@ __device__ __forceinline__ uint32_t wn_count(const DiffDev &D, int i, bool own, 
   return n;
 }
 
-// Replay of the window (k_update for h steps of a replay), a neuron per lane.
+// The neurons whose replay the reverse sweep reads (all: every one): those whose adjoint may not be
+// zero, and those with a spike on the tape in steps [e0, e1) -- the segment's, the D steps' before
+// it, whose spikes arrive in it, and the next segment's, whose sweep runs beside this replay: only a
+// neuron with such a spike can be handed an adjoint from then on. A neuron's own trajectory needs
+// the tape's spikes and nothing else of the others'. Two launches: 0 copies the marks, 1 adds the
+// spikes'.
+__global__ void k_wneed(const DiffDev *Ds, int32_t e0, int32_t e1, int32_t all, int32_t spikes) {
+  __shared__ DiffDev D;
+  load_dev(Ds, D);
+  const int64_t s0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, ns = (int64_t)gridDim.x * blockDim.x;
+  if (!spikes) {
+    for (int64_t i = s0; i < D.N; i += ns) D.wNeed[i] = all || D.wAct[i];
+    return;
+  }
+  e0 = min(e0, D.steps);
+  e1 = min(e1, D.steps);
+  const int64_t a1 = min(D.tOff[e1], D.tapeCap);
+  for (int64_t a = D.tOff[e0] + s0; a < a1; a += ns) D.wNeed[D.tIdx[a]] = 1;
+}
+
+// Replay of the window (k_update for h steps of a replay) for the needed neurons of each tile of
+// 256, gathered so that they fill warps, a neuron per lane.
 template <typename R, bool CUBA>
 __global__ void __launch_bounds__(kDB, 4) k_wreplay(const DiffDev *Ds, DP<R> P, int32_t t0, int32_t t1, int32_t row) {
   __shared__ DiffDev D;
   __shared__ uint4 stage[kDB / 32][kWSort * 32];
+  __shared__ uint16_t mark[kDB];
+  __shared__ uint32_t nMark;
   load_dev(Ds, D);
   const int h = min(t1, D.steps) - t0;
   if (h <= 0) return;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const int N = D.N, nW = (N + 31) / 32;
-  for (int wt = blockIdx.x * (kDB / 32) + warp; wt < nW; wt += gridDim.x * (kDB / 32)) {
-    const int i0 = wt * 32 + (int)lane, i = i0 < N ? i0 : N - 1;
-    const bool own = i0 < N;
+  const int N = D.N;
+  for (int tile = blockIdx.x * kDB; tile < N; tile += gridDim.x * kDB) {
+    __syncthreads();
+    if (threadIdx.x == 0) nMark = 0;
+    __syncthreads();
+    if (tile + (int)threadIdx.x < N && D.wNeed[tile + threadIdx.x]) mark[atomicAdd(&nMark, 1u)] = (uint16_t)threadIdx.x;
+    __syncthreads();
+    if (warp * 32 >= nMark) continue;
+    const bool own = threadIdx.x < nMark;
+    const int i = tile + mark[own ? threadIdx.x : warp * 32];
     uint32_t o;
     WNeuron x = wn_load(D, i);
     const int arr = (int)D.wArr[i] - 1, frc = (int)D.wForced[i] - 1;
@@ -702,17 +738,17 @@ __global__ void k_wsums(const DiffDev *Ds, DP<R> P) {
 // term is a product with it). wAct marks the neurons that may have one: at the pass's start those
 // with a loss gradient, then those k_wbarrival hands one to; also every neuron whose products with
 // zero need not be zero (a potential, threshold or surrogate width that is not finite, `dense` for
-// the parameters). The others' rows of wE and wI stay zero. 1% of the neurons of a full brain with
+// the parameters, wWild the recorded forward's). The others' rows of wE and wI stay zero. 1% of the neurons of a full brain with
 // 1,000 readouts are ever marked.
 template <typename R>
-__global__ void k_wactive(const DiffDev *Ds, DP<R> P, int32_t dense) {
+__global__ void k_wactive(const DiffDev *Ds, DP<R> P, int32_t dense, int32_t fromForward) {
   __shared__ DiffDev D;
   load_dev(Ds, D);
   const int64_t N = D.N, s0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, ns = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = s0; i < N; i += ns) {
     const bool loss = D.dL && (D.roMap ? D.roMap[i] >= 0 : !(D.dL[i] == 0.f));
     const float thr = D.thrOffset[i];
-    D.wAct[i] = dense || loss || thr != thr || !(d_beta<R>(D, P, (int)i) > R(1e-30));
+    D.wAct[i] = dense || loss || (fromForward && D.wWild[i]) || thr != thr || !(d_beta<R>(D, P, (int)i) > R(1e-30));
   }
   for (int64_t k = s0; k < 2 * D.wRows * N; k += ns) D.wE[k] = 0.f;  // and wI behind it
 }

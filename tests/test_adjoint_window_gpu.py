@@ -150,3 +150,29 @@ def test_what_the_sweep_leaves_out(what, precision):
         scale = np.abs(x[ok]).max() if ok.any() else 0.0
         assert np.abs(x[ok] - y[ok]).max() <= 1e-6 * scale + 1e-30, k
     assert a["clamped"] == b["clamped"]
+
+
+@pytest.mark.parametrize("model", [CUBA, COBA])
+@pytest.mark.parametrize("K,truncate,steps", [(1, 0, 45), (7, 0, 61), (18, 0, 90), (40, 23, 130)])
+def test_losses_on_few_neurons(model, K, truncate, steps):
+    """The replay of a segment runs the neurons that the sweep can reach; segments shorter and longer
+    than the delay, against the oracle. Values set to what they are between the passes give up the
+    selection and nothing else."""
+    N = 300
+    ins = hub_net(N, 1, K, deg=4)
+    rng = np.random.default_rng(K)
+    driven = rng.permutation(N)[:60].astype(np.int32)
+    p = dict(model, checkpoint=K)
+    prob, net = _pair(ins, p, driven, np.full(60, 900.0))
+    sc0, tape = prob.forward(steps, seed=5, checkpoint=K)
+    assert sc0.tobytes() == net.forward(steps, seed=5).tobytes()
+    dL = np.zeros(N, np.float32)
+    dL[rng.permutation(N)[:3]] = rng.normal(0, 1, 3)
+    g0 = prob.backward(tape, dL, truncate=truncate, lossFrom=0)
+    g1 = net.backward(dL, truncate=truncate, lossFrom=0)
+    _compare_grads(g0, g1)
+    net.set_array("thrOffset", np.zeros(N, np.float32))
+    g2 = net.backward(dL, truncate=truncate, lossFrom=0)
+    assert g1["params"] == g2["params"]
+    for k in ("logGain", "bias", "edge"):
+        np.testing.assert_array_equal(g1[k], g2[k])
