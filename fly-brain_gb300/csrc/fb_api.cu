@@ -442,8 +442,9 @@ struct WinRes {
   size_t smem = 0;
   uint32_t barBase = 0;                  // grid-barrier arrivals so far
   int maxD = 0;
-  // where the spikes in flight are: the ring's lists, the log, or both
-  bool ringValid = true, logValid = true;
+  // where the spikes in flight are: the ring's lists, the log, or both; and whether the grid
+  // kernel's slot records are those of the lists
+  bool ringValid = true, logValid = true, slotsValid = true;
 };
 
 struct fb_brains {
@@ -1247,7 +1248,7 @@ static int win_launch(fb_brains *br, const std::vector<int32_t> &steps, int hCap
   CU(launch_window(a, br->sms, R.smem, br->stream));
   R.barBase += (uint32_t)br->sms * (uint32_t)(a.nWin * (a.anyBg ? 3 : 2) - 1);  // arrivals of the launch
   R.logValid = true;
-  R.ringValid = false;
+  R.ringValid = R.slotsValid = false;
   return FB_OK;
 }
 
@@ -1319,7 +1320,7 @@ static int win_recover(fb_brains *br, bool backup) {
     CU(cudaMemcpyAsync(br->trials, R.backup + st, sizeof(Trial), cudaMemcpyDeviceToDevice, br->stream));
   }
   R.ringValid = true;
-  R.logValid = false;
+  R.logValid = R.slotsValid = false;
   CU(cudaStreamSynchronize(br->stream));
   return FB_OK;
 }
@@ -1367,10 +1368,9 @@ static int run_steps(fb_brains *br, int32_t maxSteps, int32_t *out_nfired) {
     }
   } else if (maxSteps > 0) {
     br->lastSchedule = FB_SCHEDULE_GRID;
-    if (br->win.ready && !br->win.ringValid) {
-      if ((rc = ring_from_log(br))) return rc;
-      CU(launch_rebuild_slots(br->trials, br->B, br->maxSlots, br->d_err, br->stream));
-    }
+    if ((rc = ring_from_log(br))) return rc;
+    if (!br->win.slotsValid) CU(launch_rebuild_slots(br->trials, br->B, br->maxSlots, br->d_err, br->stream));
+    br->win.slotsValid = true;
     br->win.logValid = false;
     br->everGrid = true;
     br->irregular = std::max(0, br->irregular - maxSteps);
