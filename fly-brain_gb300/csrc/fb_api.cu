@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "fb_internal.cuh"
+#include "fb_lagged.cuh"
 #include "fb_window.cuh"
 
 namespace fb {
@@ -428,6 +429,27 @@ struct DrivenSet {
   }
 };
 
+// Device resources of the lagged kernel (fb_lagged.cu) for a single brain, allocated at its first
+// use at the largest sizes the brain can need.
+struct LagRes {
+  bool ready = false;
+  bool noMemory = false;  // the allocation failed: AUTO does not try again
+  int D = 0, S = 0, nTB = 0, capMax = 0, nDmax = 0, bgCap = 0, grid = 0;
+  uint64_t drivenVersion = ~0ull;
+  std::vector<void *> allocs;
+  uint32_t *cnt = nullptr, *pend0 = nullptr, *sync = nullptr, *bgList = nullptr;
+  uint32_t *jumpHex = nullptr;
+  uint4 *edgeRec = nullptr;
+  uint2 *buf = nullptr;
+  uint4 *dbList = nullptr;
+  int32_t *bgCount = nullptr, *dbCnt = nullptr, *dbNF = nullptr, *tStage = nullptr, *tCnt = nullptr;
+  int32_t *ndIds = nullptr, *ndLo = nullptr, *drvPosOf = nullptr;
+  int cap = 1, nD = 0;
+  int nDB = 1, nDcap = 32, nDall = 32, dLo[kLagMaxDB + 1] = {0, 0, 0};
+  unsigned long long *liveTag = nullptr;
+  size_t smem = 0;
+};
+
 // Device resources of the windowed kernel (fb_window.cu), allocated at its first use.
 struct WinRes {
   bool ready = false;
@@ -489,16 +511,17 @@ struct fb_brains {
   int32_t subGrab = 4;
   int64_t timeoutNs = 5000000000LL;  // bound of every device-side wait (fb_tuning.timeout_us)
   int32_t tripStep = -1;             // test hook (fb_debug_trip_wait): armed for one launch
-  int32_t lagDB = 0;                 // fb_tuning.lag_driven_blocks (accepted; the schedule needs none)
+  int32_t lagDB = 0;                 // driven blocks of the lagged kernel (0: automatic)
   int32_t irregular = 0;             // steps in which a neuron may fire sooner than its refractory time
   int logging = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float lastMs = 0.f;
   int32_t schedule = FB_SCHEDULE_AUTO, lastSchedule = FB_SCHEDULE_GRID;
+  LagRes lag;
   WinRes win;
   std::vector<Topology *> topo;      // each brain's (the graphs outlive the batch)
   int maxSlots = 0;
-  bool everGrid = false;             // the grid kernel has run
+  bool everRing = false;             // a kernel that keeps the ring's lists has run
 };
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -703,6 +726,7 @@ extern "C" int fb_brains_destroy(fb_brains *br) {
   cudaFree(br->d_phase);
   cudaFree(br->d_dbg);
   cudaFree(br->d_ovf[0]); cudaFree(br->d_ovf[1]);
+  for (void *p : br->lag.allocs) cudaFree(p);
   for (void *p : br->win.allocs) cudaFree(p);
   cudaFree(br->win.arena);
   if (br->ev0) cudaEventDestroy(br->ev0);
@@ -731,9 +755,12 @@ extern "C" int fb_brains_set_tuning(fb_brains *br, const fb_tuning *t) {
     return fail(FB_EINVAL, "fb_brains_set_tuning: blocks_per_sm %d (1..%d), item_chunks %d (1..64), sub_grab %d (-1, 1..256), "
                 "timeout_us %d (>= 1)", t->blocks_per_sm, br->maxBlocksPerSm, t->item_chunks, t->sub_grab, t->timeout_us);
   if (t->timeout_us) br->timeoutNs = (int64_t)t->timeout_us * 1000;
-  if (t->lag_driven_blocks < 0 || t->lag_driven_blocks > 2)
-    return fail(FB_EINVAL, "fb_brains_set_tuning: lag_driven_blocks %d (0..2)", t->lag_driven_blocks);
-  br->lagDB = t->lag_driven_blocks;
+  if (t->lag_driven_blocks < 0 || t->lag_driven_blocks > kLagMaxDB)
+    return fail(FB_EINVAL, "fb_brains_set_tuning: lag_driven_blocks %d (0 automatic, 1..%d)", t->lag_driven_blocks, kLagMaxDB);
+  if (t->lag_driven_blocks != br->lagDB) {
+    br->lagDB = t->lag_driven_blocks;
+    br->lag.drivenVersion = ~0ull;  // the ownership is recomputed at the next launch
+  }
   if (t->blocks_per_sm) {
     br->blocksPerSm = t->blocks_per_sm;
     br->grid = br->sms * br->blocksPerSm;
@@ -1000,7 +1027,7 @@ extern "C" int fb_set_params(fb_brains *br, int32_t b, const fb_params *p) {
       if ((rc = ring_from_log(br))) return rc;
       CU(cudaStreamSynchronize(br->stream));
       br->win.ready = false;
-      br->everGrid = true;
+      br->everRing = true;
     }
   }
   T.coba = nt.coba;
@@ -1021,7 +1048,202 @@ extern "C" int fb_set_params(fb_brains *br, int32_t b, const fb_params *p) {
   return FB_OK;
 }
 
-// ---- the windowed (delay-scheduled) kernel -------------------------------------------------------
+// ---- the lagged kernel: the delay-scheduled kernel where windows are short ------------------------
+
+// AUTO: shorter launches take another kernel. The lagged launch carries a fixed ~110 us (clearing its
+// buffers, loading every block's state into shared memory and writing it back) against the grid
+// kernel's ~15 us; at the full graph they break even near 6 steps (grid 20-26 us per step, lagged
+// 4-7).
+constexpr int kLagMinSteps = 8;
+
+// Whether the delay-scheduled schedule applies to this launch (why not, in *why).
+static bool lag_applies(fb_brains *br, int32_t steps, const char **why) {
+  const Trial &T = br->host[0];
+  *why = nullptr;
+  if (br->B != 1) *why = "a batch of more than one brain";
+  else if (T.mode != FB_DELIVER_EXACT || (T.flags & kHasPreInh)) *why = "a delivery mode other than exact without presynaptic inhibition";
+  else if (br->profiling && br->schedule != FB_SCHEDULE_LAGGED) *why = "phase profiling";
+  else if (br->logging && steps > kLagRing) *why = "per-step logging of a launch longer than 64 steps";
+  // a block's wait at step s (for step s - L, L = D - help) must not need its own completion of
+  // that step, which it publishes at step s - L + 1: L >= 2
+  else if (T.nslots - 1 < 4 || T.nslots - 1 > 32) *why = "a ring depth outside 5..33 slots";
+  else if (T.bgEvents > (float)(1 << 20)) *why = "more than 2^20 background events per step";
+  return *why == nullptr;
+}
+
+template <typename X>
+static int lag_alloc(fb_brains *br, X **p, size_t n) {
+  void *q = nullptr;
+  if (cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(X)) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(FB_ENOMEM, "fb_step: %zu bytes for the lagged kernel", n * sizeof(X));
+  }
+  br->lag.allocs.push_back(q);
+  *p = (X *)q;
+  return FB_OK;
+}
+
+// Allocates the kernel's resources and (when the driven set changed) the neuron ownership.
+static int lag_setup(fb_brains *br) {
+  LagRes &R = br->lag;
+  Trial &T = br->host[0];
+  const int N = T.N;
+  const int64_t E = T.E;
+  int rc;
+  if (!R.ready) {
+    int sms = 0, optin = 0;
+    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, br->dev));
+    CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, br->dev));
+    R.grid = sms;
+    R.nTB = sms - 1;
+    R.D = T.nslots - 1;
+    R.S = 2 * R.D;
+    // tile blocks hold at most ceil(N / (sms - kLagMaxDB)) neurons (the fewest tile blocks)
+    R.capMax = std::max(1, (N + sms - kLagMaxDB - 1) / (sms - kLagMaxDB));
+    int perDB = 0;  // driven entries one driven block holds at most
+    for (int nd = 32; nd <= kLagPer * kLagThreads; nd += 32)
+      if (lagged_smem_bytes(R.capMax, nd, kLagMaxDB * nd) <= (size_t)optin) perDB = nd;
+    if (perDB == 0) return fail(FB_EINVAL, "fb_step: the lagged kernel does not fit in shared memory");
+    R.nDmax = kLagMaxDB * perDB;
+    std::vector<uint32_t> tab;
+    lagged_jump_tables(tab);
+    if ((rc = lag_alloc(br, &R.cnt, (size_t)R.S * (N + R.nDmax))) ||
+        (rc = lag_alloc(br, &R.buf, (size_t)R.S * std::max<int64_t>(E, 1))) || (rc = lag_alloc(br, &R.pend0, N)) ||
+        (rc = lag_alloc(br, &R.sync, 256)) || (rc = lag_alloc(br, &R.bgCount, kLagRing)) ||
+        (rc = lag_alloc(br, &R.dbList, (size_t)kLagRing * R.nDmax * 2)) ||
+        (rc = lag_alloc(br, &R.dbCnt, (size_t)kLagRing * kLagMaxDB)) ||
+        (rc = lag_alloc(br, &R.liveTag, (size_t)kLagRing * kLagMaxDB)) ||
+        (rc = lag_alloc(br, &R.dbNF, kLagRing)) || (rc = lag_alloc(br, &R.tStage, (size_t)kLagRing * R.grid * R.capMax)) ||
+        (rc = lag_alloc(br, &R.tCnt, (size_t)kLagRing * R.grid)) || (rc = lag_alloc(br, &R.ndIds, N)) ||
+        (rc = lag_alloc(br, &R.ndLo, R.grid + 1)) || (rc = lag_alloc(br, &R.drvPosOf, N)) || (rc = lag_alloc(br, &R.edgeRec, std::max<int64_t>(E, 1))) ||
+        (rc = lag_alloc(br, &R.jumpHex, tab.size()))) {
+      for (void *p : R.allocs) cudaFree(p);
+      R.allocs.clear();
+      R.noMemory = true;
+      return rc;
+    }
+    CU(cudaMemcpyAsync(R.jumpHex, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice, br->stream));
+    CU(cudaStreamSynchronize(br->stream));
+    R.ready = true;
+  }
+  const DrivenSet &ds = br->driven[0];
+  const int bgNeed = T.bgEvents > 0 ? (int)std::ceil((double)T.bgEvents) + 1 : 1;
+  if ((int64_t)ds.order.size() + bgNeed + 64 >= 65536)
+    return fail(FB_EINVAL, "fb_step: %lld draws per step exceed the lagged kernel's jump tables",
+                (long long)ds.order.size() + bgNeed);
+  if (bgNeed > R.bgCap) {
+    if ((rc = lag_alloc(br, &R.bgList, (size_t)kLagRing * bgNeed))) return rc;
+    R.bgCap = bgNeed;
+  }
+  if (ds.version != R.drivenVersion) {
+    const int nD = (int)ds.order.size();
+    if (nD > R.nDmax) return fail(FB_EINVAL, "fb_step: %d driven neurons exceed the lagged kernel's %d", nD, R.nDmax);
+    std::vector<uint8_t> isD(N, 0);
+    for (int32_t i : ds.order) isD[i] = 1;
+    std::vector<int32_t> nd;
+    nd.reserve(N - nD);
+    for (int i = 0; i < N; i++)
+      if (!isD[i]) nd.push_back(i);
+    const int64_t Nnd = (int64_t)nd.size();
+    // a long driven list is split over two driven blocks in list order (their draws stay in
+    // lif.c's order: each offsets its own by the other's share); the other SMs are tile blocks
+    R.nDB = br->lagDB ? br->lagDB : nD >= kLagSplit ? 2 : 1;
+    if (R.nDB > 1 && nD < R.nDB) R.nDB = 1;  // every driven block owns at least one entry
+    R.nTB = R.grid - R.nDB;
+    for (int d = 0; d <= R.nDB; d++) R.dLo[d] = (int)((int64_t)nD * d / R.nDB);
+    int part = 0;
+    for (int d = 0; d < R.nDB; d++) part = std::max(part, R.dLo[d + 1] - R.dLo[d]);
+    std::vector<int32_t> lo(R.nTB + 1);
+    for (int t = 0; t <= R.nTB; t++) lo[t] = (int32_t)(Nnd * t / R.nTB);
+    std::vector<int32_t> posOf(N, -1);
+    for (int k = 0; k < nD; k++) posOf[ds.order[k]] = k;
+    if (Nnd) CU(cudaMemcpyAsync(R.ndIds, nd.data(), Nnd * 4, cudaMemcpyHostToDevice, br->stream));
+    CU(cudaMemcpyAsync(R.ndLo, lo.data(), (R.nTB + 1) * 4, cudaMemcpyHostToDevice, br->stream));
+    CU(cudaMemcpyAsync(R.drvPosOf, posOf.data(), (size_t)N * 4, cudaMemcpyHostToDevice, br->stream));
+    CU(launch_edge_records(T.indices, T.dup, br->topo[0]->inOff, R.drvPosOf, N, E, R.edgeRec, br->stream));
+    CU(cudaStreamSynchronize(br->stream));
+    R.nD = nD;
+    R.cap = std::max<int>(1, (int)((Nnd + R.nTB - 1) / R.nTB));
+    if (R.cap > std::min(R.capMax, kLagPer * kLagTileWorkers) || part > kLagPer * kLagThreads ||
+        (nD + R.nTB - 1) / R.nTB > kLagHelpMax)
+      return fail(FB_EINVAL, "fb_step: %d neurons per tile block (at most %d) or %d driven neurons per driven block "
+                  "(at most %d) exceed the lagged kernel", R.cap, std::min(R.capMax, kLagPer * kLagTileWorkers),
+                  part, kLagPer * kLagThreads);
+    R.nDcap = std::max(32, (part + 31) / 32 * 32);
+    R.nDall = std::max(32, (nD + 31) / 32 * 32);
+    R.smem = lagged_smem_bytes(R.cap, R.nDcap, R.nDall);
+    if (lagged_blocks_per_sm(R.smem) < 1)
+      return fail(FB_EINVAL, "fb_step: the lagged kernel does not fit on an SM (%zu bytes)", R.smem);
+    R.drivenVersion = ds.version;
+  }
+  return FB_OK;
+}
+
+// `steps` steps of one brain: the spikes in flight come from and go to the ring's lists.
+static int run_lagged(fb_brains *br, int32_t steps) {
+  LagRes &R = br->lag;
+  Trial &T = br->host[0];
+  const int N = T.N;
+  CU(cudaEventRecord(br->ev0, br->stream));  // the launch's clearing is part of its time
+  int rc = ring_from_log(br);
+  if (rc) return rc;
+  CU(cudaMemsetAsync(R.sync, 0, 256 * 4, br->stream));
+  CU(cudaMemsetAsync(R.cnt, 0, (size_t)R.S * (N + R.nDmax) * 4, br->stream));
+  CU(cudaMemsetAsync(R.pend0, 0, (size_t)N * 4, br->stream));
+  CU(cudaMemsetAsync(R.liveTag, 0, sizeof(unsigned long long) * kLagRing * kLagMaxDB, br->stream));
+  LagArgs a;
+  memset(&a, 0, sizeof a);
+  a.G = br->trials;
+  a.N = N;
+  a.E = T.E;
+  a.T = steps;
+  a.D = R.D;
+  a.S = R.S;
+  a.help = lag_help(R.D);
+  a.dbPub = a.help - 1;
+  a.L = R.D - a.help;
+  a.nTB = R.nTB;
+  a.cap = R.cap;
+  a.nD = R.nD;
+  a.nDcap = R.nDcap;
+  a.nDall = R.nDall;
+  a.nDB = R.nDB;
+  for (int d = 0; d <= kLagMaxDB; d++) a.dLo[d] = R.dLo[std::min(d, R.nDB)];
+  a.hasBg = T.bgEvents > 0 ? 1 : 0;
+  a.bgCap = R.bgCap;
+  a.dt = T.dt; a.vRest = T.vRest; a.vThresh = T.vThresh; a.vReset = T.vReset; a.tRef = T.tRef;
+  a.adaptInc = T.adaptInc; a.depU = T.depU; a.dE = T.dE; a.dTr = T.dTr; a.dA = T.dA; a.kRec = T.kRec;
+  a.kM = T.kM; a.dtS = T.dtS; a.eExc = T.eExc; a.eInh = T.eInh; a.cE = T.cE; a.cI = T.cI;
+  a.bgEvents = T.bgEvents; a.bgAmp = T.bgAmp; a.coba = T.coba;
+  a.indptr = T.indptr; a.indices = T.indices; a.W = T.W; a.sign = T.sign; a.inOff = br->topo[0]->inOff;
+  a.v = T.v; a.gE = T.gE; a.gI = T.gI; a.refr = T.refr; a.trace = T.trace; a.adapt = T.adapt; a.res = T.res;
+  a.bias = T.bias; a.thr = T.thr; a.drive = T.drive; a.spikeCount = T.spikeCount;
+  a.ring = T.ring; a.ringCount = T.ringCount; a.driven = T.driven;
+  a.ndIds = R.ndIds; a.ndLo = R.ndLo; a.drvPosOf = R.drvPosOf;
+  a.cnt = R.cnt; a.cntStride = N + R.nDmax; a.buf = R.buf; a.pend0 = R.pend0;
+  a.done = R.sync; a.dbDone = R.sync + 64; a.bgReady = R.sync + 72; a.barCount = R.sync + 128;
+  a.liveTag = R.liveTag;
+  a.stepTot = (int32_t *)(R.sync + 192);
+  a.bgList = R.bgList; a.bgCount = R.bgCount; a.dbList = R.dbList; a.dbCnt = R.dbCnt;
+  a.tStage = R.tStage; a.tCnt = R.tCnt;
+  a.log = br->logging;
+  a.logCount = T.logCount; a.logRaster = T.logRaster; a.logCap = T.logCap; a.logRasterCap = T.logRasterCap;
+  a.prof = br->profiling ? br->d_phase : nullptr;
+  a.jumpHex = R.jumpHex;
+  a.edgeRec = R.edgeRec;
+  a.err = br->d_err;
+  a.timeoutNs = br->timeoutNs;
+  a.tripStep = br->tripStep;
+  br->tripStep = -1;  // one launch only
+  CU(launch_lagged(a, R.grid, R.smem, br->stream));
+  br->win.logValid = br->win.slotsValid = false;
+  br->everRing = true;
+  CU(cudaEventRecord(br->ev1, br->stream));
+  br->lastSchedule = FB_SCHEDULE_LAGGED;
+  return FB_OK;
+}
+
+// ---- the windowed kernel ------------------------------------------------------------------------
 
 // AUTO takes the windowed kernel from this many steps on. Measured on one brain (microseconds per
 // call, spike counts read back; grid / windowed): 165,122 neurons, 2 steps 83 / 62, 16 steps 354 /
@@ -1059,8 +1281,7 @@ static int window_steps(const Trial &T, int64_t nD) {
   return (int)std::min<int64_t>({T.nslots - 1, std::max(1, silent_steps(T)), kWinMax, drawn_steps(T, nD)});
 }
 
-// Whether the windowed kernel can run this batch at all, and whether it applies to this launch
-// under the delay-scheduled schedule (why not, in *why).
+// Whether the windowed kernel can run this batch at all.
 static bool win_capable(const fb_brains *br) {
   if (br->B > kWinBrains) return false;
   for (int b = 0; b < br->B; b++) {
@@ -1073,18 +1294,6 @@ static bool win_capable(const fb_brains *br) {
   }
   return true;
 }
-static bool lag_applies(fb_brains *br, int32_t steps, const char **why) {
-  const Trial &T = br->host[0];
-  *why = nullptr;
-  if (br->B != 1) *why = "a batch of more than one brain";
-  else if (T.mode != FB_DELIVER_EXACT || (T.flags & kHasPreInh)) *why = "a delivery mode other than exact without presynaptic inhibition";
-  else if (br->logging && steps > kWinLogSteps) *why = "per-step logging of a launch longer than 64 steps";
-  else if (T.nslots - 1 < 4 || T.nslots - 1 > 32) *why = "a ring depth outside 5..33 slots";
-  else if (T.bgEvents > (float)(1 << 20)) *why = "more than 2^20 background events per step";
-  else if ((int)br->driven[0].order.size() > kWinDriven) *why = "more than 4096 driven neurons";
-  return *why == nullptr;
-}
-
 template <typename X>
 static int win_alloc(fb_brains *br, X **p, size_t n) {
   void *q = nullptr;
@@ -1173,7 +1382,7 @@ static int win_create(fb_brains *br, bool early) {
   CU(cudaMemcpyAsync(R.win, R.host.data(), sizeof(WinBrain) * B, cudaMemcpyHostToDevice, br->stream));
   CU(cudaStreamSynchronize(br->stream));
   R.ready = true;
-  R.logValid = !br->everGrid;  // nothing in flight yet, unless the grid kernel ran
+  R.logValid = !br->everRing;  // nothing in flight yet, unless another kernel ran
   return FB_OK;
 }
 
@@ -1325,25 +1534,69 @@ static int win_recover(fb_brains *br, bool backup) {
   return FB_OK;
 }
 
+// One brain's launches of n steps that the lagged kernel runs faster: it takes about the same time a
+// step whatever the window's length H, a window costs its round trips however short it is.
+// Microseconds per launch, windowed / lagged, current-based at dt 0.1 ms, 20,000 neurons: H 1, 8 steps
+// 148 / 116, 512 steps 5,927 / 1,501; H 2, 8 steps 100 / 118, 16 steps 152 / 138, 512 steps 3,151 /
+// 1,506; H 3, 32 steps 184 / 176, 64 steps 323 / 272; H 4, 64 steps 259 / 273, 512 steps 1,680 / 1,502;
+// H 5, 512 steps 1,411 / 1,507. At H 4 the two are close: over 1,501 to 165,122 neurons and dt 0.1 and
+// 0.5 ms, 512 steps, windowed over lagged 0.83 to 1.21 without background events (mean 1.04); with them
+// 0.73 to 1.04 up to 60,013 neurons, 0.98 and 1.19 at 165,122 (there 64 steps 645 / 617, 32 steps 349 /
+// 367 at dt 0.5 ms). The lagged kernel's tile blocks hold at most kLagPer neurons per thread.
+static bool lag_better(const fb_brains *br, int32_t n) {
+  const Trial &T = br->host[0];
+  const int tb = br->sms - kLagMaxDB;
+  if (br->B != 1 || (T.N + tb - 1) / tb > kLagPer * kLagTileWorkers) return false;
+  switch (window_steps(T, (int64_t)br->driven[0].order.size())) {
+    case 1: return n >= kLagMinSteps;
+    case 2: return n >= 16;
+    case 3: return n >= 64;
+    case 4: return T.N >= 100000 ? n >= 64 : n >= 128 && T.bgEvents <= 0;
+    default: return false;
+  }
+}
+
+// The lagged kernel counts on one spike per neuron and step. With a refractory time under one step a
+// forced neuron is not refractory at its step's end and fires again if the reset potential crosses its
+// threshold.
+static bool fires_once_a_step(const Trial &T) {
+  return silent_steps(T) >= 1 || (T.vReset < T.vThresh && (T.flags & kThrZero) && T.adaptInc >= 0);
+}
+
+enum class StepKernel { kGrid, kLagged, kWindow };
+
+// The kernel of this launch, its resources ready.
+static int choose_kernel(fb_brains *br, int32_t n, StepKernel *k) {
+  *k = StepKernel::kGrid;
+  if (n == 0 || br->schedule == FB_SCHEDULE_GRID) return FB_OK;
+  const bool forced = br->schedule == FB_SCHEDULE_LAGGED;
+  const char *why = nullptr;
+  const bool applies = lag_applies(br, n, &why);
+  if (forced && !applies) return fail(FB_EINVAL, "fb_step: the delay-scheduled schedule does not apply to %s", why);
+  const bool window = win_capable(br) && !br->win.noMemory &&
+                      (forced || (n >= win_min_steps(br) && !br->profiling && (!br->logging || (br->B == 1 && n <= kWinLogSteps))));
+  const bool lagged = applies && fires_once_a_step(br->host[0]) && (forced || (n >= kLagMinSteps && !br->lag.noMemory));
+  int rc = FB_OK;
+  // the better one first, the other where its memory cannot be had
+  for (int k2 = 0; k2 < 2; k2++) {
+    const bool lagTurn = lag_better(br, n) == (k2 == 0);
+    if (lagTurn ? !lagged : !window) continue;
+    rc = lagTurn ? lag_setup(br) : win_setup(br);
+    if (rc == FB_OK) {
+      *k = lagTurn ? StepKernel::kLagged : StepKernel::kWindow;
+      return FB_OK;
+    }
+  }
+  if (forced) return rc;
+  g_err.clear();
+  return FB_OK;
+}
+
 static int run_steps(fb_brains *br, int32_t maxSteps, int32_t *out_nfired) {
   int rc = flush(br, false);
   if (rc) return rc;
-  bool windowed = false;
-  if (maxSteps > 0 && br->schedule != FB_SCHEDULE_GRID) {
-    const bool may = br->schedule == FB_SCHEDULE_AUTO && maxSteps >= win_min_steps(br) && !br->profiling &&
-                     (!br->logging || (br->B == 1 && maxSteps <= kWinLogSteps)) && !br->win.noMemory;
-    if (br->schedule == FB_SCHEDULE_LAGGED) {
-      const char *why = nullptr;
-      if (!lag_applies(br, maxSteps, &why)) return fail(FB_EINVAL, "fb_step: the delay-scheduled kernel does not apply to %s", why);
-      if (win_capable(br)) {
-        if ((rc = win_setup(br))) return rc;
-        windowed = true;
-      }
-    } else if (may && win_capable(br)) {
-      windowed = win_setup(br) == FB_OK;
-      if (!windowed) g_err.clear();
-    }
-  }
+  StepKernel kernel;
+  if ((rc = choose_kernel(br, maxSteps, &kernel))) return rc;
   // the error flag and the fired counts come back in one synchronisation
   auto read_back = [&]() -> int {
     CU(cudaMemcpyAsync(br->h_small, br->d_err, 4, cudaMemcpyDeviceToHost, br->stream));
@@ -1354,7 +1607,19 @@ static int run_steps(fb_brains *br, int32_t maxSteps, int32_t *out_nfired) {
     br->flushPending = false;
     return FB_OK;
   };
-  if (windowed) {
+  if (kernel == StepKernel::kLagged) {
+    if ((rc = run_lagged(br, maxSteps))) return rc;
+    br->irregular = std::max(0, br->irregular - maxSteps);
+    if ((rc = read_back())) return rc;
+    const int32_t err = br->h_small[0];
+    cudaEventElapsedTime(&br->lastMs, br->ev0, br->ev1);
+    if (err) {  // the brain is as it was
+      cudaMemsetAsync(br->d_err, 0, 4, br->stream);
+      cudaStreamSynchronize(br->stream);
+      return fail(err, err == FB_ETIMEOUT ? "fb_step: a device-side wait timed out; the step was abandoned"
+                                          : "fb_step: lagged kernel error %d", err);
+    }
+  } else if (kernel == StepKernel::kWindow) {
     const bool forced = br->schedule == FB_SCHEDULE_LAGGED;
     if ((rc = run_window(br, maxSteps, forced))) return rc;
     if ((rc = read_back())) return rc;
@@ -1372,7 +1637,7 @@ static int run_steps(fb_brains *br, int32_t maxSteps, int32_t *out_nfired) {
     if (!br->win.slotsValid) CU(launch_rebuild_slots(br->trials, br->B, br->maxSlots, br->d_err, br->stream));
     br->win.slotsValid = true;
     br->win.logValid = false;
-    br->everGrid = true;
+    br->everRing = true;
     br->irregular = std::max(0, br->irregular - maxSteps);
     if (br->stepsUploaded != br->stepsHost) {  // the last launch's counts stay on the device otherwise
       std::memcpy(br->h_steps, br->stepsHost.data(), sizeof(int32_t) * br->B);

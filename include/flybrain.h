@@ -137,12 +137,17 @@ int fb_brains_set_mode(fb_brains *br, int32_t mode);
 
 /* Kernel schedules of fb_step (both exact). No counterpart in the reference, whose lif_step is a
  * serial loop. GRID: the persistent two-phase kernel with two grid barriers per step (any batch,
- * mode and logging). LAGGED: the delay-scheduled kernel, which advances the brains in windows of
- * the synaptic delay, for exact mode without presynaptic inhibition (4 <= nslots - 1 <= 32 steps,
- * at most 4,096 driven neurons per brain; per-step logging only for one brain in launches of at
- * most 64 steps). AUTO (default) takes it where it applies and the launch has at least 2 steps (3
- * with background events), GRID otherwise. LAGGED forces it for one brain; where it does not apply
- * fb_step then fails with FB_EINVAL. */
+ * mode and logging). LAGGED: the kernels scheduled by the synaptic delay, for exact mode without
+ * presynaptic inhibition (4 <= nslots - 1 <= 32 steps, at most 4,096 driven neurons per brain;
+ * per-step logging only for one brain in launches of at most 64 steps). One advances the brains in
+ * windows of the delay, at most the steps that a neuron stays refractory; the other, for one brain
+ * and launches of at least 8 steps, takes one step at a time in blocks that synchronise only at the
+ * delay, where windows would be short or do not apply (a refractory time under one step, more draws
+ * than a block's shared memory holds). AUTO (default) takes one of them where they apply and the
+ * launch has at least 2 steps (3 with background events), GRID otherwise. LAGGED forces them for
+ * one brain; where neither applies fb_step then fails with FB_EINVAL. (With a refractory time under
+ * one step and threshold offsets, or vReset >= vThresh, a neuron may fire twice in a step: GRID, under
+ * LAGGED too.) */
 #define FB_SCHEDULE_AUTO 0
 #define FB_SCHEDULE_GRID 1
 #define FB_SCHEDULE_LAGGED 2
@@ -165,8 +170,9 @@ typedef struct fb_tuning {
   int32_t timeout_us;             /* bound of every device-side wait of both schedules, microseconds
                                      (default 5,000,000); a wait that runs out ends the launch with
                                      FB_ETIMEOUT */
-  int32_t lag_driven_blocks;      /* accepted (0..2) and kept; the delay-scheduled kernel runs each
-                                     driven list on one block */
+  int32_t lag_driven_blocks;      /* delay-scheduled kernel of single steps: blocks the driven list
+                                     is split over (1 or 2; 0 = automatic: 2 from 512 driven
+                                     neurons); the windowed one runs each list on one block */
   int32_t pad;
 } fb_tuning;
 int fb_brains_set_tuning(fb_brains *br, const fb_tuning *t);
@@ -176,9 +182,10 @@ int fb_brains_tuning(fb_brains *br, fb_tuning *t);
  * GPU path falls back on a failure, src/brainsetup.js:66-75). Arms the next launch of the
  * delay-scheduled kernel so that one block, at step `step` of that launch, waits on a flag
  * nothing sets: the wait runs out after timeout_us, every other block leaves its own bounded wait,
- * and the call returns FB_ETIMEOUT. A failed launch of that kernel for one brain (forced, or of 8
- * steps and more) leaves the brain as it was before the call (its state is copied first), so the
- * handle steps on from there. Consumed by that one launch; -1 disarms. */
+ * and the call returns FB_ETIMEOUT. A failed delay-scheduled launch for one brain (forced, or of 8
+ * steps and more) leaves the brain as it was before the call (its state is copied first, or lives in
+ * shared memory until the launch completes), so the handle steps on from there. Consumed by that
+ * one launch; -1 disarms. */
 int fb_debug_trip_wait(fb_brains *br, int32_t step);
 
 /* Advances every brain by nsteps steps in one persistent launch (lif_step, src/wasm/lif.c:29-80,
@@ -255,13 +262,18 @@ int fb_last_step_ms(fb_brains *br, float *ms);
  * [3] the neuron update, [4] the wait at the second barrier; within [0], for the brain block 0
  * serves: [5] the header and background draws, [6] the driven-list gathers, [7] the draws,
  * [8] the forced spikes' emission, [9] the RNG advance. fb_phase_times copies up to n
- * accumulated totals in ms. With the schedule forced to FB_SCHEDULE_LAGGED the delay-scheduled
- * kernel runs instead (AUTO takes the grid kernel while profiling) and the slots hold, for block 0,
+ * accumulated totals in ms. With the schedule forced to FB_SCHEDULE_LAGGED a delay-scheduled
+ * kernel runs instead (AUTO takes the grid kernel while profiling). In windows the slots hold, for block 0,
  * which serves the driven list: [0] the window's draws, [1] the wait at the deliveries' barrier,
  * [2] the driven neurons' free run, [3] the chain of their draws, [4] their spikes and state, [5]
  * the window's last barrier (and the one after the background hits); for the last block: [6] the
  * deliveries, [7] the wait at their barrier, [8] driven neurons, [9] unused, [10] the other
- * neurons' update, [11] the window's last barrier. */
+ * neurons' update, [11] the window's last barrier. In single steps: the first driven block's [0] lag
+ * wait and completion signal, [1] background and delivery, [2] draws, [3] update and spike list,
+ * [4] the next step's live entries; the first tile block's [5] wait at the step barrier for its
+ * service warps, [6] compaction, [7] own spikes' pushes, [8] the driven spikes' pushes, [9] delivery
+ * and update, [10] its publisher warp's work per step (completion signal, the next step's lag
+ * check), [11] its helper warp's work per step (the next step's driven spikes). */
 #define FB_NPHASES 12
 int fb_profile(fb_brains *br, int32_t on);
 int fb_phase_times(fb_brains *br, double *ms, int32_t n);

@@ -1,0 +1,103 @@
+"""One brain whose windows would be short or do not apply -- refractory times of a few steps and of
+none, more draws per step than a window's shared memory holds -- on the delay-scheduled kernel of single
+steps (fly-brain_gb300/csrc/fb_lagged.cu), alternating with the windowed one (fb_window.cu) and the grid
+kernel by the length of the launch. State, generator and ring equal the oracle's after each launch."""
+import numpy as np
+import pytest
+
+from test_window_gpu import GEN, make, pair, params, same
+
+pytestmark = pytest.mark.gpu
+
+BG = dict(bgRate=40.0, bgAmp=1.5)
+
+
+def brain(p, N=500, every=5, hz=600.0):
+    from flybrain import BrainBatch, DeviceGraph
+    g = make(N, 17, deg=20)
+    idx = np.arange(0, N, every, dtype=np.int32)
+    ob = pair(g, p, 3, idx, np.full(idx.shape[0], hz))
+    b = BrainBatch([DeviceGraph(g)], p, [3])
+    b.set_drive(0, idx, hz)
+    return ob, b
+
+
+@pytest.mark.parametrize("forced", [False, True])
+@pytest.mark.parametrize("over", [dict(), dict(BG, **GEN)])
+@pytest.mark.parametrize("tref,delay", [(0.0, 1.8), (0.05, 1.8), (0.15, 0.4), (0.25, 3.2), (0.35, 0.9)])
+def test_short_refractory_times(tref, delay, over, forced):
+    """8, 16, 64 and 128 steps are where the rule turns for windows of 1 to 4 steps."""
+    from flybrain import _native as nat
+    ob, b = brain(params(tRef=tref, delay=delay, vThresh=-50.0, **over))
+    if forced:
+        b.set_schedule(nat.FB_SCHEDULE_LAGGED)
+    for n in (30, 1, 5, 7, 8, 15, 1, 16, 63, 64, 2, 128, 1, 200):
+        ob.run(n)
+        b.step(n)
+        if forced or n >= 8:
+            assert b.last_schedule() == nat.FB_SCHEDULE_LAGGED
+        same(ob, b, 0, (tref, n))
+    assert int(ob.spikeCount.sum()) > 100
+
+
+def test_more_draws_than_a_window_holds():
+    """40,000 background events a step; from 2^16 draws on the forced schedule is refused."""
+    from flybrain import _native as nat
+    p = params(bgRate=40000 / (500 * 0.1e-3), bgAmp=0.001)
+    ob, b = brain(p)
+    b.set_schedule(nat.FB_SCHEDULE_LAGGED)
+    for n in (3, 20):
+        ob.run(n)
+        b.step(n)
+        assert b.last_schedule() == nat.FB_SCHEDULE_LAGGED
+        same(ob, b, 0, n)
+    b.set_background(0, 66000 / (500 * 0.1e-3), 0.001)
+    with pytest.raises(nat.FlyBrainError) as e:
+        b.step(8)
+    assert e.value.code == nat.FB_EINVAL
+    same(ob, b, 0, "refused")
+    b.set_schedule(nat.FB_SCHEDULE_AUTO)
+    ob.setBackground(66000 / (500 * 0.1e-3), 0.001)
+    ob.run(9)
+    b.step(9)
+    assert b.last_schedule() == nat.FB_SCHEDULE_GRID
+    same(ob, b, 0, "auto")
+
+
+@pytest.mark.parametrize("forced", [False, True])
+def test_neurons_that_fire_twice_in_a_step(forced):
+    """No refractory time and thresholds under the reset potential: the grid kernel."""
+    from flybrain import _native as nat
+    ob, b = brain(params(tRef=0.0))
+    for i in range(0, 500, 10):
+        ob.setThr(i, -9.0)
+    b.set_thr(0, np.arange(0, 500, 10, dtype=np.int32), -9.0)
+    if forced:
+        b.set_schedule(nat.FB_SCHEDULE_LAGGED)
+    for n in (20, 40):
+        ob.run(n)
+        b.step(n)
+        assert b.last_schedule() == nat.FB_SCHEDULE_GRID
+        same(ob, b, 0, n)
+    assert int(ob.spikeCount.max()) > 20
+
+
+@pytest.mark.parametrize("trip_at", [0, 41])
+def test_timeout_leaves_the_brain_as_it_was(trip_at):
+    from flybrain import _native as nat
+    ob, b = brain(params(tRef=0.15, depU=0.1, **BG))
+    for n in (5, 100):
+        ob.run(n)
+        b.step(n)
+    default = b.tuning()["timeout_us"]
+    b.set_tuning(timeout_us=2000)
+    b.trip_wait(trip_at)
+    with pytest.raises(nat.FlyBrainError) as e:
+        b.step(60)
+    assert e.value.code == nat.FB_ETIMEOUT
+    b.set_tuning(timeout_us=default)
+    same(ob, b, 0, "after the timeout")
+    for n in (1, 1, 4, 60, 1):
+        ob.run(n)
+        b.step(n)
+        same(ob, b, 0, n)
