@@ -512,13 +512,15 @@ struct fb_brains {
   int64_t timeoutNs = 5000000000LL;  // bound of every device-side wait (fb_tuning.timeout_us)
   int32_t tripStep = -1;             // test hook (fb_debug_trip_wait): armed for one launch
   int32_t lagDB = 0;                 // driven blocks of the lagged kernel (0: automatic)
-  int32_t irregular = 0;             // steps in which a neuron may fire sooner than its refractory time
+  // steps of each brain for which spikes closer than its refractory time may be in flight
+  std::vector<int32_t> irregular;
   int logging = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float lastMs = 0.f;
   int32_t schedule = FB_SCHEDULE_AUTO, lastSchedule = FB_SCHEDULE_GRID;
   LagRes lag;
   WinRes win;
+  char *d_before = nullptr;          // one brain: its state before a call of two launches
   std::vector<Topology *> topo;      // each brain's (the graphs outlive the batch)
   int maxSlots = 0;
   bool everRing = false;             // a kernel that keeps the ring's lists has run
@@ -585,6 +587,7 @@ extern "C" int fb_brains_create(const fb_graph *const *graphs, int32_t B, const 
   br->topo.assign(B, nullptr);
   br->dts.assign(B, 0.0);
   br->driven.resize(B);
+  br->irregular.assign(B, 0);
   int tileBase = 0;
   for (int b = 0; b < B; b++) {
     const fb_graph *g = graphs[b];
@@ -729,6 +732,7 @@ extern "C" int fb_brains_destroy(fb_brains *br) {
   for (void *p : br->lag.allocs) cudaFree(p);
   for (void *p : br->win.allocs) cudaFree(p);
   cudaFree(br->win.arena);
+  cudaFree(br->d_before);
   if (br->ev0) cudaEventDestroy(br->ev0);
   if (br->ev1) cudaEventDestroy(br->ev1);
   if (br->flushDone) cudaEventDestroy(br->flushDone);
@@ -972,6 +976,7 @@ extern "C" int fb_reset(fb_brains *br, int32_t b) {
   for (int32_t k = b < 0 ? 0 : b; k < (b < 0 ? br->B : b + 1); k++) {  // adapt 0 and res 1 again
     Trial &T = br->host[k];
     T.flags = (T.flags & ~(kAdaptZero | kResRest)) | rest_flags(T);
+    br->irregular[k] = 0;  // nothing is in flight
     CU(cudaMemcpyAsync(&br->trials[k].flags, &T.flags, 4, cudaMemcpyHostToDevice, br->stream));
   }
   if (br->win.ready && br->win.logValid)  // the spikes in flight are dropped from the log too
@@ -1022,7 +1027,7 @@ extern "C" int fb_set_params(fb_brains *br, int32_t b, const fb_params *p) {
   if (T.tRef != nt.tRef || T.dt != nt.dt) {
     // neurons may now fire sooner than the windows and the log assume: the windowed kernel's
     // resources are sized again at its next launch, from the ring
-    br->irregular = std::max(br->irregular, T.nslots - 1);
+    br->irregular[b] = T.nslots - 1;
     if (br->win.ready) {
       if ((rc = ring_from_log(br))) return rc;
       CU(cudaStreamSynchronize(br->stream));
@@ -1415,8 +1420,8 @@ static int win_setup(fb_brains *br) {
   return FB_OK;
 }
 
-// One windowed launch of steps[b] steps (windows of at most hCap steps).
-static int win_launch(fb_brains *br, const std::vector<int32_t> &steps, int hCap) {
+// One windowed launch of steps[b] steps.
+static int win_launch(fb_brains *br, const std::vector<int32_t> &steps) {
   WinRes &R = br->win;
   WinArgs a;
   memset(&a, 0, sizeof a);
@@ -1424,7 +1429,7 @@ static int win_launch(fb_brains *br, const std::vector<int32_t> &steps, int hCap
   bool changed = false;  // some brain's window
   for (int b = 0; b < br->B; b++) {
     const Trial &T = br->host[b];
-    const int32_t H = std::min(window_steps(T, (int64_t)br->driven[b].order.size()), hCap);
+    const int32_t H = window_steps(T, (int64_t)br->driven[b].order.size());
     changed = changed || H != R.host[b].H;
     R.host[b].H = H;
     a.nWin = std::max(a.nWin, (steps[b] + H - 1) / H);
@@ -1461,9 +1466,8 @@ static int win_launch(fb_brains *br, const std::vector<int32_t> &steps, int hCap
   return FB_OK;
 }
 
-// steps[b] steps of every brain through the windowed kernel: the log holds the spikes in flight,
-// the steps after an irregular host write run one at a time, logged launches are recorded a window
-// at a time.
+// The launch's steps of every brain through the windowed kernel: the log holds the spikes in flight,
+// logged launches are recorded a window at a time.
 static int run_window(fb_brains *br, int32_t maxSteps, bool forced) {
   WinRes &R = br->win;
   CU(cudaEventRecord(br->ev0, br->stream));
@@ -1481,25 +1485,18 @@ static int run_window(fb_brains *br, int32_t maxSteps, bool forced) {
     R.logValid = true;
   }
   std::vector<int32_t> left = br->stepsHost, part(br->B);
-  auto go = [&](int32_t most, int hCap) -> int {
-    for (int b = 0; b < br->B; b++) {
-      part[b] = std::min(left[b], most);
-      left[b] -= part[b];
-    }
-    return win_launch(br, part, hCap);
-  };
-  int32_t done = 0;
-  while (done < maxSteps) {
-    const bool slow = br->irregular > 0;
-    int32_t n = slow ? std::min(br->irregular, maxSteps - done) : maxSteps - done;
+  for (int32_t done = 0, n; done < maxSteps; done += n) {
+    n = maxSteps - done;
     if (br->logging) n = std::min(n, (int32_t)window_steps(br->host[0], (int64_t)br->driven[0].order.size()));
     if (done) CU(cudaStreamSynchronize(br->stream));  // the pinned step counts are free again
-    int rc = go(n, slow ? 1 : kWinMax);
+    for (int b = 0; b < br->B; b++) {
+      part[b] = std::min(left[b], n);
+      left[b] -= part[b];
+    }
+    int rc = win_launch(br, part);
     if (rc) return rc;
     br->tripStep = br->tripStep >= n ? br->tripStep - n : -1;
     if (br->logging) CU(launch_log_record(br->trials, R.win, n, br->stream));
-    if (slow) br->irregular -= n;
-    done += n;
   }
   br->tripStep = -1;  // one launch only
   CU(cudaEventRecord(br->ev1, br->stream));
@@ -1534,6 +1531,15 @@ static int win_recover(fb_brains *br, bool backup) {
   return FB_OK;
 }
 
+// Windows rest on the refractory time: a neuron has at most one spike in a window, and one to arrive in
+// it, and the log's size counts on no more in flight. After a host write of refr, or a new refractory
+// time or dt, that holds again once the delay has passed in that brain's own steps (irregular).
+static bool is_irregular(const fb_brains *br) {
+  for (int32_t k : br->irregular)
+    if (k > 0) return true;
+  return false;
+}
+
 // One brain's launches of n steps that the lagged kernel runs faster: it takes about the same time a
 // step whatever the window's length H, a window costs its round trips however short it is.
 // Microseconds per launch, windowed / lagged, current-based at dt 0.1 ms, 20,000 neurons: H 1, 8 steps
@@ -1547,6 +1553,7 @@ static bool lag_better(const fb_brains *br, int32_t n) {
   const Trial &T = br->host[0];
   const int tb = br->sms - kLagMaxDB;
   if (br->B != 1 || (T.N + tb - 1) / tb > kLagPer * kLagTileWorkers) return false;
+  if (is_irregular(br)) return n >= kLagMinSteps;
   switch (window_steps(T, (int64_t)br->driven[0].order.size())) {
     case 1: return n >= kLagMinSteps;
     case 2: return n >= 16;
@@ -1565,17 +1572,19 @@ static bool fires_once_a_step(const Trial &T) {
 
 enum class StepKernel { kGrid, kLagged, kWindow };
 
-// The kernel of this launch, its resources ready.
-static int choose_kernel(fb_brains *br, int32_t n, StepKernel *k) {
+// The kernel of this launch, its resources ready. head: the steps before a call's windows, for which
+// the lagged kernel's buffers (16 bytes per edge and step of the delay) are not allocated.
+static int choose_kernel(fb_brains *br, int32_t n, bool head, StepKernel *k) {
   *k = StepKernel::kGrid;
   if (n == 0 || br->schedule == FB_SCHEDULE_GRID) return FB_OK;
   const bool forced = br->schedule == FB_SCHEDULE_LAGGED;
   const char *why = nullptr;
   const bool applies = lag_applies(br, n, &why);
   if (forced && !applies) return fail(FB_EINVAL, "fb_step: the delay-scheduled schedule does not apply to %s", why);
-  const bool window = win_capable(br) && !br->win.noMemory &&
+  const bool window = win_capable(br) && !br->win.noMemory && !is_irregular(br) &&
                       (forced || (n >= win_min_steps(br) && !br->profiling && (!br->logging || (br->B == 1 && n <= kWinLogSteps))));
-  const bool lagged = applies && fires_once_a_step(br->host[0]) && (forced || (n >= kLagMinSteps && !br->lag.noMemory));
+  const bool lagged = applies && fires_once_a_step(br->host[0]) &&
+                      (forced || (n >= kLagMinSteps && !br->lag.noMemory && (!head || br->lag.ready)));
   int rc = FB_OK;
   // the better one first, the other where its memory cannot be had
   for (int k2 = 0; k2 < 2; k2++) {
@@ -1592,11 +1601,11 @@ static int choose_kernel(fb_brains *br, int32_t n, StepKernel *k) {
   return FB_OK;
 }
 
-static int run_steps(fb_brains *br, int32_t maxSteps, int32_t *out_nfired) {
-  int rc = flush(br, false);
-  if (rc) return rc;
+// One launch of br->stepsHost steps on the kernel that suits it.
+static int run_launch(fb_brains *br, int32_t maxSteps, bool head, int32_t *out_nfired) {
+  int rc;
   StepKernel kernel;
-  if ((rc = choose_kernel(br, maxSteps, &kernel))) return rc;
+  if ((rc = choose_kernel(br, maxSteps, head, &kernel))) return rc;
   // the error flag and the fired counts come back in one synchronisation
   auto read_back = [&]() -> int {
     CU(cudaMemcpyAsync(br->h_small, br->d_err, 4, cudaMemcpyDeviceToHost, br->stream));
@@ -1609,7 +1618,6 @@ static int run_steps(fb_brains *br, int32_t maxSteps, int32_t *out_nfired) {
   };
   if (kernel == StepKernel::kLagged) {
     if ((rc = run_lagged(br, maxSteps))) return rc;
-    br->irregular = std::max(0, br->irregular - maxSteps);
     if ((rc = read_back())) return rc;
     const int32_t err = br->h_small[0];
     cudaEventElapsedTime(&br->lastMs, br->ev0, br->ev1);
@@ -1638,7 +1646,6 @@ static int run_steps(fb_brains *br, int32_t maxSteps, int32_t *out_nfired) {
     br->win.slotsValid = true;
     br->win.logValid = false;
     br->everRing = true;
-    br->irregular = std::max(0, br->irregular - maxSteps);
     if (br->stepsUploaded != br->stepsHost) {  // the last launch's counts stay on the device otherwise
       std::memcpy(br->h_steps, br->stepsHost.data(), sizeof(int32_t) * br->B);
       CU(cudaMemcpyAsync(br->d_steps, br->h_steps, sizeof(int32_t) * br->B, cudaMemcpyHostToDevice, br->stream));
@@ -1688,6 +1695,7 @@ static int run_steps(fb_brains *br, int32_t maxSteps, int32_t *out_nfired) {
                   br->ovfCap);
     }
   }
+  for (int b = 0; b < br->B; b++) br->irregular[b] = std::max(0, br->irregular[b] - br->stepsHost[b]);
   if (out_nfired) {
     if (maxSteps > 0) {
       std::memcpy(out_nfired, br->h_small + 2, sizeof(int32_t) * br->B);
@@ -1697,6 +1705,70 @@ static int run_steps(fb_brains *br, int32_t maxSteps, int32_t *out_nfired) {
     }
   }
   return FB_OK;
+}
+
+// The steps of a call that run apart, before its windows: those for which brains are irregular, where
+// windows repay a second launch. Microseconds for refr written and n steps, whole / apart, 18 of them
+// irregular: one brain of 20,000 neurons, 49 steps 237 / 252 for 50, of 165,122 neurons 344 / 367 (the
+// whole on the lagged kernel); a batch of four, 20,000 each, 49 steps 642 / 384 (on the grid kernel).
+constexpr int kSplitRest = 32, kSplitRestBatch = 8;
+static int32_t split_steps(fb_brains *br, int32_t maxSteps) {
+  int32_t head = 0;
+  for (int b = 0; b < br->B; b++) {
+    if (br->irregular[b] > br->stepsHost[b]) return 0;
+    head = std::max(head, br->irregular[b]);
+  }
+  if (head == 0 || maxSteps - head < (br->B == 1 ? kSplitRest : kSplitRestBatch) || br->schedule == FB_SCHEDULE_GRID || br->logging || br->profiling) return 0;
+  if (!win_capable(br) || br->win.noMemory) return 0;
+  std::vector<int32_t> now(br->B, 0);
+  now.swap(br->irregular);
+  const bool lagged = lag_better(br, maxSteps - head);
+  now.swap(br->irregular);
+  return lagged ? 0 : head;
+}
+
+static int run_steps(fb_brains *br, int32_t maxSteps, int32_t *out_nfired) {
+  int rc = flush(br, false);
+  if (rc) return rc;
+  const int32_t head = split_steps(br, maxSteps);
+  if (head == 0) return run_launch(br, maxSteps, false, out_nfired);
+  // one brain: as it was before the call if a launch fails
+  const std::vector<int32_t> all = br->stepsHost, irregular = br->irregular;
+  const Trial &T = br->host[0];
+  const size_t st = 11 * align256((size_t)T.N * 4), ring = (char *)(T.ringCount + T.nslots) - (char *)T.ring;
+  if (br->B == 1) {
+    if (!br->d_before && cudaMalloc(&br->d_before, st + sizeof(Trial) + ring) != cudaSuccess) {
+      cudaGetLastError();
+      return run_launch(br, maxSteps, false, out_nfired);
+    }
+    if ((rc = ring_from_log(br))) return rc;
+    CU(cudaMemcpyAsync(br->d_before, T.v, st, cudaMemcpyDeviceToDevice, br->stream));
+    CU(cudaMemcpyAsync(br->d_before + st, br->trials, sizeof(Trial), cudaMemcpyDeviceToDevice, br->stream));
+    CU(cudaMemcpyAsync(br->d_before + st + sizeof(Trial), T.ring, ring, cudaMemcpyDeviceToDevice, br->stream));
+  }
+  const int32_t trip = br->tripStep;
+  if (trip >= head) br->tripStep = -1;
+  for (int b = 0; b < br->B; b++) br->stepsHost[b] = std::min(all[b], head);
+  rc = run_launch(br, head, true, nullptr);
+  const float ms = br->lastMs;
+  if (rc == FB_OK) {
+    if (trip >= head) br->tripStep = trip - head;
+    for (int b = 0; b < br->B; b++) br->stepsHost[b] = all[b] - std::min(all[b], head);
+    rc = run_launch(br, maxSteps - head, false, out_nfired);
+    br->lastMs += ms;
+  }
+  if (rc && br->B == 1) {
+    const std::string why = g_err;
+    CU(cudaMemcpyAsync(T.v, br->d_before, st, cudaMemcpyDeviceToDevice, br->stream));
+    CU(cudaMemcpyAsync(br->trials, br->d_before + st, sizeof(Trial), cudaMemcpyDeviceToDevice, br->stream));
+    CU(cudaMemcpyAsync(T.ring, br->d_before + st + sizeof(Trial), ring, cudaMemcpyDeviceToDevice, br->stream));
+    CU(cudaStreamSynchronize(br->stream));
+    br->win.ringValid = true;
+    br->win.logValid = br->win.slotsValid = false;
+    br->irregular = irregular;
+    g_err = why;
+  }
+  return rc;
 }
 
 extern "C" int fb_step(fb_brains *br, int32_t nsteps, int32_t *out_nfired) {
@@ -1848,7 +1920,7 @@ extern "C" int fb_write(fb_brains *br, int32_t field, int32_t b, const void *src
   if (field == FB_FIELD_DRIVE) return fail(FB_EINVAL, "fb_write: the drive field is written through fb_set_drive, which keeps the driven set");
   rc = flush(br);
   if (rc) return rc;
-  if (field == FB_FIELD_REFR) br->irregular = std::max(br->irregular, br->host[b].nslots - 1);
+  if (field == FB_FIELD_REFR) br->irregular[b] = br->host[b].nslots - 1;
   const int32_t clear = field == FB_FIELD_ADAPT ? kAdaptZero : field == FB_FIELD_RES ? kResRest
                         : field == FB_FIELD_BIAS ? kBiasZero : field == FB_FIELD_THR ? kThrZero : 0;
   if (br->host[b].flags & clear) {  // the field may no longer be at rest: the update reads it again

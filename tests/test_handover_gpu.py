@@ -76,3 +76,90 @@ def test_single_steps_after_a_windowed_launch(what, before):
     assert sum(int(ob.ringCount.sum()) for ob in obs) > 30
     steps(obs, batch, 25, what)
     assert batch.last_schedule() == nat.FB_SCHEDULE_GRID
+
+
+@pytest.mark.parametrize("rest", [[[(0, 40), (5, 0), (45, 5)]], [[(3, 25), (60, 70)], [(2, 100), (7, 0), (40, 60), (50, 1)]]])
+def test_refractory_write_of_a_brain_that_waits(rest):
+    """What a write of refr allows (two spikes of a neuron in flight closer than its refractory time)
+    holds for as many steps of that brain, however far the others are taken meanwhile."""
+    p = params(**DEP)
+    obs, batch = brains(2, p, hz=5000.0)
+
+    def go(n):
+        for ob, k in zip(obs, n):
+            ob.run(k)
+        batch.step_uneven(np.array(n, np.int32))
+        for b, ob in enumerate(obs):
+            same(ob, batch, b, (n, b))
+
+    go((30, 30))
+    for n in rest:
+        obs[0].refr[:] = 0.0
+        batch.write("refr", 0, np.zeros(obs[0].N, np.float32))
+        for m in n:
+            go(m)
+
+
+def test_refractory_write_before_a_launch_that_times_out():
+    """The launch leaves the brain as it was, what the write allows included."""
+    from flybrain import _native as nat
+    obs, batch = brains(1, params(**DEP), hz=5000.0)
+    ob = obs[0]
+    ob.run(30)
+    batch.step(30)
+    ob.refr[:] = 0.0
+    batch.write("refr", 0, np.zeros(ob.N, np.float32))
+    default = batch.tuning()["timeout_us"]
+    for trip, n in ((2, 100), (25, 100), (90, 100), (3, 12)):
+        batch.set_tuning(timeout_us=2000)
+        batch.trip_wait(trip)
+        with pytest.raises(nat.FlyBrainError) as e:
+            batch.step(n)
+        assert e.value.code == nat.FB_ETIMEOUT
+        batch.set_tuning(timeout_us=default)
+        same(ob, batch, 0, ("timeout", trip))
+    for n in (5, 100, 1, 30):
+        ob.run(n)
+        batch.step(n)
+        same(ob, batch, 0, n)
+
+
+@pytest.mark.parametrize("B", [1, 2])
+@pytest.mark.parametrize("n", [2, 12])
+def test_refractory_written_before_every_launch(n, B):
+    """Every neuron fires in every launch: far more spikes in flight than the refractory time allows."""
+    from flybrain import _native as nat
+    obs, batch = brains(B, params(), hz=1e5, every=1)
+    for k in range(12):
+        for b, ob in enumerate(obs):
+            ob.refr[:] = 0.0
+            batch.write("refr", b, np.zeros(ob.N, np.float32))
+            ob.run(n)
+        batch.step(n)
+        for b, ob in enumerate(obs):
+            same(ob, batch, b, (n, k, b))
+    if n == 2:
+        assert int(obs[0].ringCount.sum()) > 8 * obs[0].N
+    for ob in obs:
+        ob.run(70)
+    batch.step(70)
+    assert batch.last_schedule() == nat.FB_SCHEDULE_LAGGED
+    for b, ob in enumerate(obs):
+        same(ob, batch, b, ("after", b))
+
+
+@pytest.mark.parametrize("trefs", [(0.15, 2.2, 0.6), (2.2, 0.0, 1.0)])
+def test_refractory_time_changed(trefs):
+    """The spikes in flight are those of the refractory time before."""
+    p = params(depU=0.1)
+    obs, batch = brains(2, dict(p, tRef=trefs[0]), hz=1e5, every=1)
+    for k, tref in enumerate(trefs):
+        if k:
+            for b, ob in enumerate(obs):
+                set_tref(ob, batch, b, p, tref)
+        for n in (6, 30, 64):
+            for ob in obs:
+                ob.run(n)
+            batch.step(n)
+            for b, ob in enumerate(obs):
+                same(ob, batch, b, (trefs, tref, n, b))
