@@ -1570,6 +1570,20 @@ static bool fires_once_a_step(const Trial &T) {
   return silent_steps(T) >= 1 || (T.vReset < T.vThresh && (T.flags & kThrZero) && T.adaptInc >= 0);
 }
 
+// Whether windows pay for this launch of a batch: a window costs as much as one and a half steps of the
+// grid kernel, so not where most hold a single step. Microseconds for 200 steps of eight brains of
+// 20,000 neurons, windowed / grid: windows of one step 4,344 / 2,920, of two 2,253 / 2,929; of 165,122
+// neurons 9,385 / 6,542 and 4,989 / 6,497; for four steps of 1,501 neurons 116 / 102 and 80 / 100.
+static bool windows_pay(const fb_brains *br, int32_t n) {
+  if (br->B == 1) return true;  // the lagged kernel has the short ones
+  int64_t windows = 0;
+  for (int b = 0; b < br->B; b++) {
+    const int H = window_steps(br->host[b], (int64_t)br->driven[b].order.size());
+    windows = std::max<int64_t>(windows, (br->stepsHost[b] + H - 1) / H);
+  }
+  return 3 * windows <= 2 * (int64_t)n;
+}
+
 enum class StepKernel { kGrid, kLagged, kWindow };
 
 // The kernel of this launch, its resources ready. head: the steps before a call's windows, for which
@@ -1582,7 +1596,8 @@ static int choose_kernel(fb_brains *br, int32_t n, bool head, StepKernel *k) {
   const bool applies = lag_applies(br, n, &why);
   if (forced && !applies) return fail(FB_EINVAL, "fb_step: the delay-scheduled schedule does not apply to %s", why);
   const bool window = win_capable(br) && !br->win.noMemory && !is_irregular(br) &&
-                      (forced || (n >= win_min_steps(br) && !br->profiling && (!br->logging || (br->B == 1 && n <= kWinLogSteps))));
+                      (forced || (n >= win_min_steps(br) && !br->profiling && (!br->logging || (br->B == 1 && n <= kWinLogSteps)) &&
+                                  windows_pay(br, n)));
   const bool lagged = applies && fires_once_a_step(br->host[0]) &&
                       (forced || (n >= kLagMinSteps && !br->lag.noMemory && (!head || br->lag.ready)));
   int rc = FB_OK;

@@ -141,13 +141,13 @@ int fb_brains_set_mode(fb_brains *br, int32_t mode);
  * presynaptic inhibition (4 <= nslots - 1 <= 32 steps, at most 4,096 driven neurons per brain;
  * per-step logging only for one brain in launches of at most 64 steps). One advances the brains in
  * windows of the delay, at most the steps that a neuron stays refractory; the other, for one brain
- * and launches of at least 8 steps, takes one step at a time in blocks that synchronise only at the
- * delay, where windows would be short or do not apply (a refractory time under one step, more draws
- * than a block's shared memory holds). AUTO (default) takes one of them where they apply and the
- * launch has at least 2 steps (3 with background events), GRID otherwise. LAGGED forces them for
- * one brain; where neither applies fb_step then fails with FB_EINVAL. (With a refractory time under
- * one step and threshold offsets, or vReset >= vThresh, a neuron may fire twice in a step: GRID, under
- * LAGGED too.) */
+ * and launches of at least 8 steps, takes one step at a time in blocks that synchronise only at
+ * the delay, where windows would be short or do not apply (a refractory time under one step, more
+ * draws than a block's shared memory holds). AUTO (default) takes one of them where they apply and
+ * the launch has at least 2 steps (3 with background events) and, in a batch, windows of more than
+ * one, GRID otherwise. LAGGED forces them for one brain; where neither applies fb_step then fails
+ * with FB_EINVAL. (With a refractory time under one step and threshold offsets, or vReset >=
+ * vThresh, a neuron may fire twice in a step: GRID, under LAGGED too.) */
 #define FB_SCHEDULE_AUTO 0
 #define FB_SCHEDULE_GRID 1
 #define FB_SCHEDULE_LAGGED 2

@@ -101,3 +101,26 @@ def test_timeout_leaves_the_brain_as_it_was(trip_at):
         ob.run(n)
         b.step(n)
         same(ob, b, 0, n)
+
+
+@pytest.mark.parametrize("trefs,n,windows", [((0.05, 0.05, 0.05), 40, False), ((0.15, 0.15, 0.15), 40, True),
+                                             ((0.05, 2.2, 2.2), 40, False), ((0.15, 2.2, 2.2), 3, True),
+                                             ((2.2, 0.15, 0.05), 2, False), ((2.2, 2.2, 2.2), 2, True)])
+def test_batches_of_short_windows(trefs, n, windows):
+    """Windows of one step in a batch cost more than the grid kernel's steps."""
+    from flybrain import BrainBatch, DeviceGraph
+    from flybrain import _native as nat
+    gs = [make(300 + 50 * b, 60 + b, deg=15) for b in range(3)]
+    ps = [params(tRef=t, depU=0.1) for t in trefs]
+    idx = np.arange(0, 300, 4, dtype=np.int32)
+    obs = [pair(g, p, b + 1, idx, np.full(75, 700.0)) for b, (g, p) in enumerate(zip(gs, ps))]
+    batch = BrainBatch([DeviceGraph(g) for g in gs], ps, [1, 2, 3])
+    for b in range(3):
+        batch.set_drive(b, idx, 700.0)
+    for k in range(3):
+        for ob in obs:
+            ob.run(n)
+        batch.step(n)
+        assert batch.last_schedule() == (nat.FB_SCHEDULE_LAGGED if windows else nat.FB_SCHEDULE_GRID)
+        for b, ob in enumerate(obs):
+            same(ob, batch, b, (trefs, k, b))
