@@ -529,11 +529,12 @@ __device__ __forceinline__ void tile_run(const WarpBrain &T, const Tile &t, bool
     }
   } else {
     int j = 0;
-    if (kWT > 512 && !__any_sync(0xffffffffu, K.vReset >= thB)) {
+    if (kWT > 512 && !__any_sync(0xffffffffu, K.vReset >= thB || x.r != x.r)) {
       // The refractory count as the step it ends before: a neuron that fires stays refractory to the
-      // window's end, and while it is it cannot cross a threshold above vReset. Four instructions
-      // fewer per step, which U of a batch is bound by (96 brains 641 -> 617 us a window); one
-      // brain's is not (its warps have two tiles at most).
+      // window's end, and while it is it cannot cross a threshold above vReset. (A count that is not a
+      // number lets the neuron integrate but never fire: the other path.) Four instructions fewer per
+      // step, which U of a batch is bound by (96 brains 641 -> 617 us a window); one brain's is not
+      // (its warps have two tiles at most).
       int silent = 0;
       float r = x.r;
       for (int q = 0; q < h && __any_sync(0xffffffffu, r > 0); q++)

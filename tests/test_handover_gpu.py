@@ -163,3 +163,24 @@ def test_refractory_time_changed(trefs):
             batch.step(n)
             for b, ob in enumerate(obs):
                 same(ob, batch, b, (trefs, tref, n, b))
+
+
+def test_refractory_count_that_is_not_a_number():
+    """It is neither over zero nor at most zero (lif.c:61-76): the neuron integrates and never fires."""
+    for B in (1, 3):
+        obs, batch = brains(B, params(), hz=300.0)
+        ix = np.arange(1, 400, 3)
+        for b, ob in enumerate(obs):
+            ob.setBias(np.arange(ob.N), 9.0)
+            batch.set_bias(b, np.arange(ob.N, dtype=np.int32), 9.0)
+            r = np.zeros(ob.N, np.float32)
+            r[ix] = np.nan
+            ob.refr[:] = r
+            batch.write("refr", b, r)
+        for n in (30, 100, 40):
+            for ob in obs:
+                ob.run(n)
+            batch.step(n)
+            for b, ob in enumerate(obs):
+                same(ob, batch, b, (B, n, b))
+        assert int(obs[0].spikeCount.sum()) > 200
