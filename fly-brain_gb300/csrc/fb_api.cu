@@ -565,9 +565,6 @@ static uint32_t seed_state(uint32_t seed) {
   return s ? s : 1u;
 }
 
-static bool win_capable(const fb_brains *br);
-static int win_create(fb_brains *br, bool early);
-
 extern "C" int fb_brains_create(const fb_graph *const *graphs, int32_t B, const fb_params *params,
                                 int32_t params_stride, const uint32_t *seeds, fb_brains **out) {
   if (!out) return fail(FB_EINVAL, "fb_brains_create: out is null");
@@ -711,7 +708,6 @@ extern "C" int fb_brains_create(const fb_graph *const *graphs, int32_t B, const 
     return brains_fail_cleanup(br, fail(FB_ENOMEM, "fb_brains_create: pinned host staging"));
   if (cudaStreamSynchronize(br->stream) != cudaSuccess)
     return brains_fail_cleanup(br, fail(FB_ECUDA, "fb_brains_create: %s", cudaGetErrorString(cudaGetLastError())));
-  if (win_capable(br) && win_create(br, true) != FB_OK) g_err.clear();  // short of memory: the grid kernel only
   *out = br;
   return FB_OK;
 }
@@ -1312,9 +1308,9 @@ static int win_alloc(fb_brains *br, X **p, size_t n) {
 }
 
 static size_t bg_hit_bytes(const Trial &T) { return align256((size_t)T.N * std::min(T.nslots - 1, kWinMax) * 4); }
-// The kernel's resources: one allocation for the batch. At the batch's creation (early) they wait
-// for the first launch if they would take much of the free memory.
-static int win_create(fb_brains *br, bool early) {
+// The kernel's resources: one allocation for the batch, at its first windowed launch (batches that only
+// take single steps or the grid schedule do without).
+static int win_create(fb_brains *br) {
   WinRes &R = br->win;
   const int B = br->B;
   cudaFree(R.arena);
@@ -1338,11 +1334,6 @@ static int win_create(fb_brains *br, bool early) {
     while (cap[b] < (uint64_t)T.N * ((D + H - 1) / H + 2)) cap[b] *= 2;
     zero += 2 * n4(b) + align256(T.N) + ((T.flags & kHasBg) ? bg_hit_bytes(T) : 0);
     rest += n4(b) + align256(cap[b] * 16) + align256((size_t)T.E * 8) + align256((size_t)kWinDriven * (4 + kWinSaved * 4 + 1));
-  }
-  if (early && zero + rest > ((size_t)8 << 30)) {
-    size_t avail = 0, total = 0;
-    CU(cudaMemGetInfo(&avail, &total));
-    if (zero + rest > avail / 4) return FB_OK;
   }
   if (cudaMalloc(&R.arena, zero + rest) != cudaSuccess) {
     cudaGetLastError();
@@ -1395,7 +1386,7 @@ static int win_create(fb_brains *br, bool early) {
 static int win_setup(fb_brains *br) {
   WinRes &R = br->win;
   int rc;
-  if (!R.ready && (rc = win_create(br, false))) return rc;
+  if (!R.ready && (rc = win_create(br))) return rc;
   bool moved = false;
   size_t need = 0;  // brains that draw background events since they were created (then in the arena)
   for (int b = 0; b < br->B; b++)

@@ -184,3 +184,22 @@ def test_refractory_count_that_is_not_a_number():
             for b, ob in enumerate(obs):
                 same(ob, batch, b, (B, n, b))
         assert int(obs[0].spikeCount.sum()) > 200
+
+
+def test_single_steps_take_no_window_buffers():
+    """The windowed kernel's buffers (8 bytes per edge and more) come with the first windowed launch."""
+    import torch
+    from flybrain import BrainBatch, DeviceGraph
+    from flybrain import _native as nat
+    g = make(1500, 3, deg=4000)
+    batch = BrainBatch([DeviceGraph(g)] * 2, params(), [1, 2])
+    for b in range(2):
+        batch.set_drive(b, np.arange(50, dtype=np.int32), 200.0)
+    batch.step(1)
+    batch.set_schedule(nat.FB_SCHEDULE_GRID)
+    batch.step(20)
+    before = torch.cuda.mem_get_info()[0]
+    batch.set_schedule(nat.FB_SCHEDULE_AUTO)
+    batch.step(20)
+    assert batch.last_schedule() == nat.FB_SCHEDULE_LAGGED
+    assert before - torch.cuda.mem_get_info()[0] >= 2 * 8 * g.E
