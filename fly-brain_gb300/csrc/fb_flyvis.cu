@@ -135,14 +135,15 @@ __device__ __forceinline__ void fv_update(int32_t i, int32_t b0, int32_t B, int3
 
 // One step, bound by the L1's wavefronts and the latency of its misses. A lane takes V instances of a
 // target: wider gathers mean fewer of them (64 eyes of the full network: 38 us a step; a thread per
-// instance, its load and issue slots full, took 74; 16 eyes 18.5 and 24.6). The instances
-// are cut into `chunks` of `width` vectors, and each block takes a run of neighbouring targets in
-// one chunk, so that the sources that a block's targets share stay in its L1.
+// instance, its load and issue slots full, took 74; 16 eyes 18.5 and 24.6), where there are enough
+// of them to fill the lanes (fv_width). The instances are cut into `chunks` of `width` vectors, and
+// each block takes a run of neighbouring targets in one chunk, so that the sources that a block's
+// targets share stay in its L1. Rows of `gin` hold `pitch` words, rows of `rout` `rpitch`.
 template <int V, int MODE>
 __global__ void __launch_bounds__(kFvStepThreads, 1)
-    fv_step_kernel(int32_t N, int32_t B, int32_t pitch, int32_t width, int32_t chunks, const uint32_t *__restrict__ ptr,
-                   const int4 *__restrict__ rec, const float *__restrict__ bias, const float *__restrict__ kdt,
-                   const float *__restrict__ gin, float *__restrict__ rout, const float *vin, float *vout,
+    fv_step_kernel(int32_t N, int32_t B, int32_t pitch, int32_t rpitch, int32_t width, int32_t chunks,
+                   const uint32_t *__restrict__ ptr, const int4 *__restrict__ rec, const float *__restrict__ bias,
+                   const float *__restrict__ kdt, const float *__restrict__ gin, float *__restrict__ rout, const float *vin, float *vout,
                    const float *__restrict__ x, float nz) {
   const int64_t row = (int64_t)N * width, per = (row * chunks + gridDim.x - 1) / gridDim.x;
   const int64_t t0 = per * blockIdx.x, t1 = min(t0 + per, row * chunks);
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(kFvStepThreads, 1)
         fv_add<V, MODE>(acc, __int_as_float(q[u].w), r[2 * u + 1], nz);
       }
     }
-    fv_update<V>(i, b0, B, pitch, acc, bias, kdt, rout, vin, vout, x);
+    fv_update<V>(i, b0, B, rpitch, acc, bias, kdt, rout, vin, vout, x);
   }
 }
 
@@ -497,6 +498,16 @@ extern "C" int fb_flyvis_read(fb_flyvis *f, int32_t field, int32_t b, float *out
   return FB_OK;
 }
 
+// Instances per lane, at most `most`: one while all (target, instance) pairs take a third of the chip's
+// 311,296 resident threads, two until they take all of them, then four. Microseconds for 20 steps at
+// 1 / 2 / 4: 3,000 neurons and 4 eyes 135 / 175 / 216, 6,000 and 16 (96,000 pairs) 175 / 175 / 176,
+// 45,669 and 3 (137,000) 296 / 257 / 296, 24,000 and 8 (192,000) 218 / 216 / 230, 45,669 and 5 (228,000)
+// 339 / 337 / 337, 12,000 and 33 (396,000) 339 / 334 / 299, 45,669 and 64 1,472 / 963 / 787.
+static int32_t fv_width(const fb_flyvis *f, int32_t most) {
+  const int64_t pairs = (int64_t)f->N * f->B;
+  return pairs <= 100000 ? 1 : std::min(most, pairs <= 300000 ? 2 : 4);
+}
+
 // One step from `gin` (rows of `pitch` words). The chunks are at most kFvWidth vectors. Blocks of
 // 1,024 threads, one per SM, leave one block to balance a run of targets in; with fewer lanes than
 // that, blocks of 256 spread them over the SMs (8 eyes of the full network 14.5 us a step against
@@ -510,7 +521,7 @@ static void fv_launch(fb_flyvis *f, int V, int mode, int32_t pitch, const float 
   (mode == kFvFinite ? fv_step_kernel<V_, kFvFinite> : mode == kFvR ? fv_step_kernel<V_, kFvR> : fv_step_kernel<V_, kFvV>)
   auto kernel = V == 4 ? FV_PICK(4) : V == 2 ? FV_PICK(2) : FV_PICK(1);
 #undef FV_PICK
-  kernel<<<grid, threads, 0, f->st>>>(f->N, f->B, pitch, width, chunks, f->ptr, f->rec, f->bias, f->kdt, gin, rout,
+  kernel<<<grid, threads, 0, f->st>>>(f->N, f->B, pitch, f->pitch, width, chunks, f->ptr, f->rec, f->bias, f->kdt, gin, rout,
                                       f->v[f->cur], vout, f->x, -0.f);
 }
 
@@ -519,11 +530,15 @@ extern "C" int fb_flyvis_step(fb_flyvis *f, int32_t nsteps) {
   if (rc) return rc;
   if (nsteps < 0) return fvfail(FB_EINVAL, "fb_flyvis_step: nsteps=%d", nsteps);
   FVCU(cudaEventRecord(f->ev0, f->st));
-  // a row of v holds whole vectors of this many instances
-  const int32_t vecV = f->r[0] ? f->vec : f->B % 4 == 0 ? 4 : f->B % 2 == 0 ? 2 : 1;
+  // instances per lane from r, and from v, whose rows hold whole vectors of this many
+  const int32_t vecR = fv_width(f, f->vec), vecV = fv_width(f, f->B % 4 == 0 ? 4 : f->B % 2 == 0 ? 2 : 1);
+  // a first step that would gather narrower than r allows: a pass that makes r costs 5 us and repays
+  // itself from about a million pairs on (13 eyes of the full network 32 us with narrow gathers, 40
+  // with the pass, 33 eyes 58 and 53)
+  const bool pass = f->r[0] && vecV < vecR && (int64_t)f->N * f->B >= 1000000;
   for (int32_t s = 0, in = 0; s < nsteps; s++) {
     const bool more = f->r[0] && s + 1 < nsteps;
-    if (!f->r[0] || (s == 0 && f->B % f->vec == 0)) {
+    if (!f->r[0] || (s == 0 && !pass)) {
       fv_launch(f, vecV, kFvV, f->B, f->v[f->cur], more ? f->r[0] : nullptr, f->v[f->cur ^ 1]);
       f->cur ^= 1;
     } else {
@@ -532,7 +547,7 @@ extern "C" int fb_flyvis_step(fb_flyvis *f, int32_t nsteps) {
         const int g = (int)std::min<int64_t>((words + kFvThreads - 1) / kFvThreads, (int64_t)f->sms * 8);
         fv_rectify_kernel<<<g, kFvThreads, 0, f->st>>>(f->N, f->B, f->pitch, f->v[f->cur], f->r[0]);
       }
-      fv_launch(f, f->vec, f->finite ? kFvFinite : kFvR, f->pitch, f->r[in], more ? f->r[in ^ 1] : nullptr, f->v[f->cur]);
+      fv_launch(f, vecR, f->finite ? kFvFinite : kFvR, f->pitch, f->r[in], more ? f->r[in ^ 1] : nullptr, f->v[f->cur]);
       in ^= 1;
     }
   }

@@ -133,3 +133,24 @@ def test_input_lists(n):
             fv.set_input(idx, val, 1)
         np.testing.assert_array_equal(fv.read("x", 1), ref)
     assert not fv.read("x", 0).any() and not fv.read("x", 2).any()
+
+
+@pytest.mark.parametrize("N,B", [(33333, 3), (33334, 3), (25000, 4), (25001, 4), (60000, 5), (60001, 5), (42857, 7),
+                                 (42858, 7), (50001, 6),
+                                 (45669, 21), (45669, 22), (10001, 101)])
+def test_instances_per_lane(N, B):
+    """Both sides of where a lane takes two and four instances, calls of one and of several steps."""
+    from oracle import oracle as O
+    from flybrain.flyvis import FlyVis, synth_flyvis
+    m = synth_flyvis(N=N, seed=5, mean_in=6.0)
+    rng = np.random.default_rng(N)
+    x = rng.normal(0.0, 0.6, (B, N)).astype(np.float32)
+    fv = FlyVis(m, B=B)
+    v = np.tile(m["bias"], (B, 1)).astype(np.float32)
+    for b in range(B):
+        fv.write("x", b, x[b])
+    for steps in (1, 3):
+        fv.step(steps)
+        O.fv_run(m, v, x, steps)
+        for b in range(B):
+            np.testing.assert_array_equal(fv.v(b), v[b])
