@@ -1959,10 +1959,8 @@ size_t chain_smem(const fb_diff_batch *b) {  // lane tables, 2 words per driven 
   return (kWinJumpWords + 2 * std::min<size_t>(n, kChainDriven) + std::min<size_t>(kWinStream, n * kWindowMax) + 64) * 4;
 }
 int chain_setup(fb_diff_batch *b) {
-  const int bytes = (int)chain_smem(b);
   DCU(cudaFuncSetAttribute(k_wchain<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((kWinJumpWords + 2 * kChainDriven + kWinStream + 64) * 4)));
   DCU(cudaFuncSetAttribute(k_wchain<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((kWinJumpWords + 2 * kChainDriven + kWinStream + 64) * 4)));
-  (void)bytes;
   if (!b->winJump) {
     std::vector<uint32_t> tab(kWinJumpWords);
     window_jump_tables(kChainThreads, tab.data());

@@ -164,7 +164,6 @@ __global__ void __launch_bounds__(kDB, 4) k_wdeliver(const DiffDev *Ds, DP<R> P,
   load_dev(Ds, D);
   const WSpan S = w_span(D, t0, t1, off);
   if (S.h <= 0) return;
-  const bool ex = row < 0 && D.exact32;
   const int lane = threadIdx.x & 31, d = D.nslots - 1;
   const int64_t th = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (int64_t)gridDim.x * blockDim.x;
   if (row < 0 && th < kWindowMax) D.wSpikes[th] = 0;  // a forward's spike counts of the window
@@ -180,24 +179,14 @@ __global__ void __launch_bounds__(kDB, 4) k_wdeliver(const DiffDev *Ds, DP<R> P,
     const int ek = w_step_of(S, off, a), j = S.e0 + ek + d - t0;
     const uint32_t k = (uint32_t)(a - off[ek]);
     const int32_t pre = D.tIdx[a];
-    const float sg = ex ? D.signW32[pre] : D.sign[pre];
+    const float sg = D.sign[pre];
     float r = D.res[pre];
-    R eff = 0;
-    float sv = 0.f;
-    if (ex) {
-      for (int q = 0; q < j; q++) r = r + (1.f - r) * P.xkRec;
-      const float amp = D.tAmp[a];
-      sv = sg * r;
-      if (amp != 1.f) sv = sv * amp;
-      if (sv == 0.f) continue;
-    } else {
-      if (sg == 0) continue;
-      for (int q = 0; q < j; q++) r = (float)((R)r + (R(1) - (R)r) * P.kRec);
-      if (row >= 0 && part == 0 && lane == 0) D.resAt[(int64_t)(row + j) * D.maxArr + k] = r;
-      eff = (R)sg * P.wSyn * d_out<R>(D, pre) * exp((R)D.logGain[pre]) * (R)r * (R)D.tAmp[a];
-    }
+    if (sg == 0) continue;
+    for (int q = 0; q < j; q++) r = (float)((R)r + (R(1) - (R)r) * P.kRec);
+    if (row >= 0 && part == 0 && lane == 0) D.resAt[(int64_t)(row + j) * D.maxArr + k] = r;
+    const R eff = (R)sg * P.wSyn * d_out<R>(D, pre) * exp((R)D.logGain[pre]) * (R)r * (R)D.tAmp[a];
     if (part == 0 && lane == 0) D.wArr[pre] = (uint8_t)(j + 1);
-    const bool inh = ex ? !(sv > 0.f) : !(eff > 0);
+    const bool inh = !(eff > 0);
     const uint32_t key = ((uint32_t)j << 27) | (k << 1) | (inh ? 1u : 0u);
     const uint32_t lo = D.indptr[pre], hi = D.indptr[pre + 1];
     for (uint32_t j0 = lo + 32u * kEdgeILP * part + lane; j0 < hi; j0 += 32u * kEdgeILP * parts) {
@@ -218,11 +207,7 @@ __global__ void __launch_bounds__(kDB, 4) k_wdeliver(const DiffDev *Ds, DP<R> P,
         const uint32_t e = j0 + 32u * u;
         if (!on[u]) continue;
         c[u] = make_uint4(key, e, 0u, 0u);
-        if (ex) {
-          const float dlt = D.W32[e] * sv;
-          on[u] = dlt != 0.f;
-          c[u].z = __float_as_uint(dlt);
-        } else if (sizeof(R) == 8) {
+        if (sizeof(R) == 8) {
           const R p = (R)D.P[e], x = inh ? p * P.inhGain * eff : p * eff;
           const long long b = __double_as_longlong((double)x);
           c[u].z = (uint32_t)b;

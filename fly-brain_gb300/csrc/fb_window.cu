@@ -1555,7 +1555,6 @@ __global__ void driven_pos_kernel(const Trial *trials, WinBrain *win, int set) {
     if (set) W.drvPos[T.driven[k]] = k;
     else W.drvPos[k] = -1;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) W.hasDriven = T.nDriven > 0;
 }
 
 // ---- launch glue ---------------------------------------------------------------------------------
