@@ -159,10 +159,24 @@ def replica_throughput(events, seconds, world):
     return sum_over_ranks(events, world) / max_over_ranks(seconds, world)
 
 
-def algorithmic_bytes(N, steps, spikes, events):
-    """Bytes the step must move (per brain step: 64 B of state per neuron; per delivered spike
-    20 B of row/sign/resource access; 16 B per synaptic event; 16 B per emitted spike)."""
-    return 64.0 * N * steps + 20.0 * spikes + 16.0 * events + 16.0 * spikes
+def algorithmic_bytes(N, passes, spikes, events):
+    """Bytes the steps must move: 64 B of state per neuron and pass over it; per delivered spike
+    20 B of row/sign/resource access; 16 B per synaptic event; 16 B per emitted spike."""
+    return 64.0 * N * passes + 20.0 * spikes + 16.0 * events + 16.0 * spikes
+
+
+def state_passes(steps, sched, p):
+    """Passes over the state that `steps` brain steps take: one a step on the grid schedule, one a
+    window on the delay-scheduled one (the shorter of the delay and the refractory time)."""
+    if sched == "grid":
+        return float(steps)
+    return float(steps) / min(round(p["delay"] / p["dt"]), int(p["tRef"] / p["dt"]))
+
+
+def launches_of(sched, n):
+    """Kernels of n calls after a reset: a windowed call of one brain keeps a copy to go back to, for
+    which the spikes in flight are first written out of the last launch's log."""
+    return 2 * n - 1 if sched == "lagged" else n
 
 
 def cpu_baseline(g, idx, hz, params, sample_steps, bias_mv=0.0, warm_steps=200):
@@ -309,7 +323,7 @@ def run_ours(args, rank, world):
     peak, kind = peaks()
     from flybrain import _native as nat
     sched = "lagged" if brain._batch.last_schedule() == nat.FB_SCHEDULE_LAGGED else "grid"
-    per_launch_bytes = algorithmic_bytes(g.N, S, spikes / args.steps, events / args.steps)
+    per_launch_bytes = algorithmic_bytes(g.N, state_passes(S, sched, SYNTH_PARAMS), spikes / args.steps, events / args.steps)
     achieved = per_launch_bytes / (np.mean(launch_ms) / 1e3) / 1e9
     res = dict(
         metric=METRIC, value=tot_events / dev_s, unit="synaptic events/s", n_gpus=world,
@@ -326,9 +340,9 @@ def run_ours(args, rank, world):
         events=tot_events,
         e2e=dict(value=e2e_events / e2e_s, unit="synaptic events/s", h2d_bytes_per_step=h2d // args.steps,
                  d2h_bytes_per_step=d2h // args.steps, sim_s_per_wall_s=sim_s / e2e_s),
-        gpu_launches=args.steps,  # one persistent kernel each
+        gpu_launches=launches_of(sched, args.steps),
         schedule=sched,
-        roofline=dict(bound="hbm", achieved=achieved, peak=peak, unit="GB/s", frac=achieved / peak,
+        roofline=dict(bound="latency", achieved=achieved, peak=peak, unit="GB/s", frac=achieved / peak,
                       peak_kind=kind, traffic=DRAM_BYTES_PER_STEP_SINGLE[sched] * S,
                       kernel=KERNEL_NAME[sched], algorithmic_bytes_per_launch=per_launch_bytes),
         clocks=clk.summary(),
@@ -421,7 +435,7 @@ def run_high_activity(g, idx, hz, args, bias_mv=HIGH_ACTIVITY_BIAS_MV, launches=
     sim_s = launches * S * SYNTH_PARAMS["dt"] / 1000.0
     sched = "lagged" if brain._batch.last_schedule() == nat.FB_SCHEDULE_LAGGED else "grid"
     peak, kind = peaks()
-    byts = algorithmic_bytes(g.N, S, spikes / launches, events / launches)
+    byts = algorithmic_bytes(g.N, state_passes(S, sched, SYNTH_PARAMS), spikes / launches, events / launches)
     ach = byts / (np.mean(ms) / 1e3) / 1e9
     del brain
     sample = int(os.environ.get("FB_CPU_ACTIVE_SAMPLE_STEPS", "1000"))
@@ -429,8 +443,8 @@ def run_high_activity(g, idx, hz, args, bias_mv=HIGH_ACTIVITY_BIAS_MV, launches=
     return dict(bias_mv=bias_mv, launches=launches, brain_steps=launches * S, events_per_s=events / secs,
                 ms_per_1000_steps=1e3 * secs / (launches * S) * 1000, realtime_factor=sim_s / secs,
                 spikes_per_step=spikes / (launches * S), recurrent_fraction=1.0 - dspikes / max(spikes, 1.0),
-                events_per_step=events / (launches * S), schedule=sched, gpu_launches=launches,
-                roofline=dict(bound="hbm", achieved=ach, peak=peak, unit="GB/s", frac=ach / peak, peak_kind=kind,
+                events_per_step=events / (launches * S), schedule=sched, gpu_launches=launches_of(sched, launches),
+                roofline=dict(bound="latency", achieved=ach, peak=peak, unit="GB/s", frac=ach / peak, peak_kind=kind,
                               traffic=None, kernel=KERNEL_NAME[sched], algorithmic_bytes_per_launch=byts),
                 clocks=clk.summary(),
                 cpu_baseline=dict(value=v, unit="synaptic events/s", cores=1, kind="port",
@@ -605,9 +619,7 @@ def run_batched(g, args, n_trials=256, seed=7, rank=0, world=1):
     mine = trials_of_rank(n_trials, rank, world, "interleaved")
     batch, graphs, _ = build_ensemble(g, spec, p, mine)
     steps = spec["steps"][mine]
-    batch.step(args.warmup * 10)  # warm-up
-    from flybrain.autotune import tune_brains
-    tune = tune_brains(batch, steps=100, key=f"bench-ensemble|B={len(mine)}|N={g.N}|E={g.E}")
+    batch.step(max(2, args.warmup) * 10)  # warm-up
     batch.reset(-1)  # back to rest
     outdeg = g.outdeg().astype(np.int64)
     torch.cuda.synchronize()
@@ -627,7 +639,9 @@ def run_batched(g, args, n_trials=256, seed=7, rank=0, world=1):
     secs = max_over_ranks(secs_local, world)
     trial_sim_s = sum_over_ranks(float(steps.sum()) * p["dt"] / 1000.0, world)
     events_all = sum_over_ranks(events, world)
-    byts = algorithmic_bytes(g.N, float(steps.sum()), spikes, events)
+    from flybrain import _native as nat
+    sched = "lagged" if batch.last_schedule() == nat.FB_SCHEDULE_LAGGED else "grid"
+    byts = algorithmic_bytes(g.N, state_passes(float(steps.sum()), sched, p), spikes, events)
     peak, kind = peaks()
     ach = byts / secs_local / 1e9
     traffic = DRAM_BYTES_PER_TRIAL_STEP_BATCHED * float(steps.sum())
@@ -635,15 +649,13 @@ def run_batched(g, args, n_trials=256, seed=7, rank=0, world=1):
                trial_steps_total=int(steps.sum()), max_steps=int(steps.max()), trial_sim_s=trial_sim_s, wall_s=secs,
                trial_s_per_wall_s=trial_sim_s / secs, events_per_s=events_all / secs, spikes=spikes,
                mean_readout_rate_hz=float(np.mean(readout)),
-               roofline=dict(bound="hbm", achieved=ach, peak=peak, unit="GB/s", frac=ach / peak,
+               roofline=dict(bound="latency", achieved=ach, peak=peak, unit="GB/s", frac=ach / peak,
                              peak_kind=kind, traffic=traffic, algorithmic_bytes=byts,
                              dram_gbs=traffic / secs_local / 1e9, dram_frac=traffic / secs_local / 1e9 / peak,
                              traffic_note="DRAM bytes scaled from a 32-trial ncu capture of the same kernel by "
-                                          "trial-steps; achieved/frac count lif.c's algorithmic bytes, dram_gbs/"
-                                          "dram_frac what DRAM actually carried"),
-               clocks=clk.summary(), gpu_launches=1,
-               tuning=dict(blocks_per_sm=tune["blocks_per_sm"], item_chunks=tune["item_chunks"],
-                           cached=tune["cached"], candidates=len(tune.get("table", []))),
+                                          "trial-steps; achieved/frac count the algorithmic bytes (the state once a "
+                                          "window), dram_gbs/dram_frac what DRAM actually carried"),
+               clocks=clk.summary(), gpu_launches=1, schedule=sched,
                config=f"{n_trials} trials x N=165,122, own seeds, durations U(200,2000) ms, drives "
                       "U{500..4000} neurons at U(50,250) Hz, 64 cell-type gains lognormal(0,0.2); "
                       "one persistent launch, uneven steps; state in HBM (no L2 flush needed: "
