@@ -33,10 +33,12 @@
 // steps at 165,122 neurons and 2,000 driven ones, 1.5 us a step against 4.1 with one synchronised
 // step at a time, and 0.9 at 20,000 and 200. Many brains: U, latency of the state's loads at 32 warps
 // an SM (96 full brains: 780 tiles of 32 neurons per microsecond, 634 us of a window's 970; state
-// crosses HBM once per window instead of once per step), then the deliveries' slot claims (19e9 a
-// second).
+// crosses HBM once per window instead of once per step; the whole launch keeps 45% of the issue slots
+// and a sixth of DRAM busy), then the deliveries' slot claims (19e9 a second).
 //
-// Not covered (the grid kernel runs these): presynaptic inhibition, sequential and fast delivery.
+// Not covered (the grid kernel runs these): presynaptic inhibition, sequential and fast delivery. One
+// brain whose windows would be a few steps long is faster on the lagged kernel (fb_lagged.cu; lag_better
+// in fb_api.cu has the rule).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -422,8 +424,9 @@ __device__ __forceinline__ int find_brain(const uint32_t *pre, int B, uint32_t x
 // ---- U: the other neurons, the whole window ---------------------------------------------------
 //
 // A warp takes tiles of 32 neurons, and the steps between two contributions to any of them run
-// without looking at the lists: about 14 instructions per neuron and step. Bound by instructions
-// (72% of the issue slots). Measured on 96 full brains, a window's U: 769 us when a warp also loaded
+// without looking at the lists: about 14 instructions per neuron and step. Bound by the latency of
+// the state's loads and by instructions: the other warps' steps are what hides a tile's loads. Measured
+// on 96 full brains, a window's U: 769 us when a warp also loaded
 // its next tile ahead (the registers for it spill, and the block's shared memory leaves little L1 to
 // spill to), 641 us with a tile at a time and the other 31 warps to hide its loads, 592 us now; with
 // the next two tiles copied to shared memory ahead no less.
@@ -533,8 +536,8 @@ __device__ __forceinline__ void tile_run(const WarpBrain &T, const Tile &t, bool
       // The refractory count as the step it ends before: a neuron that fires stays refractory to the
       // window's end, and while it is it cannot cross a threshold above vReset. (A count that is not a
       // number lets the neuron integrate but never fire: the other path.) Four instructions fewer per
-      // step, which U of a batch is bound by (96 brains 641 -> 617 us a window); one brain's is not
-      // (its warps have two tiles at most).
+      // step: 96 brains 641 -> 617 us a window; one brain gains nothing (its warps have two tiles at
+      // most).
       int silent = 0;
       float r = x.r;
       for (int q = 0; q < h && __any_sync(0xffffffffu, r > 0); q++)

@@ -9,6 +9,9 @@ namespace fb {
 // us with 32 warps, 1,039 with 16). One brain: the window is a chain of round trips and block
 // barriers, which 16 warps with twice the registers run faster (60,013 conductance-based neurons,
 // window of 4 steps: 32.6 us with 32 warps, 27.3 with 16; the full graph, 18 steps: 28.2 and 26.1).
+// Few brains share the wide form, since the narrow one keeps a single brain's headers: 200 steps of
+// 2 / 4 / 8 brains of 20,000 neurons 303 / 311 / 370 us (one brain 242), on the grid kernel 2,436 /
+// 2,528 / 2,881.
 constexpr int kWinWide = 1024, kWinNarrow = 512;
 inline int window_threads(int B) { return B == 1 ? kWinNarrow : kWinWide; }
 constexpr int kWinMax = 31;         // steps per window at most (five key bits; 31 marks "no entry")
@@ -21,7 +24,10 @@ constexpr int kWarpBrainBytes = 384;
 constexpr int kWinPool = 44032;     // words of that memory: a window's draws and its driven entries
 // Words a driven list's entries take of it.
 __host__ __device__ constexpr int window_entry_words(int nD) { return 3 * nD + (3 * nD + 3) / 4; }
-constexpr int kWinDriven = 4096;    // driven neurons per brain at most
+// Driven neurons per brain at most: the chain's warps hold eight words of 32 entries each, and their
+// entries share the block's memory with a window's draws. A brain beyond that, and its batch, goes to
+// the grid kernel: 20,000 neurons, 200 steps, 4,090 driven 852 us, 4,097 driven 3,593.
+constexpr int kWinDriven = 4096;
 constexpr int kWinSaved = 12;       // words kept of a driven entry at the window's start
 constexpr int kWinBrains = 512;     // brains per launch at most (per-brain words in shared memory)
 constexpr int kWinSpikes = 256;     // arrivals a block delivers at a time

@@ -124,3 +124,31 @@ def test_batches_of_short_windows(trefs, n, windows):
         assert batch.last_schedule() == (nat.FB_SCHEDULE_LAGGED if windows else nat.FB_SCHEDULE_GRID)
         for b, ob in enumerate(obs):
             same(ob, batch, b, (trefs, k, b))
+
+
+@pytest.mark.parametrize("nD,blocks", [(511, 0), (512, 0), (1500, 0), (1500, 1), (33, 2), (2049, 0)])
+@pytest.mark.parametrize("bg", [False, True])
+def test_driven_lists_over_one_and_two_blocks(nD, blocks, bg):
+    """Each driven block's draws follow the other's live entries; launches recorded step by step, too."""
+    from flybrain import BrainBatch, DeviceGraph
+    from flybrain import _native as nat
+    g = make(3000, 23, deg=12)
+    p = params(tRef=0.15, **(dict(BG, depU=0.1) if bg else {}))
+    idx = np.random.default_rng(nD).permutation(g.N)[:nD].astype(np.int32)
+    hz = np.linspace(80.0, 900.0, nD)
+    ob = pair(g, p, 9, idx, hz)
+    b = BrainBatch([DeviceGraph(g)], p, [9])
+    b.set_drive(0, idx, hz)
+    b.set_tuning(lag_driven_blocks=blocks)
+    for n in (40, 7, 150):
+        ob.run(n)
+        b.step(n)
+        assert n < 16 or b.last_schedule() == nat.FB_SCHEDULE_LAGGED
+        same(ob, b, 0, (nD, n))
+    counts, raster = ob.run(64, raster=True)
+    b.record(64, 1 << 20)
+    b.step(64)
+    k, r = b.spike_log(0, 64, 1 << 20)
+    np.testing.assert_array_equal(k, counts)
+    np.testing.assert_array_equal(r, raster)
+    same(ob, b, 0, "recorded")
