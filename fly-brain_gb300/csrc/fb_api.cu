@@ -1472,7 +1472,7 @@ static int run_window(fb_brains *br, int32_t maxSteps, bool forced) {
     CU(cudaMemcpyAsync(R.backup + st, br->trials, sizeof(Trial), cudaMemcpyDeviceToDevice, br->stream));
   }
   if (!R.logValid) {
-    CU(launch_log_import(br->trials, R.win, br->B, br->stream));
+    CU(launch_log_import(br->trials, R.win, br->B, R.maxD, br->stream));
     R.logValid = true;
   }
   std::vector<int32_t> left = br->stepsHost, part(br->B);

@@ -1425,21 +1425,34 @@ extern __shared__ __align__(16) uint32_t s_sort[];
 // ---- the log and the ring ----------------------------------------------------------------------
 
 // The log's spikes of step e, in rank order, to out[0 .. ) (at most cap entries are stored);
-// returns their number. Ranks are marked in a bitmap, `kBits` at a time.
+// returns their number. A thread each: ranks are counted against each other; more: marked in a bitmap,
+// 32 kSortWords at a time.
 constexpr int kSortThreads = 512;
 constexpr int kSortWords = 8192;
 __device__ uint32_t sorted_list(const Trial &T, const WinBrain *W, int64_t e, int32_t *out, int64_t cap, uint32_t *bits,
                                 uint32_t *scan, uint32_t *s_n) {
-  const int tid = threadIdx.x;
+  const uint32_t tid = threadIdx.x;
   const uint32_t lo = W->ls[(uint64_t)e & (kWinRing - 1)], hi = W->logTop, e8 = (uint32_t)e & 255u;
   if (e < 0) return 0;
   if (tid == 0) *s_n = 0;
   __syncthreads();
-  uint32_t mine = 0;
-  for (uint32_t k = lo + tid; k - lo < hi - lo; k += kSortThreads) mine += (W->log[k & W->logMask].x >> 24) == e8;
-  if (mine) atomicAdd(s_n, mine);
+  uint2 *few = (uint2 *)bits;  // {rank, id} of the first kSortThreads
+  for (uint32_t k = lo + tid; k - lo < hi - lo; k += kSortThreads) {
+    const uint4 s = W->log[k & W->logMask];
+    if ((s.x >> 24) != e8) continue;
+    const uint32_t at = atomicAdd(s_n, 1u);
+    if (at < kSortThreads) few[at] = make_uint2(s.y, s.x & 0xffffffu);
+  }
   __syncthreads();
   const uint32_t n = *s_n;
+  if (n <= kSortThreads) {
+    const uint2 s = tid < n ? few[tid] : make_uint2(0u, 0u);
+    uint32_t at = 0;
+    for (uint32_t k = 0; k < n; k++) at += few[k].x < s.x;
+    if (tid < n && (int64_t)at < cap) out[at] = (int32_t)s.y;
+    __syncthreads();
+    return n;
+  }
   uint32_t done = 0;
   constexpr uint32_t kPer = kSortWords / kSortThreads;
   for (uint32_t r0 = 0; done < n && r0 < 2u * (uint32_t)T.N; r0 += kSortWords * 32u) {
@@ -1489,24 +1502,35 @@ __global__ void __launch_bounds__(kSortThreads) log_export_kernel(Trial *trials,
   }
 }
 
-__global__ void __launch_bounds__(1024) log_import_kernel(Trial *trials, WinBrain *win) {
-  const Trial &T = trials[blockIdx.x];
-  WinBrain *W = win + blockIdx.x;
-  const uint32_t top0 = W->logTop;
-  uint32_t top = top0;
-  for (int j = 0; j < W->D; j++) {
-    const int slot = (T.head + j) % T.nslots;
-    const int64_t e = T.stepsDone + j - W->D;
-    const int32_t n = T.ringCount[slot];
-    for (int32_t k = threadIdx.x; k < n; k += blockDim.x) {
-      const int32_t i = T.ring[(int64_t)slot * T.N + k];
-      W->log[(top + k) & W->logMask] = make_uint4((uint32_t)i | (((uint32_t)e & 255u) << 24), (uint32_t)k, T.indptr[i], T.indptr[i + 1]);
+// One block per slot in flight and brain; the log starts over. Two steps and one step in turn, 20,000
+// neurons: 120 us a pair with one block for all slots of a brain and bitmaps for every list, 110 now.
+__global__ void __launch_bounds__(256) log_import_kernel(const Trial *trials, WinBrain *win) {
+  __shared__ uint32_t s_top, s_end;
+  const Trial &T = trials[blockIdx.y];
+  WinBrain *W = win + blockIdx.y;
+  const int D = W->D, j = (int)blockIdx.x;  // D <= 32
+  if (j >= D) return;
+  if (threadIdx.x < 32) {
+    const int k = (int)threadIdx.x;
+    const uint32_t n = k < D ? (uint32_t)T.ringCount[(T.head + k) % T.nslots] : 0u;
+    const uint32_t before = __reduce_add_sync(0xffffffffu, k < j ? n : 0u), own = __shfl_sync(0xffffffffu, n, j);
+    if (k == 0) {
+      s_top = before;
+      s_end = before + own;
     }
-    if (threadIdx.x == 0) W->ls[(uint64_t)e & (kWinRing - 1)] = top;
-    top += n;
   }
   __syncthreads();
-  if (threadIdx.x == 0) W->logTop = top;
+  const uint32_t top = s_top, n = s_end - top;
+  const int64_t e = T.stepsDone + j - D;
+  const int32_t *list = T.ring + (int64_t)((T.head + j) % T.nslots) * T.N;
+  for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
+    const int32_t i = list[k];
+    W->log[(top + k) & W->logMask] = make_uint4((uint32_t)i | (((uint32_t)e & 255u) << 24), k, T.indptr[i], T.indptr[i + 1]);
+  }
+  if (threadIdx.x == 0) {
+    W->ls[(uint64_t)e & (kWinRing - 1)] = top;
+    if (j == D - 1) W->logTop = top + n;
+  }
 }
 
 __global__ void log_clear_kernel(WinBrain *win, int b0) {
@@ -1652,8 +1676,8 @@ cudaError_t launch_driven_pos(const Trial *trials, WinBrain *win, int B, cudaStr
   return cudaGetLastError();
 }
 
-cudaError_t launch_log_import(Trial *trials, WinBrain *win, int B, cudaStream_t st) {
-  log_import_kernel<<<B, 1024, 0, st>>>(trials, win);
+cudaError_t launch_log_import(const Trial *trials, WinBrain *win, int B, int maxD, cudaStream_t st) {
+  log_import_kernel<<<dim3(maxD, B), 256, 0, st>>>(trials, win);
   return cudaGetLastError();
 }
 cudaError_t launch_log_export(Trial *trials, WinBrain *win, int b0, int b1, int maxD, bool lastOnly, cudaStream_t st) {

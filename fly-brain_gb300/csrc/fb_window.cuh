@@ -96,7 +96,7 @@ cudaError_t launch_in_offsets(const uint32_t *indices, int32_t N, int64_t E, uin
 cudaError_t launch_driven_pos(const Trial *trials, WinBrain *win, int B, cudaStream_t st);
 // The ring's spikes in flight into the log (import), the log's into the ring (export: every slot
 // in flight, or the last step's list only), the log emptied (brains b0 .. b1-1).
-cudaError_t launch_log_import(Trial *trials, WinBrain *win, int B, cudaStream_t st);
+cudaError_t launch_log_import(const Trial *trials, WinBrain *win, int B, int maxD, cudaStream_t st);
 cudaError_t launch_log_export(Trial *trials, WinBrain *win, int b0, int b1, int maxD, bool lastOnly, cudaStream_t st);
 cudaError_t launch_log_clear(WinBrain *win, int b0, int b1, cudaStream_t st);
 // Appends the fired lists of the last n steps (at most the window's) to the per-step record.

@@ -203,3 +203,25 @@ def test_single_steps_take_no_window_buffers():
     batch.step(20)
     assert batch.last_schedule() == nat.FB_SCHEDULE_LAGGED
     assert before - torch.cuda.mem_get_info()[0] >= 2 * 8 * g.E
+
+
+@pytest.mark.parametrize("nD", [1, 511, 512, 513, 1700])
+@pytest.mark.parametrize("B", [1, 3])
+def test_fired_lists_handed_over(nD, B):
+    """Lists of as many spikes as the export has threads (512), fewer and more, out of the log and back
+    into it, several slots at once."""
+    p = params(tRef=0.9, **DEP)
+    obs, batch = brains(B, p, N=2000, hz=1e5, every=1)
+    for b, ob in enumerate(obs):
+        for i in range(nD, ob.N):
+            ob.setDriveOne(i, 0.0)
+        batch.set_drive(b, np.arange(nD, ob.N, dtype=np.int32), 0.0)
+    most = 0
+    for n in (13, 1, 1, 24, 1, 3, 40, 1):
+        for ob in obs:
+            ob.run(n)
+        batch.step(n)
+        most = max(most, int(obs[0].ringCount.max()))
+        for b, ob in enumerate(obs):
+            same(ob, batch, b, (nD, n, b))
+    assert most >= nD
