@@ -489,7 +489,8 @@ struct fb_brains {
   int32_t *h_groups = nullptr;
   size_t hDeltaCap = 0, hGroupCap = 0;
   int32_t *h_small = nullptr;  // [2 + B]: error flag, unused, fired count of each brain
-  int32_t *h_steps = nullptr;  // [B]
+  int32_t *h_steps = nullptr;  // [2][B]: an upload takes the half that the one before did not
+  int stepsHalf = 0;
   std::vector<int32_t> stepsUploaded, groupStarts;
   cudaEvent_t flushDone = nullptr;
   bool flushPending = false;
@@ -705,7 +706,7 @@ extern "C" int fb_brains_create(const fb_graph *const *graphs, int32_t B, const 
   cudaEventCreate(&br->ev1);
   cudaEventCreateWithFlags(&br->flushDone, cudaEventDisableTiming);
   if (cudaMallocHost(&br->h_small, sizeof(int32_t) * (2 + (size_t)B)) != cudaSuccess ||
-      cudaMallocHost(&br->h_steps, sizeof(int32_t) * (size_t)B) != cudaSuccess)
+      cudaMallocHost(&br->h_steps, sizeof(int32_t) * 2 * (size_t)B) != cudaSuccess)
     return brains_fail_cleanup(br, fail(FB_ENOMEM, "fb_brains_create: pinned host staging"));
   if (cudaStreamSynchronize(br->stream) != cudaSuccess)
     return brains_fail_cleanup(br, fail(FB_ECUDA, "fb_brains_create: %s", cudaGetErrorString(cudaGetLastError())));
@@ -1412,6 +1413,17 @@ static int win_setup(fb_brains *br) {
   return FB_OK;
 }
 
+// The step counts of a launch, unless the last one's are the same. A call uploads at most twice (a
+// recorded launch's whole windows and its last one) and ends synchronised.
+static int upload_steps(fb_brains *br, const std::vector<int32_t> &steps) {
+  if (br->stepsUploaded == steps) return FB_OK;
+  int32_t *h = br->h_steps + (size_t)br->B * (br->stepsHalf ^= 1);
+  std::memcpy(h, steps.data(), sizeof(int32_t) * br->B);
+  CU(cudaMemcpyAsync(br->d_steps, h, sizeof(int32_t) * br->B, cudaMemcpyHostToDevice, br->stream));
+  br->stepsUploaded = steps;
+  return FB_OK;
+}
+
 // One windowed launch of steps[b] steps.
 static int win_launch(fb_brains *br, const std::vector<int32_t> &steps) {
   WinRes &R = br->win;
@@ -1431,11 +1443,8 @@ static int win_launch(fb_brains *br, const std::vector<int32_t> &steps) {
   if (a.nWin == 0) return FB_OK;
   if (changed)
     CU(cudaMemcpy2DAsync(&R.win[0].H, sizeof(WinBrain), &R.host[0].H, sizeof(WinBrain), 4, br->B, cudaMemcpyHostToDevice, br->stream));
-  if (br->stepsUploaded != steps) {  // the last launch's counts stay on the device otherwise
-    std::memcpy(br->h_steps, steps.data(), sizeof(int32_t) * br->B);
-    CU(cudaMemcpyAsync(br->d_steps, br->h_steps, sizeof(int32_t) * br->B, cudaMemcpyHostToDevice, br->stream));
-    br->stepsUploaded = steps;
-  }
+  int rc = upload_steps(br, steps);
+  if (rc) return rc;
   a.trials = br->trials;
   a.win = R.win;
   a.B = br->B;
@@ -1480,7 +1489,6 @@ static int run_window(fb_brains *br, int32_t maxSteps, bool forced) {
   for (int32_t done = 0, n; done < maxSteps; done += n) {
     n = maxSteps - done;
     if (br->logging) n = std::min(n, (int32_t)window_steps(br->host[0], (int64_t)br->driven[0].order.size()));
-    if (done) CU(cudaStreamSynchronize(br->stream));  // the pinned step counts are free again
     for (int b = 0; b < br->B; b++) {
       part[b] = std::min(left[b], n);
       left[b] -= part[b];
@@ -1540,13 +1548,19 @@ static bool is_irregular(const fb_brains *br) {
 // H 5, 512 steps 1,411 / 1,507. At H 4 the two are close: over 1,501 to 165,122 neurons and dt 0.1 and
 // 0.5 ms, 512 steps, windowed over lagged 0.83 to 1.21 without background events (mean 1.04); with them
 // 0.73 to 1.04 up to 60,013 neurons, 0.98 and 1.19 at 165,122 (there 64 steps 645 / 617, 32 steps 349 /
-// 367 at dt 0.5 ms). The lagged kernel's tile blocks hold at most kLagPer neurons per thread.
+// 367 at dt 0.5 ms). The lagged kernel's tile blocks hold at most kLagPer neurons per thread. A recorded
+// window is a launch with its record of its own, about 30 us (dt 0.5 ms, windows of four steps, windowed /
+// lagged: 20,000 neurons, 8 steps 89 / 98, 16 steps 136 / 122, 64 steps 458 / 259; 165,122 neurons, 16
+// steps 185 / 199, 24 steps 266 / 234; windows of eight, 20,000 neurons, 32 steps 147 / 171, 64 steps 268 /
+// 252).
 static bool lag_better(const fb_brains *br, int32_t n) {
   const Trial &T = br->host[0];
   const int tb = br->sms - kLagMaxDB;
   if (br->B != 1 || (T.N + tb - 1) / tb > kLagPer * kLagTileWorkers) return false;
   if (is_irregular(br)) return n >= kLagMinSteps;
-  switch (window_steps(T, (int64_t)br->driven[0].order.size())) {
+  const int H = window_steps(T, (int64_t)br->driven[0].order.size());
+  if (br->logging) return n >= kLagMinSteps && 14 * ((n + H - 1) / H) > n + (T.N >= 50000 ? 40 : 28);
+  switch (H) {
     case 1: return n >= kLagMinSteps;
     case 2: return n >= 16;
     case 3: return n >= 64;
@@ -1671,11 +1685,7 @@ static int run_launch(fb_brains *br, int32_t maxSteps, bool head, int32_t *out_n
     br->win.slotsValid = true;
     br->win.logValid = false;
     br->everRing = true;
-    if (br->stepsUploaded != br->stepsHost) {  // the last launch's counts stay on the device otherwise
-      std::memcpy(br->h_steps, br->stepsHost.data(), sizeof(int32_t) * br->B);
-      CU(cudaMemcpyAsync(br->d_steps, br->h_steps, sizeof(int32_t) * br->B, cudaMemcpyHostToDevice, br->stream));
-      br->stepsUploaded = br->stepsHost;
-    }
+    if ((rc = upload_steps(br, br->stepsHost))) return rc;
     StepArgs a;
     memset(&a, 0, sizeof a);
     a.trials = br->trials;

@@ -152,3 +152,20 @@ def test_driven_lists_over_one_and_two_blocks(nD, blocks, bg):
     np.testing.assert_array_equal(k, counts)
     np.testing.assert_array_equal(r, raster)
     same(ob, b, 0, "recorded")
+
+
+@pytest.mark.parametrize("tref,delay", [(0.25, 3.2), (2.2, 0.4), (0.7, 1.8)])
+@pytest.mark.parametrize("over", [dict(), dict(BG, **GEN)])
+def test_recorded_launches(tref, delay, over):
+    """A record of few windows is written by the windowed kernel, one of many by the other: both sides of
+    the rule in turn, last windows whole and partial, counts and lists of every step."""
+    ob, b = brain(params(tRef=tref, delay=delay, **over))
+    for n in (5, 8, 9, 16, 12, 64, 3, 24, 20, 63, 32):
+        counts, raster = ob.run(n, raster=True)
+        b.record(n, 1 << 18)
+        b.step(n)
+        k, r = b.spike_log(0, n, 1 << 18)
+        b.record(0, 0)
+        np.testing.assert_array_equal(k, counts, err_msg=str(n))
+        np.testing.assert_array_equal(r, raster, err_msg=str(n))
+        same(ob, b, 0, (tref, n))
