@@ -997,6 +997,8 @@ extern "C" int fb_set_background(fb_brains *br, int32_t b, double rate_hz, doubl
   return FB_OK;
 }
 
+static uint64_t log_capacity(const Trial &T);
+
 // LIFGpu.setParams (src/lifgpu.js:349): new parameters for brain b's header constants, taking
 // effect at the next step. The ring depth round(delay/dt)+1 must not change (the ring and the
 // windowed buffers are sized by it). Constant-state flags stay only while their condition
@@ -1024,9 +1026,9 @@ extern "C" int fb_set_params(fb_brains *br, int32_t b, const fb_params *p) {
   else if ((T.flags & kHasPreInh) && mode == FB_DELIVER_SEQUENTIAL) mode = FB_DELIVER_EXACT;
   if (T.tRef != nt.tRef || T.dt != nt.dt) {
     // neurons may now fire sooner than the windows and the log assume: the windowed kernel's
-    // resources are sized again at its next launch, from the ring
+    // resources are sized again at its next launch, from the ring, if the log is too small
     br->irregular[b] = T.nslots - 1;
-    if (br->win.ready) {
+    if (br->win.ready && log_capacity(nt) > (uint64_t)br->win.host[b].logMask + 1) {
       if ((rc = ring_from_log(br))) return rc;
       CU(cudaStreamSynchronize(br->stream));
       br->win.ready = false;
@@ -1309,6 +1311,13 @@ static int win_alloc(fb_brains *br, X **p, size_t n) {
   return FB_OK;
 }
 
+// Spikes of the last D + H steps: a neuron fires at most once in any H of them (H 0: windows do not apply).
+static uint64_t log_capacity(const Trial &T) {
+  const int D = T.nslots - 1, H = std::min(D, silent_steps(T));
+  uint64_t cap = 1024;
+  while (H > 0 && cap < (uint64_t)T.N * ((D + H - 1) / H + 2)) cap *= 2;
+  return cap;
+}
 static size_t bg_hit_bytes(const Trial &T) { return align256((size_t)T.N * std::min(T.nslots - 1, kWinMax) * 4); }
 // The kernel's resources: one allocation for the batch, at its first windowed launch (batches that only
 // take single steps or the grid schedule do without).
@@ -1328,12 +1337,10 @@ static int win_create(fb_brains *br) {
   auto n4 = [&](int b) { return align256((size_t)br->host[b].N * 4); };
   // what must start at zero comes first: per brain drvPos, bgMask and arr (wcnt from the offsets)
   size_t zero = align256(sizeof(WinBrain) * B) + align256(256 * 4 + (size_t)B * kWarpBrainBytes), rest = 0;
-  std::vector<uint64_t> cap(B, 1024);
+  std::vector<uint64_t> cap(B);
   for (int b = 0; b < B; b++) {
     const Trial &T = br->host[b];
-    // spikes of the last D + H steps: a neuron fires at most once in any H of them (H >= 1)
-    const int D = T.nslots - 1, H = std::min(D, silent_steps(T));
-    while (cap[b] < (uint64_t)T.N * ((D + H - 1) / H + 2)) cap[b] *= 2;
+    cap[b] = log_capacity(T);
     zero += 2 * n4(b) + align256(T.N) + ((T.flags & kHasBg) ? bg_hit_bytes(T) : 0);
     rest += n4(b) + align256(cap[b] * 16) + align256((size_t)T.E * 8) + align256((size_t)kWinDriven * (4 + kWinSaved * 4 + 1));
   }
@@ -1744,16 +1751,23 @@ static int run_launch(fb_brains *br, int32_t maxSteps, bool head, int32_t *out_n
 
 // The steps of a call that run apart, before its windows: those for which brains are irregular, where
 // windows repay a second launch. Microseconds for refr written and n steps, whole / apart, 18 of them
-// irregular: one brain of 20,000 neurons, 49 steps 237 / 252 for 50, of 165,122 neurons 344 / 367 (the
-// whole on the lagged kernel); a batch of four, 20,000 each, 49 steps 642 / 384 (on the grid kernel).
-constexpr int kSplitRest = 32, kSplitRestBatch = 8;
+// irregular: one brain of 20,000 neurons, 49 steps 237 / 252, 100 steps 389 / 302, of 165,122 neurons 49
+// steps 344 / 367 (the whole on the lagged kernel); a batch of four, 20,000 each, 49 steps 642 / 384 (on the
+// grid kernel). A window costs one brain as much as 6.5 steps of the lagged kernel, the second launch as much
+// as 35: in windows of four steps, 20,000 neurons, 100 steps 398 / 485.
+constexpr int kSplitRestBatch = 8;
+static bool split_pays(const fb_brains *br, int32_t rest) {
+  if (br->B > 1) return rest >= kSplitRestBatch;
+  const int H = window_steps(br->host[0], (int64_t)br->driven[0].order.size());
+  return (int64_t)rest * (2 * H - 13) > 70 * H;
+}
 static int32_t split_steps(fb_brains *br, int32_t maxSteps) {
   int32_t head = 0;
   for (int b = 0; b < br->B; b++) {
     if (br->irregular[b] > br->stepsHost[b]) return 0;
     head = std::max(head, br->irregular[b]);
   }
-  if (head == 0 || maxSteps - head < (br->B == 1 ? kSplitRest : kSplitRestBatch) || br->schedule == FB_SCHEDULE_GRID || br->logging || br->profiling) return 0;
+  if (head == 0 || !split_pays(br, maxSteps - head) || br->schedule == FB_SCHEDULE_GRID || br->logging || br->profiling) return 0;
   if (!win_capable(br) || br->win.noMemory) return 0;
   std::vector<int32_t> now(br->B, 0);
   now.swap(br->irregular);

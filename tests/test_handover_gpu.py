@@ -240,3 +240,23 @@ def test_short_launches_between_single_steps(N, n, grid):
         want = nat.FB_SCHEDULE_GRID if m == 1 or (grid and k != 5 and m == n) else nat.FB_SCHEDULE_LAGGED
         assert batch.last_schedule() == want, k
         same(ob, batch, 0, (N, n, k))
+
+
+@pytest.mark.parametrize("trefs", [(2.2, 3.0, 2.2, 1.6, 2.4), (2.2, 0.0, 2.2, 0.3, 0.2, 1.8)])
+def test_new_refractory_times_keep_the_window_buffers(trefs):
+    """They are made again only where the log must hold more spikes than before."""
+    import torch
+    p = params(depU=0.1)
+    obs, batch = brains(1, p, N=1500, hz=1e5, every=2, deg=700)
+    ob = obs[0]
+    free = None
+    for k, tref in enumerate(trefs):
+        set_tref(ob, batch, 0, p, tref)
+        for n in (6, 90, 25):
+            ob.run(n)
+            batch.step(n)
+            same(ob, batch, 0, (tref, n))
+        if k == 0:
+            free = torch.cuda.mem_get_info()[0]
+        elif min(trefs) > 1.0:
+            assert torch.cuda.mem_get_info()[0] == free, tref
