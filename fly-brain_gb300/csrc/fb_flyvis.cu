@@ -50,7 +50,7 @@ int fvfail(int code, const char *fmt, ...) {
 
 constexpr int kFvThreads = 256;       // the other kernels
 constexpr int kFvStepThreads = 1024;
-constexpr int kFvWidth = 16;  // vectors per chunk
+constexpr int kFvWidth = 64;  // words per chunk at most
 
 // V instances of a row of r.
 template <int V>
@@ -500,20 +500,23 @@ extern "C" int fb_flyvis_read(fb_flyvis *f, int32_t field, int32_t b, float *out
 
 // Instances per lane, at most `most`: one while all (target, instance) pairs take a third of the chip's
 // 311,296 resident threads, two until they take all of them, then four. Microseconds for 20 steps at
-// 1 / 2 / 4: 3,000 neurons and 4 eyes 135 / 175 / 216, 6,000 and 16 (96,000 pairs) 175 / 175 / 176,
-// 45,669 and 3 (137,000) 296 / 257 / 296, 24,000 and 8 (192,000) 218 / 216 / 230, 45,669 and 5 (228,000)
-// 339 / 337 / 337, 12,000 and 33 (396,000) 339 / 334 / 299, 45,669 and 64 1,472 / 963 / 787.
+// 1 / 2 / 4: 3,000 neurons and 4 eyes 136 / 175 / 217, 6,000 and 16 (96,000 pairs) 167 / 175 / 177, 20,000
+// and 6 (120,000) 214 / 202 / 263, 24,000 and 8 (192,000) 219 / 216 / 226, 45,669 and 6 (274,000) 299 / 283 /
+// 298, 24,000 and 13 (312,000) 299 / 299 / 295, 45,669 and 8 (365,000) 341 / 328 / 299, 45,669 and 64 1,332 /
+// 919 / 785.
 static int32_t fv_width(const fb_flyvis *f, int32_t most) {
   const int64_t pairs = (int64_t)f->N * f->B;
   return pairs <= 100000 ? 1 : std::min(most, pairs <= 300000 ? 2 : 4);
 }
 
-// One step from `gin` (rows of `pitch` words). The chunks are at most kFvWidth vectors. Blocks of
-// 1,024 threads, one per SM, leave one block to balance a run of targets in; with fewer lanes than
-// that, blocks of 256 spread them over the SMs (8 eyes of the full network 14.5 us a step against
-// 18.6, 24 eyes 22.7 against 20.9).
+// One step from `gin` (rows of `pitch` words). The lanes are those of the instances, not of the rows'
+// padding (20,000 neurons and 5 eyes, 20 steps 265 us with lanes for it, 198 without). A chunk is at most
+// kFvWidth words wide whatever the lane's width: in chunks of 16 words a row of 17 eyes was read in two
+// parts (the full network, a call of one step: 43 us, now 37). Blocks of 1,024 threads, one per SM, leave
+// one block to balance a run of targets in; with fewer lanes than that, blocks of 256 spread them over the
+// SMs (8 eyes of the full network 14.5 us a step against 18.6, 24 eyes 22.7 against 20.9).
 static void fv_launch(fb_flyvis *f, int V, int mode, int32_t pitch, const float *gin, float *rout, float *vout) {
-  const int32_t vecs = pitch / V, chunks = (vecs + kFvWidth - 1) / kFvWidth, width = (vecs + chunks - 1) / chunks;
+  const int32_t vecs = (f->B + V - 1) / V, chunks = (vecs * V + kFvWidth - 1) / kFvWidth, width = (vecs + chunks - 1) / chunks;
   const int64_t lanes = (int64_t)f->N * width * chunks;
   const int threads = lanes <= (int64_t)f->sms * kFvStepThreads ? 256 : kFvStepThreads;
   const int grid = (int)std::min<int64_t>((lanes + threads - 1) / threads, (int64_t)f->sms * (kFvStepThreads / threads));
@@ -532,10 +535,10 @@ extern "C" int fb_flyvis_step(fb_flyvis *f, int32_t nsteps) {
   FVCU(cudaEventRecord(f->ev0, f->st));
   // instances per lane from r, and from v, whose rows hold whole vectors of this many
   const int32_t vecR = fv_width(f, f->vec), vecV = fv_width(f, f->B % 4 == 0 ? 4 : f->B % 2 == 0 ? 2 : 1);
-  // a first step that would gather narrower than r allows: a pass that makes r costs 5 us and repays
-  // itself from about a million pairs on (13 eyes of the full network 32 us with narrow gathers, 40
-  // with the pass, 33 eyes 58 and 53)
-  const bool pass = f->r[0] && vecV < vecR && (int64_t)f->N * f->B >= 1000000;
+  // a first step that would gather one instance per lane where r allows more: the pass that makes r
+  // repays itself from some 2.2 million pairs on (the full network, calls of one step without / with it: 35
+  // eyes 53 / 53 us, 49 eyes 65 / 63, 97 eyes 118 / 102); two per lane do as well without (66 eyes 66 / 84)
+  const bool pass = f->r[0] && vecV == 1 && vecV < vecR && (int64_t)f->N * f->B >= 2200000;
   for (int32_t s = 0, in = 0; s < nsteps; s++) {
     const bool more = f->r[0] && s + 1 < nsteps;
     if (!f->r[0] || (s == 0 && !pass)) {

@@ -154,3 +154,23 @@ def test_instances_per_lane(N, B):
         O.fv_run(m, v, x, steps)
         for b in range(B):
             np.testing.assert_array_equal(fv.v(b), v[b])
+
+
+@pytest.mark.parametrize("N,B", [(1000, 64), (1000, 65), (700, 129), (20000, 17), (20000, 66), (22222, 99), (22223, 99)])
+def test_odd_eyes(N, B):
+    """Rows whose padding has no lanes, chunks of 64 words and one more, and both sides of where a call
+    first makes the rectified rows; calls of one and of several steps."""
+    from oracle import oracle as O
+    from flybrain.flyvis import FlyVis, synth_flyvis
+    m = synth_flyvis(N=N, seed=6, mean_in=5.0)
+    rng = np.random.default_rng(N + B)
+    x = rng.normal(0.0, 0.6, (B, N)).astype(np.float32)
+    fv = FlyVis(m, B=B)
+    v = np.tile(m["bias"], (B, 1)).astype(np.float32)
+    for b in range(B):
+        fv.write("x", b, x[b])
+    for steps in (2, 1, 4):
+        fv.step(steps)
+        O.fv_run(m, v, x, steps)
+        for b in range(B):
+            np.testing.assert_array_equal(fv.v(b), v[b])
