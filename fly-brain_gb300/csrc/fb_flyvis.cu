@@ -291,7 +291,8 @@ struct fb_flyvis {
   bool finite = true;                     // every weight is
   int32_t *idxBuf = nullptr, *err = nullptr, *win = nullptr;
   int64_t idxCap = 0;
-  int32_t *list = nullptr;  // pinned: kFvList indices and values, the error word; null: none to be had
+  int32_t *list = nullptr;  // pinned: kFvList indices and values, the error word; null: none yet
+  int32_t lists = 0;        // host lists set until it was there; kFvPinAfter: none to be had
   int cur = 0, grid = 0, sms = 0;
   cudaStream_t st = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -381,10 +382,6 @@ extern "C" int fb_flyvis_create(int32_t N, int64_t E, const int32_t *indptr, con
   if (cudaStreamCreateWithFlags(&f->st, cudaStreamNonBlocking) != cudaSuccess || cudaEventCreate(&f->ev0) != cudaSuccess ||
       cudaEventCreate(&f->ev1) != cudaSuccess)
     return bail(fvfail(FB_ECUDA, "fb_flyvis_create: stream setup failed"));
-  if (cudaHostAlloc((void **)&f->list, (2 * kFvList + 1) * 4, cudaHostAllocDefault) != cudaSuccess) {
-    f->list = nullptr;
-    cudaGetLastError();
-  }
   // without room for r every step gathers v
   if (cudaMalloc(&f->r[0], rb) != cudaSuccess || cudaMalloc(&f->r[1], rb) != cudaSuccess) {
     if (f->r[0]) cudaFree(f->r[0]);
@@ -430,6 +427,10 @@ extern "C" int fb_flyvis_reset(fb_flyvis *f, int32_t b) {
   return FB_OK;
 }
 
+// The pinned copy costs 300 us and saves a list 5 to 9: it comes with this many lists. (A model of 100
+// neurons, created and given one list: 670 us with a copy made at creation, now 390.)
+constexpr int32_t kFvPinAfter = 32;
+
 // Whether p is plain host memory.
 static bool fv_host(const void *p) {
   cudaPointerAttributes a;
@@ -447,7 +448,13 @@ extern "C" int fb_flyvis_set_input(fb_flyvis *f, int32_t b, int32_t n, const int
   if (n == 0) return FB_OK;
   // one kernel that reads the pinned copy, where a block holds the list (5,768 values: 31 us a call,
   // with two copies, two kernels and the error word's copy 36)
-  if (f->list && n <= kFvList && fv_host(idx) && fv_host(values)) {
+  const bool small = n <= kFvList && fv_host(idx) && fv_host(values);
+  if (small && f->lists < kFvPinAfter && ++f->lists == kFvPinAfter &&
+      cudaHostAlloc((void **)&f->list, (2 * kFvList + 1) * 4, cudaHostAllocDefault) != cudaSuccess) {
+    f->list = nullptr;
+    cudaGetLastError();
+  }
+  if (f->list && small) {
     int32_t *err = f->list + 2 * n;
     memcpy(f->list, idx, (size_t)n * 4);
     memcpy(f->list + n, values, (size_t)n * 4);

@@ -174,3 +174,30 @@ def test_odd_eyes(N, B):
         O.fv_run(m, v, x, steps)
         for b in range(B):
             np.testing.assert_array_equal(fv.v(b), v[b])
+
+
+def test_many_input_lists():
+    """The lists before, at and after the one that brings the pinned copy (the 32nd), a bad index in
+    some."""
+    from flybrain import _native as nat
+    from flybrain.flyvis import FlyVis, synth_flyvis
+    m = synth_flyvis(N=700, seed=4, columns=12)
+    rng = np.random.default_rng(9)
+    fv = FlyVis(m, B=2)
+    ref = np.zeros(700, np.float32)
+    for k in range(36):
+        idx = rng.integers(0, 700, 500).astype(np.int32)
+        val = rng.normal(0, 1, 500).astype(np.float32)
+        bad = k % 3 == 1
+        if bad:
+            idx[77] = -1
+        for i, y in zip(idx, val):
+            if i >= 0:
+                ref[i] = y
+        if bad:
+            with pytest.raises(nat.FlyBrainError):
+                fv.set_input(idx, val, 1)
+        else:
+            fv.set_input(idx, val, 1)
+        np.testing.assert_array_equal(fv.read("x", 1), ref)
+    assert not fv.read("x", 0).any()
