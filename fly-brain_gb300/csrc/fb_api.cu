@@ -525,7 +525,8 @@ struct fb_brains {
   std::vector<Topology *> topo;      // each brain's (the graphs outlive the batch)
   int maxSlots = 0;
   bool everRing = false;             // a kernel that keeps the ring's lists has run
-  bool wasShort = false;             // the last launch had too few steps for windows
+  int32_t sinceShort = kLongAgo;     // launches since one that had too few steps for windows
+  static constexpr int32_t kLongAgo = 1 << 20;
 };
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -1598,12 +1599,13 @@ static bool windows_pay(const fb_brains *br, int32_t n) {
 }
 
 // Whether this launch repays the way of the spikes in flight into the log and, if the caller goes back
-// to single steps, out of it: some 40 us after a launch that was too short for windows. Microseconds for n
-// steps and one step in turn, on the grid kernel / with windows: 1,501 neurons, n 2 86 / 108, n 4 106 / 108,
-// n 6 121 / 108; 20,000 neurons 98 / 112, 120 / 110, 138 / 111; four brains of 20,000 in windows of four
-// steps, n 4 145 / 138, n 5 157 / 168, n 6 172 / 169; 165,122 neurons, n 2 122 / 127, n 3 147 / 127.
+// to single steps, out of it: some 40 us soon after a launch that was too short for windows. Microseconds for
+// n steps and one step in turn, on the grid kernel / with windows: 1,501 neurons, n 2 86 / 108, n 4 106 /
+// 108, n 6 121 / 108; 20,000 neurons 98 / 112, 120 / 110, 138 / 111; four brains of 20,000 in windows of four
+// steps, n 4 145 / 138, n 5 157 / 168, n 6 172 / 169; 165,122 neurons, n 2 122 / 127, n 3 147 / 127. Three
+// launches of two steps and one step: 1,501 neurons 173 / 190, 20,000 neurons 207 / 203.
 static bool handover_pays(const fb_brains *br, int32_t n) {
-  if (br->win.logValid || !br->wasShort || n >= 6) return true;
+  if (br->win.logValid || n >= 6) return true;
   int64_t neurons = 0;
   int H = kWinMax;
   for (int b = 0; b < br->B; b++) {
@@ -1611,6 +1613,7 @@ static bool handover_pays(const fb_brains *br, int32_t n) {
     H = std::min(H, window_steps(br->host[b], (int64_t)br->driven[b].order.size()));
   }
   neurons /= br->B;
+  if (br->sinceShort >= (neurons >= 10000 ? 1 : 4)) return true;
   return neurons >= 100000 ? n >= 3 : neurons >= 10000 && n >= 4 && n <= H;
 }
 
@@ -1651,7 +1654,8 @@ static int run_launch(fb_brains *br, int32_t maxSteps, bool head, int32_t *out_n
   int rc;
   StepKernel kernel;
   if ((rc = choose_kernel(br, maxSteps, head, &kernel))) return rc;
-  if (maxSteps > 0) br->wasShort = kernel == StepKernel::kGrid && maxSteps < win_min_steps(br);
+  if (maxSteps > 0)
+    br->sinceShort = kernel == StepKernel::kGrid && maxSteps < win_min_steps(br) ? 0 : std::min(br->sinceShort + 1, fb_brains::kLongAgo);
   // the error flag and the fired counts come back in one synchronisation
   auto read_back = [&]() -> int {
     CU(cudaMemcpyAsync(br->h_small, br->d_err, 4, cudaMemcpyDeviceToHost, br->stream));

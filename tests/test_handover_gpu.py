@@ -227,17 +227,19 @@ def test_fired_lists_handed_over(nD, B):
     assert most >= nD
 
 
-@pytest.mark.parametrize("N,n,grid", [(400, 5, True), (400, 6, False), (12000, 3, True), (12000, 4, False), (12000, 5, False)])
-def test_short_launches_between_single_steps(N, n, grid):
-    """They stay on the grid kernel where the way into the log and back costs more; a second one in
-    a row does not."""
+@pytest.mark.parametrize("N,n,first", [(400, 2, 5), (400, 5, 5), (400, 6, 1), (12000, 3, 2), (12000, 4, 1), (12000, 5, 1)])
+def test_short_launches_between_single_steps(N, n, first):
+    """They stay on the grid kernel where the way into the log and back costs more: `first` is the
+    launch after a single step that takes windows."""
     from flybrain import _native as nat
     obs, batch = brains(1, params(**DEP), N=N, hz=2000.0, deg=6)
     ob = obs[0]
-    for k, m in enumerate((30, 1, n, 1, n, n, 1)):
+    since = 100
+    for k, m in enumerate([30, 1, n, 1] + 7 * [n] + [1, n, n, 1]):
         ob.run(m)
         batch.step(m)
-        want = nat.FB_SCHEDULE_GRID if m == 1 or (grid and k != 5 and m == n) else nat.FB_SCHEDULE_LAGGED
+        since = 0 if m == 1 else since + 1
+        want = nat.FB_SCHEDULE_LAGGED if m > 1 and since >= first else nat.FB_SCHEDULE_GRID
         assert batch.last_schedule() == want, k
         same(ob, batch, 0, (N, n, k))
 
