@@ -1336,14 +1336,14 @@ static int win_create(fb_brains *br) {
   R.smem = window_smem_bytes(B);
   if (window_blocks_per_sm(B, R.smem) < 1) return fail(FB_EINVAL, "fb_step: the windowed kernel does not fit on an SM (%zu bytes)", R.smem);
   auto n4 = [&](int b) { return align256((size_t)br->host[b].N * 4); };
-  // what must start at zero comes first: per brain drvPos, bgMask and arr (wcnt from the offsets)
+  // what must start at zero comes first: per brain bgMask and arr (wcnt from the offsets, drvPos all ones)
   size_t zero = align256(sizeof(WinBrain) * B) + align256(256 * 4 + (size_t)B * kWarpBrainBytes), rest = 0;
   std::vector<uint64_t> cap(B);
   for (int b = 0; b < B; b++) {
     const Trial &T = br->host[b];
     cap[b] = log_capacity(T);
-    zero += 2 * n4(b) + align256(T.N) + ((T.flags & kHasBg) ? bg_hit_bytes(T) : 0);
-    rest += n4(b) + align256(cap[b] * 16) + align256((size_t)T.E * 8) + align256((size_t)kWinDriven * (4 + kWinSaved * 4 + 1));
+    zero += n4(b) + align256(T.N) + ((T.flags & kHasBg) ? bg_hit_bytes(T) : 0);
+    rest += 2 * n4(b) + align256(cap[b] * 16) + align256((size_t)T.E * 8) + align256((size_t)kWinDriven * (4 + 4 + kWinSaved * 4 + 1));
   }
   if (cudaMalloc(&R.arena, zero + rest) != cudaSuccess) {
     cudaGetLastError();
@@ -1365,10 +1365,12 @@ static int win_create(fb_brains *br) {
     const Trial &T = br->host[b];
     WinBrain &W = R.host[b];
     W.bgMask = (uint32_t *)take(n4(b));
-    W.drvPos = (int32_t *)take(n4(b));
     W.arr = (uint8_t *)take(T.N);
     if (T.flags & kHasBg) W.bgHit = (uint32_t *)take(bg_hit_bytes(T));
   }
+  char *places = at;  // no neuron has one yet
+  for (int b = 0; b < B; b++) R.host[b].drvPos = (int32_t *)take(n4(b));
+  CU(cudaMemsetAsync(places, 0xff, (size_t)(at - places), br->stream));
   for (int b = 0; b < B; b++) {
     const Trial &T = br->host[b];
     WinBrain &W = R.host[b];
@@ -1379,10 +1381,11 @@ static int win_create(fb_brains *br) {
     W.wcnt = (uint32_t *)take(n4(b));
     W.log = (uint4 *)take(cap[b] * 16);
     W.wbuf = (uint2 *)take((size_t)T.E * 8);
-    char *d = take((size_t)kWinDriven * (4 + kWinSaved * 4 + 1));
+    char *d = take((size_t)kWinDriven * (4 + 4 + kWinSaved * 4 + 1));
     W.dSave = (float4 *)d;
     W.dLive = (uint32_t *)(d + (size_t)kWinDriven * kWinSaved * 4);
-    W.dFired = (uint8_t *)(W.dLive + kWinDriven);
+    W.placed = (int32_t *)(W.dLive + kWinDriven);
+    W.dFired = (uint8_t *)(W.placed + kWinDriven);
     CU(cudaMemcpyAsync(W.wcnt, W.inOff, (size_t)T.N * 4, cudaMemcpyDeviceToDevice, br->stream));
   }
   CU(cudaMemcpyAsync(R.win, R.host.data(), sizeof(WinBrain) * B, cudaMemcpyHostToDevice, br->stream));

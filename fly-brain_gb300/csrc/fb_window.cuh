@@ -40,7 +40,8 @@ constexpr int32_t kWinIds = 1 << 23;  // neurons at most: ids and ranks (driven 
 struct WinBrain {
   int32_t D, H;        // arrival delay in steps; window length
   uint32_t logMask;    // log capacity - 1
-  int32_t pad;
+  int32_t nPlaced;     // neurons with a place in drvPos, and which (kWinDriven at most)
+  int32_t *placed;
   const uint32_t *inOff;  // [N+1] in-degree prefix: where a target's contributions start in wbuf
   int32_t *drvPos;     // [N] place in the driven list, -1 if not driven
   uint32_t *wcnt;      // [N] end of each target's contributions of the window in wbuf (inOff: none)
@@ -92,7 +93,7 @@ const void *window_kernel_wide();
 const void *window_kernel_narrow();
 // In-degree prefix of a topology (off: [N+1]).
 cudaError_t launch_in_offsets(const uint32_t *indices, int32_t N, int64_t E, uint32_t *off, cudaStream_t st);
-// drvPos of every brain from its driven list.
+// drvPos of every brain from its driven list (at most kWinDriven entries).
 cudaError_t launch_driven_pos(const Trial *trials, WinBrain *win, int B, cudaStream_t st);
 // The ring's spikes in flight into the log (import), the log's into the ring (export: every slot
 // in flight, or the last step's list only), the log emptied (brains b0 .. b1-1).

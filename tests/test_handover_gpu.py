@@ -262,3 +262,29 @@ def test_new_refractory_times_keep_the_window_buffers(trefs):
             free = torch.cuda.mem_get_info()[0]
         elif min(trefs) > 1.0:
             assert torch.cuda.mem_get_info()[0] == free, tref
+
+
+@pytest.mark.parametrize("B", [1, 2])
+def test_driven_lists_replaced(B):
+    """The windows' places in the driven lists follow lists that shrink, grow past a block's threads, turn
+    around, empty and come back, also past what windows take; background hits look them up."""
+    p = params(bgRate=30.0, bgAmp=1.0, **GEN)
+    obs, batch = brains(B, p, N=4500, hz=300.0, every=1500, deg=6)
+    rng = np.random.default_rng(4)
+    now = [list(range(0, ob.N, 1500)) for ob in obs]
+    for nD in (3, 1100, 40, 0, 4096, 4200, 1023, 1025, 1):
+        for b in range(B if nD != 40 else 1):  # one brain's alone, too
+            new = rng.permutation(obs[b].N)[:nD].astype(np.int32)
+            for i in now[b]:
+                obs[b].setDriveOne(int(i), 0.0)
+            batch.set_drive(b, np.array(now[b], np.int32), 0.0)
+            for i in new:
+                obs[b].setDriveOne(int(i), 150.0)
+            batch.set_drive(b, new, 150.0)
+            now[b] = new.tolist()
+        for n in (4, 30):
+            for ob in obs:
+                ob.run(n)
+            batch.step(n)
+            for b, ob in enumerate(obs):
+                same(ob, batch, b, (nD, n, b))
