@@ -527,6 +527,7 @@ struct fb_brains {
   bool everRing = false;             // a kernel that keeps the ring's lists has run
   int32_t sinceShort = kLongAgo;     // launches since one that had too few steps for windows
   static constexpr int32_t kLongAgo = 1 << 20;
+  int32_t shortLaunches = 0;         // before the windowed kernel's buffers were there
 };
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -1620,6 +1621,16 @@ static bool handover_pays(const fb_brains *br, int32_t n) {
   return neurons >= 100000 ? n >= 3 : neurons >= 10000 && n >= 4 && n <= H;
 }
 
+// Whether this launch is worth the windowed kernel's buffers, where they are not there yet: 130 to 180 us
+// from some 100,000 edges on, against 20 to 60 us that a short launch saves. The first four go without.
+// (A brain of 165,122 neurons created and given two steps: 920 us with them, 820 without.)
+static bool buffers_pay(fb_brains *br, int32_t n) {
+  if (br->win.ready || n >= 8) return true;
+  int64_t edges = 0;
+  for (const Trial &T : br->host) edges += T.E;
+  return edges < (1 << 17) || br->shortLaunches++ >= 4;
+}
+
 enum class StepKernel { kGrid, kLagged, kWindow };
 
 // The kernel of this launch, its resources ready. head: the steps before a call's windows, for which
@@ -1633,7 +1644,7 @@ static int choose_kernel(fb_brains *br, int32_t n, bool head, StepKernel *k) {
   if (forced && !applies) return fail(FB_EINVAL, "fb_step: the delay-scheduled schedule does not apply to %s", why);
   const bool window = win_capable(br) && !br->win.noMemory && !is_irregular(br) &&
                       (forced || (n >= win_min_steps(br) && !br->profiling && (!br->logging || (br->B == 1 && n <= kWinLogSteps)) &&
-                                  windows_pay(br, n) && handover_pays(br, n)));
+                                  windows_pay(br, n) && handover_pays(br, n) && buffers_pay(br, n)));
   const bool lagged = applies && fires_once_a_step(br->host[0]) &&
                       (forced || (n >= kLagMinSteps && !br->lag.noMemory && (!head || br->lag.ready)));
   int rc = FB_OK;

@@ -288,3 +288,16 @@ def test_driven_lists_replaced(B):
             batch.step(n)
             for b, ob in enumerate(obs):
                 same(ob, batch, b, (nD, n, b))
+
+
+@pytest.mark.parametrize("deg,first", [(20, 1), (700, 5)])
+def test_first_short_launches(deg, first):
+    """The windowed kernel's buffers are made for the fifth short launch where they cost something."""
+    from flybrain import _native as nat
+    obs, batch = brains(1, params(**DEP), deg=deg)
+    ob = obs[0]
+    for k, n in enumerate((2, 3, 7, 2, 4, 2, 9, 1)):
+        ob.run(n)
+        batch.step(n)
+        assert batch.last_schedule() == (nat.FB_SCHEDULE_LAGGED if k + 1 >= first and n > 1 else nat.FB_SCHEDULE_GRID), k
+        same(ob, batch, 0, (deg, k))
