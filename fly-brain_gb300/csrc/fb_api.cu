@@ -1621,14 +1621,14 @@ static bool handover_pays(const fb_brains *br, int32_t n) {
   return neurons >= 100000 ? n >= 3 : neurons >= 10000 && n >= 4 && n <= H;
 }
 
-// Whether this launch is worth the windowed kernel's buffers, where they are not there yet: 130 to 180 us
-// from some 100,000 edges on, against 20 to 60 us that a short launch saves. The first four go without.
+// Whether this launch is worth the windowed kernel's buffers, where they are not there yet: 100 to 180 us
+// from some 30,000 edges on, against 5 to 60 us that a short launch saves. The first four go without.
 // (A brain of 165,122 neurons created and given two steps: 920 us with them, 820 without.)
 static bool buffers_pay(fb_brains *br, int32_t n) {
   if (br->win.ready || n >= 8) return true;
   int64_t edges = 0;
   for (const Trial &T : br->host) edges += T.E;
-  return edges < (1 << 17) || br->shortLaunches++ >= 4;
+  return edges < (1 << 15) || br->shortLaunches++ >= 4;
 }
 
 enum class StepKernel { kGrid, kLagged, kWindow };

@@ -145,7 +145,9 @@ int fb_brains_set_mode(fb_brains *br, int32_t mode);
  * the delay, where windows would be short or do not apply (a refractory time under one step, more
  * draws than a block's shared memory holds). AUTO (default) takes one of them where they apply and
  * the launch has at least 2 steps (3 with background events) and, in a batch, windows of more than
- * one, GRID otherwise. LAGGED forces them for one brain; where neither applies fb_step then fails
+ * one, GRID otherwise; the first launches of a few steps, and such launches soon after a single step,
+ * stay on GRID, where the windows' buffers or the way of the spikes in flight would cost more than
+ * they save. LAGGED forces them for one brain; where neither applies fb_step then fails
  * with FB_EINVAL. (With a refractory time under one step and threshold offsets, or vReset >=
  * vThresh, a neuron may fire twice in a step: GRID, under LAGGED too.) */
 #define FB_SCHEDULE_AUTO 0
