@@ -128,7 +128,7 @@ struct LagShared {
   int32_t known;   // highest step known finished by every block
   int32_t head0;   // ring head at launch
   int64_t steps0;  // steps done before the launch
-  int64_t logBase;
+  int64_t logLen, logBase;  // the record's length before the launch, before the step
   uint32_t scan[33];
   uint64_t scan64[33];
   uint32_t dbCount;               // epilogue scratch
@@ -1138,6 +1138,8 @@ __global__ void __launch_bounds__(kLB, 1) lagged_kernel(LagArgs a) {
   // slots delivered during the launch are empty (lif.c:44) unless refilled below
   if (blockIdx.x == 0)
     for (int u = tid; u < min(a.T, ns); u += blockDim.x) a.ringCount[(head0 + u) % ns] = 0;
+  // read before any block writes the new length: after an even number of steps it is the same word
+  if (tid == 0) sh.logLen = a.log ? ldcg(&a.G->logRasterLen[steps0 & 1]) : 0;
   if (!lag_grid_sync(a)) return;
   if (tid == 0) sh.dbCount = 0;
   __syncthreads();
@@ -1184,7 +1186,7 @@ __global__ void __launch_bounds__(kLB, 1) lagged_kernel(LagArgs a) {
       tOff[a.nTB] = (int32_t)carry;
       int64_t rb = 0;
       if (a.log) {  // launches with logging have at most kLagRing steps
-        rb = ldcg(&a.G->logRasterLen[steps0 & 1]);
+        rb = sh.logLen;
         for (int x = 0; x < s; x++) rb += ldcg(a.stepTot + x);
       }
       sh.logBase = rb;

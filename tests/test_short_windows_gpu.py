@@ -169,3 +169,24 @@ def test_recorded_launches(tref, delay, over):
         np.testing.assert_array_equal(k, counts, err_msg=str(n))
         np.testing.assert_array_equal(r, raster, err_msg=str(n))
         same(ob, b, 0, (tref, n))
+
+
+@pytest.mark.parametrize("n", [8, 16, 20, 40, 64])
+@pytest.mark.parametrize("nD", [60, 600])
+def test_recorded_lists_of_many_spikes(n, nD):
+    """Every step's list is placed after the record as it was before the launch, also where the length
+    after it (an even number of steps) takes the same word and one list is ready long before another."""
+    from flybrain import BrainBatch, DeviceGraph
+    g = make(794, 3, deg=20)
+    p = params(tRef=0.15)
+    idx = np.random.default_rng(1).permutation(g.N)[:nD].astype(np.int32)
+    ob = pair(g, p, 5, idx, np.full(nD, 1e5))
+    b = BrainBatch([DeviceGraph(g)], p, [5])
+    b.set_drive(0, idx, 1e5)
+    b.record(10 * n, 1 << 18)
+    want = [ob.run(n, raster=True) for _ in range(10)]
+    for _ in range(10):
+        b.step(n)
+    k, r = b.spike_log(0, 10 * n, 1 << 18)
+    np.testing.assert_array_equal(k, np.concatenate([c for c, _ in want]))
+    np.testing.assert_array_equal(r, np.concatenate([x for _, x in want]))
